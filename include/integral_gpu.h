@@ -94,7 +94,7 @@ typedef struct {
   uint64_t quartets_fp32;     /* of them, evaluated in FP32 (MIXED) */
   uint64_t prim_quartets;     /* surviving primitive quartets */
   double model_flops;         /* fixed Rys flop model of the surviving work */
-  double kernel_ms;           /* device time of the quartet kernels */
+  double kernel_ms;           /* device time of the quartet kernels, first start to last end */
   uint32_t launches;          /* kernels launched by the call */
 } igpu_stats;
 
@@ -107,7 +107,8 @@ typedef struct {
   uint64_t tasks;             /* quartets in the launch's task list */
   uint64_t quartets;          /* of them accepted by the screening */
   uint64_t prim_quartets;
-  double ms;                  /* device time (CUDA events) */
+  double ms;                  /* device time (CUDA events); launches of one call overlap, so
+                               * this includes waiting for the others (not while autotuning) */
   double model_flops;         /* fixed Rys flop model of the accepted work */
   uint32_t chunk;             /* tasks a warp claims per grab */
   uint32_t reserved;

@@ -241,53 +241,153 @@ size_t slot_with_acc(const KernelEntry* e, int pcb, const KernelArgs& A) {
   return e->slot + 1 + (size_t)A.jk.ndens * nab;
 }
 
+// The other streams of a run and their join events, made on first use.
+static int ensure_side_streams(igpu_plan* P, size_t n) {
+  while (P->side_ev.size() < n + 1) {  // event n forks, the others join
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    P->side_ev.push_back(ev);
+  }
+  while (P->side.size() < n) {
+    cudaStream_t st;
+    CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    P->side.push_back(st);
+  }
+  return IGPU_OK;
+}
+
 // Run every launch of a task set; quartet kernels only.  Per-launch device
 // time and counters are kept for igpu_last_profile.
+//
+// The launches are independent (J/K, gradient and counters are summed with
+// atomics, every other mode stores each element once), so those with fewer
+// than kFullRounds quartets per resident team are spread over up to
+// kRunStreams streams, longest first, each onto the stream with the least
+// estimated load; `s` waits for all of them.  A class of a small molecule
+// fills a fraction of the device (the 120 (gg|gg) quartets of a 5-atom
+// molecule run on 30 of 148 SMs for 19 ms), and a launch of a few rounds
+// leaves it idle over its last quartets.  Longer launches gain nothing from
+// company and stay on `s`, one after another: each stream has a scratch region
+// of its own, and allocating one costs 50 us/MB.  The launch-shape tuner times
+// all launches one after another.
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches) {
   const bool grad = A.mode == MODE_GRAD;
   auto entry = [grad](int pcb, int pck) { return grad ? grad_entry(pcb, pck) : kernel_entry(pcb, pck); };
-  size_t need = 0;
-  for (auto& L : ts.launches) {
+  const size_t nl = ts.launches.size();
+  struct Planned {
+    size_t li, grid, slot, stream;
+    const KernelEntry* e;
+    double load;
+    bool full;  // enough rounds to fill the device by itself
+  };
+  std::vector<Planned> run;
+  for (size_t li = 0; li < nl; ++li) {
+    Launch* L = ts.launches[li].get();
     if (L->total == 0) continue;
     const KernelEntry* e = entry(L->pcb, L->pck);
     if (!e) return fail(IGPU_ERR_UNSUPPORTED, "angular class not compiled for the GPU");
     if (A.mode == MODE_JK && L->fp32 && !A.jk.Df)
       return fail(IGPU_ERR_INVALID_ARGUMENT, "FP32 J/K launch without the FP32 densities");
-    need = std::max(need, grid_for(e, L->fp32, L->total) * (128 / e->team) * slot_with_acc(e, L->pcb, A));
+    int bps_cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
+    if (P->tune_bps) {
+      bps_cap = P->tune_bps > 0 ? P->tune_bps : 0;
+    } else if (A.mode == MODE_JK || grad) {
+      auto t = P->tuned_bps.find(tune_key(L->pcb, L->pck, L->fp32, grad));
+      if (t != P->tuned_bps.end()) bps_cap = t->second;
+    }
+    Planned r{};
+    r.li = li;
+    r.e = e;
+    r.grid = grid_for(e, L->fp32, L->total, bps_cap);
+    r.slot = slot_with_acc(e, L->pcb, A);
+    // rounds of quartets over the resident teams times one quartet's work on
+    // a team's lanes
+    const int la = pc_la_host(L->pcb), lb = L->pcb - la * (la + 1) / 2;
+    const int lc = pc_la_host(L->pck), ld = L->pck - lc * (lc + 1) / 2;
+    const double teams = (double)r.grid * (128 / e->team);
+    const double np = (double)L->prim_pairs * L->prim_pairs;
+    r.full = (double)L->total >= kFullRounds * teams;
+    r.load = std::ceil((double)L->total / teams) * np *
+             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / e->team;
+    run.push_back(r);
   }
-  CK(P->d_scratch.ensure(need));
-  const size_t nl = ts.launches.size();
+  // longest first; fewer streams while the scratch regions exceed the budget
+  std::vector<size_t> order(run.size());
+  std::iota(order.begin(), order.end(), (size_t)0);
+  std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
+    return run[x].full != run[y].full ? run[x].full : run[x].load > run[y].load;
+  });
+  auto doubles = [](const Planned& r) { return r.grid * (128 / r.e->team) * r.slot; };
+  size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(kRunStreams, run.size()));
+  std::vector<size_t> region;  // scratch doubles per stream
+  size_t largest = 0;
+  for (const Planned& r : run) largest = std::max(largest, doubles(r));
+  for (;; ns = (ns + 1) / 2) {
+    std::vector<double> load(ns, 0.0);
+    region.assign(ns, 0);
+    for (size_t x : order) {
+      Planned& r = run[x];
+      r.stream = r.full ? 0 : (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+      load[r.stream] += r.load;
+      region[r.stream] = std::max(region[r.stream], doubles(r));
+    }
+    if (ns == 1 || std::accumulate(region.begin(), region.end(), (size_t)0) <= std::max(2 * largest, kScratchBudget))
+      break;
+  }
+  if (ns == 1) std::iota(order.begin(), order.end(), (size_t)0);
+  CK(P->d_scratch.ensure(std::accumulate(region.begin(), region.end(), (size_t)0)));
+  std::vector<double*> base(ns, P->d_scratch.p);
+  for (size_t k = 1; k < ns; ++k) base[k] = base[k - 1] + region[k - 1];
+  if (ns > 1) {
+    const int rc = ensure_side_streams(P, ns - 1);
+    if (rc) return rc;
+  }
   LaunchLog& lg = *P->cur_log;
   CK(lg.counters.ensure(nl));
   CK(cudaMemsetAsync(lg.counters.p, 0, nl * sizeof(Counters), s));
   CK(lg.work.ensure(nl));
   CK(cudaMemsetAsync(lg.work.p, 0, nl * sizeof(unsigned long long), s));
-  while (lg.events.size() < 2 * nl) {
+  while (lg.events.size() < 2 * nl + 2) {
     cudaEvent_t ev;
     CK(cudaEventCreate(&ev));
     lg.events.push_back(ev);
   }
-  lg.profile.clear();
-  lg.profile_launch.clear();
+  lg.profile.assign(run.size(), igpu_launch_record{});
+  lg.profile_launch.resize(run.size());
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(s, &cap));
   const bool capturing = cap == cudaStreamCaptureStatusActive;
+  // under stream capture the records are external nodes, so that the graph
+  // records them on every replay (the flag is only valid there)
+  auto record = [capturing](cudaEvent_t ev, cudaStream_t st) {
+    return capturing ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal) : cudaEventRecord(ev, st);
+  };
   const double prim_cut0 = A.prim_cut;
-  for (size_t li = 0; li < nl; ++li) {
-    Launch* L = ts.launches[li].get();
-    if (L->total == 0) continue;
-    const KernelEntry* e = entry(L->pcb, L->pck);
-    const int key = tune_key(L->pcb, L->pck, L->fp32, A.mode == MODE_GRAD);
-    int cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
-    if (P->tune_bps) {
-      cap = P->tune_bps > 0 ? P->tune_bps : 0;
-    } else if (A.mode == MODE_JK || A.mode == MODE_GRAD) {
-      auto t = P->tuned_bps.find(key);
-      if (t != P->tuned_bps.end()) cap = t->second;
+  Counters* const counters = A.counters ? lg.counters.p : nullptr;
+  CK(record(lg.events[2 * nl], s));
+  auto stream_of = [&](size_t k) { return k == 0 ? s : P->side[k - 1]; };
+  // a return before the join leaves no launch behind that the caller's
+  // stream does not wait for
+  struct Finish {
+    igpu_plan* P;
+    size_t n;
+    bool armed;
+    ~Finish() {
+      for (size_t k = 0; armed && k < n; ++k) cudaStreamSynchronize(P->side[k]);
     }
-    const size_t grid = grid_for(e, L->fp32, L->total, cap);
-    A.scratch = P->d_scratch.p;
-    A.slot_doubles = slot_with_acc(e, L->pcb, A);
+  } finish{P, ns - 1, !capturing};
+  if (ns > 1) {
+    CK(cudaEventRecord(P->side_ev[ns - 1], s));
+    for (size_t k = 1; k < ns; ++k) CK(cudaStreamWaitEvent(stream_of(k), P->side_ev[ns - 1], 0));
+  }
+  for (size_t x : order) {
+    const Planned& pl = run[x];
+    Launch* L = ts.launches[pl.li].get();
+    const KernelEntry* e = pl.e;
+    const size_t li = pl.li, grid = pl.grid;
+    const cudaStream_t st = stream_of(pl.stream);
+    A.scratch = base[pl.stream];
+    A.slot_doubles = pl.slot;
     A.acc_offset = e->slot;
     A.work_counter = lg.work.p + li;
     // tasks a warp claims per grab: (32 / team) x mult.  Untuned, mult is 16,
@@ -300,12 +400,12 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     int mult = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(16, fill));
     if (P->tune_mult) {
       mult = P->tune_mult;
-    } else if (A.mode == MODE_JK || A.mode == MODE_GRAD) {
-      auto t = P->tuned_mult.find(key);
+    } else if (A.mode == MODE_JK || grad) {
+      auto t = P->tuned_mult.find(tune_key(L->pcb, L->pck, L->fp32, grad));
       if (t != P->tuned_mult.end()) mult = t->second;
     }
     A.chunk = (unsigned long long)(32 / e->team) * mult;
-    if (A.counters) A.counters = lg.counters.p + li;
+    A.counters = counters ? counters + li : nullptr;
     A.task.bra_pair = L->bra_pair.p;
     A.task.ket_pairs = L->ket_list;
     A.task.prefix = L->prefix.p;
@@ -315,15 +415,11 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     A.fp32 = L->fp32 ? 1 : 0;
     A.prim_cut = prim_cut0 / fp32_class_scale(class_lmax(L->pcb, L->pck));
     A.builder_swap = L->builder_swap;
-    // under stream capture the records are external nodes, so that the
-    // graph records them on every replay (the flag is only valid there)
-    CK(capturing ? cudaEventRecordWithFlags(lg.events[2 * li], s, cudaEventRecordExternal)
-                 : cudaEventRecord(lg.events[2 * li], s));
-    CK(launch_quartets(e, L->fp32, (int)grid, A, s));
-    CK(capturing ? cudaEventRecordWithFlags(lg.events[2 * li + 1], s, cudaEventRecordExternal)
-                 : cudaEventRecord(lg.events[2 * li + 1], s));
+    CK(record(lg.events[2 * li], st));
+    CK(launch_quartets(e, L->fp32, (int)grid, A, st));
+    CK(record(lg.events[2 * li + 1], st));
     ++launches;
-    igpu_launch_record r{};
+    igpu_launch_record& r = lg.profile[x];
     r.la = pc_la_host(L->pcb);
     r.lb = L->pcb - r.la * (r.la + 1) / 2;
     r.lc = pc_la_host(L->pck);
@@ -333,16 +429,23 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     r.grid = (uint32_t)grid;
     r.tasks = L->total;
     r.chunk = (uint32_t)A.chunk;
-    lg.profile.push_back(r);
-    lg.profile_launch.push_back(li);
+    lg.profile_launch[x] = li;
   }
+  for (size_t k = 1; k < ns; ++k) {
+    CK(cudaEventRecord(P->side_ev[k - 1], stream_of(k)));
+    CK(cudaStreamWaitEvent(s, P->side_ev[k - 1], 0));
+  }
+  finish.armed = false;
+  CK(record(lg.events[2 * nl + 1], s));
+  lg.span_event = 2 * nl;
   return IGPU_OK;
 }
 
 // After the stream is synchronised: per-launch times, counters, model flops.
 int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c, int grad_terms_x) {
   LaunchLog& lg = *P->cur_log;
-  const size_t nl = lg.profile.empty() ? 0 : lg.profile_launch.back() + 1;
+  size_t nl = 0;
+  for (size_t li : lg.profile_launch) nl = std::max(nl, li + 1);
   std::vector<Counters> c(nl);
   if (nl) CK(cudaMemcpy(c.data(), lg.counters.p, nl * sizeof(Counters), cudaMemcpyDeviceToHost));
   P->last = igpu_stats{};
@@ -369,8 +472,15 @@ int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c, int grad
     P->last.quartets_fp32 += c[li].fp32_quartets;
     P->last.prim_quartets += c[li].prim_quartets;
     P->last.model_flops += r.model_flops;
-    P->last.kernel_ms += ms;
   }
+  // the launches overlap: the run's device time is its span
+  float span = 0.f;
+  if (!lg.profile.empty() &&
+      cudaEventElapsedTime(&span, lg.events[lg.span_event], lg.events[lg.span_event + 1]) != cudaSuccess) {
+    cudaGetLastError();
+    span = 0.f;
+  }
+  P->last.kernel_ms = span;
   P->last.launches = (uint32_t)lg.profile.size();
   return IGPU_OK;
 }
@@ -395,6 +505,7 @@ std::unique_ptr<Launch> make_launch(igpu_plan* P, int pcb, int pck, bool fp32, c
   }
   L->nbra = (int)b.size();
   L->total = pre.back();
+  if (!b.empty()) L->prim_pairs = std::max(1, P->pairs[b[0]].nprim);
   L->ket_list = ket_list_dev;
   rc = IGPU_OK;
   cudaError_t e;

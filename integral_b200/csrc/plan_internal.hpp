@@ -81,6 +81,7 @@ struct Launch {
   bool fp32 = false;
   int builder_swap = 0;
   int nbra = 0;
+  int prim_pairs = 1;  // primitive pairs of its first bra, for the load estimate
   unsigned long long total = 0;
   DevBuf<int> bra_pair, ket_start, own_kets;
   DevBuf<unsigned long long> prefix;
@@ -96,13 +97,24 @@ struct TaskSet {
 struct LaunchLog {
   DevBuf<Counters> counters;
   DevBuf<unsigned long long> work;
-  std::vector<cudaEvent_t> events;
+  std::vector<cudaEvent_t> events;  // start and end of every launch, then of the whole run
+  size_t span_event = 0;  // first of the run's two events
   std::vector<igpu_launch_record> profile;
   std::vector<size_t> profile_launch;
   ~LaunchLog() {
     for (cudaEvent_t ev : events) cudaEventDestroy(ev);
   }
 };
+
+// Streams that a run's class launches are spread over, the caller's among
+// them (device connections by default: more would share one queue).
+constexpr size_t kRunStreams = 8;
+// Scratch doubles (256 MiB, or twice the largest launch's) above which a run
+// uses fewer streams, each of which needs a scratch region of its own.
+constexpr size_t kScratchBudget = (size_t)1 << 25;
+// Quartets per resident team from which a launch fills the device by itself:
+// its last round is then at most a sixteenth of it.
+constexpr double kFullRounds = 16.0;
 
 // Mixed-precision J/K task lists kept per plan (see igpu_plan::mixed_keys).
 constexpr size_t kMixedTaskSets = 4;
@@ -145,6 +157,13 @@ struct igpu_plan {
   bool schwarz_upper_done = false;
   // device
   cudaStream_t stream = nullptr;
+  // the other streams of a run and the events that join them (run_tasks)
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> side_ev;
+  ~igpu_plan() {
+    for (cudaEvent_t ev : side_ev) cudaEventDestroy(ev);
+    for (cudaStream_t st : side) cudaStreamDestroy(st);
+  }
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   DevBuf<DevShell> d_shells;
   DevBuf<PairD> d_pairs;
