@@ -93,7 +93,6 @@ __device__ __forceinline__ void static_for(F&& f) {
 // Triples by global address (degree <= 20): packed lx | ly<<8 | lz<<16.
 constexpr int ADDR_TAB_DEG = ADDR_TAB_DEG_HOST;
 static __constant__ int c_addr_lxyz[n_addr(ADDR_TAB_DEG)];
-static __constant__ RysMeta c_rys[MAX_ROOTS + 1];
 static __constant__ double c_lag_x[MAX_ROOTS][MAX_ROOTS];
 static __constant__ double c_lag_w[MAX_ROOTS][MAX_ROOTS];
 static __constant__ float c_lag_xf[MAX_ROOTS][MAX_ROOTS];
@@ -104,7 +103,6 @@ static __constant__ const float* c_rys_tab_f;
 static inline cudaError_t upload_module_constants(const ConstData& c) {
   cudaError_t e;
   if ((e = cudaMemcpyToSymbol(c_addr_lxyz, c.addr_lxyz, sizeof(int) * c.n_addr))) return e;
-  if ((e = cudaMemcpyToSymbol(c_rys, c.meta, sizeof(RysMeta) * (MAX_ROOTS + 1)))) return e;
   if ((e = cudaMemcpyToSymbol(c_lag_x, c.lag_x, sizeof(double) * MAX_ROOTS * MAX_ROOTS))) return e;
   if ((e = cudaMemcpyToSymbol(c_lag_w, c.lag_w, sizeof(double) * MAX_ROOTS * MAX_ROOTS))) return e;
   if ((e = cudaMemcpyToSymbol(c_lag_xf, c.lag_xf, sizeof(float) * MAX_ROOTS * MAX_ROOTS))) return e;
@@ -120,122 +118,138 @@ __device__ __forceinline__ int addr_lz(int a) { return (c_addr_lxyz[a] >> 16) & 
 
 // ----------------------------------------------------------------- Rys
 
-template <typename R>
-__device__ __forceinline__ R chebev(const R* __restrict__ c, R xi) {
-  R two_xi = R(2) * xi;
-  R d = R(0), dd = R(0);
-#pragma unroll
-  for (int k = RYS_NC - 1; k >= 1; --k) {
-    R sv = d;
-    d = two_xi * d - dd + __ldg(c + k);
-    dd = sv;
-  }
-  return xi * d - dd + R(0.5) * __ldg(c);
+// Whether a kernel stages its N-root table in shared memory: the
+// one-thread classes and the FP32 teams up to four roots (at most 39 KB in
+// FP64, 14 KB in FP32 per block).  FP64 teams, whose shared memory holds the
+// recurrence tables of their primitive quartets, and larger N read it through
+// L1 (a team evaluates one root per lane, a small part of its work).
+template <int N, typename R>
+__host__ __device__ constexpr bool rys_staged(int team) {
+  return N <= 4 && (team == 1 || sizeof(R) == 4);
+}
+template <int N, typename R>
+__host__ __device__ constexpr int rys_smem(int team) {
+  return rys_staged<N, R>(team) ? rys_nsub(N) * rys_row<R>(N) : 4;
 }
 
-// Largest number of Chebyshev subintervals of any n (15 for n = 13).
-constexpr int RYS_MAX_SUB = 16;
-
-// Copy the N-root table (all subintervals) into shared memory; every thread
-// of the block must call it.  Lookups of different T by the lanes of a warp
-// are then shared-memory reads instead of scattered L1 sectors.
 template <int N, typename R>
-__device__ __forceinline__ void stage_rys_table(R* s_tab) {
-  const RysMeta m = c_rys[N];
-  const R* src;
+__device__ __forceinline__ const R* rys_global() {
   if constexpr (sizeof(R) == 8)
-    src = c_rys_tab + m.off;
+    return c_rys_tab + rys_off<double>(N);
   else
-    src = c_rys_tab_f + m.off;
-  const int sub = m.n_sub < RYS_MAX_SUB ? m.n_sub : RYS_MAX_SUB;
-  const int cnt = sub * N * 2 * RYS_NC;
-  for (int i = threadIdx.x; i < cnt; i += blockDim.x) s_tab[i] = __ldg(src + i);
+    return c_rys_tab_f + rys_off<float>(N);
+}
+
+// Copy the N-root table into shared memory where the kernel stages it; every
+// thread of the block must call it (it ends in a block barrier either way).
+template <int N, typename R, int TEAM>
+__device__ __forceinline__ void stage_rys_table(R* s_tab) {
+  if constexpr (rys_staged<N, R>(TEAM)) {
+    constexpr int PER = 16 / sizeof(R);
+    const uint4* src = reinterpret_cast<const uint4*>(rys_global<N, R>());
+    uint4* dst = reinterpret_cast<uint4*>(s_tab);
+    for (int i = threadIdx.x; i < rys_nsub(N) * rys_row<R>(N) / PER; i += blockDim.x) dst[i] = __ldg(src + i);
+  }
   __syncthreads();
 }
 
-template <typename R>
-__device__ __forceinline__ R chebev_s(const R* c, R xi) {
-  R two_xi = R(2) * xi;
-  R d = R(0), dd = R(0);
+// One polynomial of a table row (16-byte aligned; GLOBAL: read through the
+// read-only path) by Horner's scheme.  The series on unit intervals replaces
+// 17-term Chebyshev sums on intervals about six times as wide: 11 FP64
+// operations and 6 wide reads a value for 32 and 17, and xi without rounding
+// or division.
+template <bool GLOBAL>
+__device__ __forceinline__ double rys_poly(const double* c, double xi) {
+  const double2* q = reinterpret_cast<const double2*>(c);
+  auto at = [q](int k) {
+    if constexpr (GLOBAL)
+      return __ldg(q + k);
+    else
+      return q[k];
+  };
+  double2 t = at(5);
+  double v = fma(t.y, xi, t.x);
 #pragma unroll
-  for (int k = RYS_NC - 1; k >= 1; --k) {
-    R sv = d;
-    d = two_xi * d - dd + c[k];
-    dd = sv;
+  for (int k = 4; k >= 0; --k) {
+    t = at(k);
+    v = fma(v, xi, t.y);
+    v = fma(v, xi, t.x);
   }
-  return xi * d - dd + R(0.5) * c[0];
+  return v;
+}
+template <bool GLOBAL>
+__device__ __forceinline__ float rys_poly(const float* c, float xi) {
+  const float4* q = reinterpret_cast<const float4*>(c);
+  auto at = [q](int k) {
+    if constexpr (GLOBAL)
+      return __ldg(q + k);
+    else
+      return q[k];
+  };
+  const float4 u = at(1), t = at(0);
+  float v = fmaf(u.w, xi, u.z);
+  v = fmaf(v, xi, u.y);
+  v = fmaf(v, xi, u.x);
+  v = fmaf(v, xi, t.w);
+  v = fmaf(v, xi, t.z);
+  v = fmaf(v, xi, t.y);
+  return fmaf(v, xi, t.x);
 }
 
-// Roots/weights from the shared-memory copy of the N-root table.
-template <int N, typename R>
-__device__ __forceinline__ void rys_roots_s(const R* s_tab, R T, R* x, R* w) {
-  const RysMeta m = c_rys[N];
-  if (T >= R(m.t_hi)) {
-    R inv_t = R(1) / T;
-    R sc = R(0.5) * rsqrt(T);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      if constexpr (sizeof(R) == 8) {
-        x[i] = c_lag_x[N - 1][i] * inv_t;
-        w[i] = c_lag_w[N - 1][i] * sc;
-      } else {
-        x[i] = c_lag_xf[N - 1][i] * inv_t;
-        w[i] = c_lag_wf[N - 1][i] * sc;
-      }
-    }
-    return;
-  }
-  R width = R(m.width);
-  int s = (int)(T / width);
-  s = s < 0 ? 0 : (s >= m.n_sub ? m.n_sub - 1 : s);
-  R a = R(s) * width;
-  R b = a + width;
-  R xi = (R(2) * T - (a + b)) / (b - a);
-  const R* base = s_tab + (size_t)s * N * 2 * RYS_NC;
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    x[i] = chebev_s<R>(base + (2 * i) * RYS_NC, xi);
-    w[i] = chebev_s<R>(base + (2 * i + 1) * RYS_NC, xi);
-  }
+// Interval of T < rys_t_hi(N) and the position in it.
+template <typename R>
+__device__ __forceinline__ int rys_interval(R T, R& xi) {
+  const int s = (int)T;
+  xi = R(2) * (T - R(s)) - R(1);
+  return s;
 }
 
 // N-point Rys quadrature at parameter T (src/math/rys.rs:174-215): the
-// generalized-Laguerre(-1/2) limit above asymptotic_boundary(2N-1), else the
-// piecewise Chebyshev interpolation.  x = squared roots, w = weights.
-template <int N, typename R>
-__device__ __forceinline__ void rys_roots(R T, R* x, R* w) {
-  const RysMeta m = c_rys[N];
-  if (T >= R(m.t_hi)) {
-    R inv_t = R(1) / T;
-    R sc = R(0.5) * rsqrt(T);
+// generalized-Laguerre(-1/2) limit above the crossover, else the tables.
+// x = squared roots, w = weights.
+template <int N, bool GLOBAL, typename R>
+__device__ __forceinline__ void rys_roots_s(const R* tab, R T, R* x, R* w) {
+  if (T >= R(rys_t_hi(N))) {
+    const R r = rsqrt(T);
+    const R inv_t = R(1) / T;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       if constexpr (sizeof(R) == 8) {
         x[i] = c_lag_x[N - 1][i] * inv_t;
-        w[i] = c_lag_w[N - 1][i] * sc;
+        w[i] = c_lag_w[N - 1][i] * (R(0.5) * r);
       } else {
         x[i] = c_lag_xf[N - 1][i] * inv_t;
-        w[i] = c_lag_wf[N - 1][i] * sc;
+        w[i] = c_lag_wf[N - 1][i] * (R(0.5) * r);
       }
     }
     return;
   }
-  R width = R(m.width);
-  int s = (int)(T / width);
-  s = s < 0 ? 0 : (s >= m.n_sub ? m.n_sub - 1 : s);
-  R a = R(s) * width;
-  R b = a + width;
-  R xi = (R(2) * T - (a + b)) / (b - a);
-  const R* base;
-  if constexpr (sizeof(R) == 8)
-    base = c_rys_tab + m.off + (size_t)s * N * 2 * RYS_NC;
-  else
-    base = c_rys_tab_f + m.off + (size_t)s * N * 2 * RYS_NC;
+  R xi;
+  const R* row = tab + rys_interval(T, xi) * rys_row<R>(N);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    x[i] = chebev<R>(base + (2 * i) * RYS_NC, xi);
-    w[i] = chebev<R>(base + (2 * i + 1) * RYS_NC, xi);
+    x[i] = rys_poly<GLOBAL>(row + (2 * i) * rys_nc<R>(), xi);
+    w[i] = rys_poly<GLOBAL>(row + (2 * i + 1) * rys_nc<R>(), xi);
   }
+}
+
+// Root r of the N-point quadrature.
+template <int N, bool GLOBAL, typename R>
+__device__ __forceinline__ void rys_root_one(const R* tab, R T, int r, R& x, R& w) {
+  if (T >= R(rys_t_hi(N))) {
+    if constexpr (sizeof(R) == 8) {
+      x = c_lag_x[N - 1][r] / T;
+      w = c_lag_w[N - 1][r] * R(0.5) * rsqrt(T);
+    } else {
+      x = c_lag_xf[N - 1][r] / T;
+      w = c_lag_wf[N - 1][r] * R(0.5) * rsqrt(T);
+    }
+    return;
+  }
+  R xi;
+  const R* c = tab + rys_interval(T, xi) * rys_row<R>(N) + 2 * r * rys_nc<R>();
+  x = rys_poly<GLOBAL>(c, xi);
+  w = rys_poly<GLOBAL>(c + rys_nc<R>(), xi);
 }
 
 // Per-axis Rys vertical recurrence g[n][m], n <= NE (bra power on A),
@@ -269,37 +283,28 @@ __device__ __forceinline__ void vrr_axis(R g00, R c00, R cp0, R b10, R b01, R b0
 // Coulomb operator, with T and pref untouched and xs = 1.
 template <typename R>
 struct QuartetHdr {
-  R T, pref, pq, p, q;
+  R T, pref;
+  R qpq, ppq;       // q / (p + q), p / (p + q)
+  R hpq;            // 1 / (2 (p + q))
+  R inv2p, inv2q;   // 1 / (2 p), 1 / (2 q)
   R pqx, pqy, pqz;  // P - Q
   R pax, pay, paz;  // P - A
   R qcx, qcy, qcz;  // Q - C
   R xs;             // root scale (1 for Coulomb)
 };
 
+// r = 1 / sqrt(s) and inv = 1 / s from one rsqrt and a Newton step shared by
+// both (FP32's approximate rsqrt is otherwise off by up to two units).
 template <typename R>
-__device__ __forceinline__ QuartetHdr<R> quartet_header(const PrimPairD& bp, const PrimPairD& kp,
-                                                        double omega) {
-  QuartetHdr<R> h;
-  // 2 pi^{5/2}
-  const double TWO_PI_2_5 = 34.98683665524972;
-  R p = R(bp.zeta), q = R(kp.zeta);
-  h.p = p;
-  h.q = q;
-  h.pq = p + q;
-  R rho = p * q / h.pq;
-  // centre differences in double first: absolute coordinates would lose
-  // the separation to cancellation in FP32
-  h.pqx = R(bp.px - kp.px);
-  h.pqy = R(bp.py - kp.py);
-  h.pqz = R(bp.pz - kp.pz);
-  h.T = rho * (h.pqx * h.pqx + h.pqy * h.pqy + h.pqz * h.pqz);
-  h.pref = R(TWO_PI_2_5) / (p * q * sqrt(h.pq)) * R(bp.e) * R(kp.e);
-  h.pax = R(bp.pax);
-  h.pay = R(bp.pay);
-  h.paz = R(bp.paz);
-  h.qcx = R(kp.pax);
-  h.qcy = R(kp.pay);
-  h.qcz = R(kp.paz);
+__device__ __forceinline__ void inv_and_rsqrt(R s, R& r, R& inv) {
+  const R y = rsqrt(s);
+  const R e = fma(-(s * y), y, R(1));
+  r = fma(R(0.5) * y, e, y);
+  inv = r * r;
+}
+
+template <typename R>
+__device__ __forceinline__ void erf_scale(QuartetHdr<R>& h, R rho, double omega) {
   h.xs = R(1);
   if (omega > 0.0) {
     const R w2 = R(omega) * R(omega);
@@ -308,6 +313,35 @@ __device__ __forceinline__ QuartetHdr<R> quartet_header(const PrimPairD& bp, con
     h.pref *= sqrt(sc);
     h.xs = sc;
   }
+}
+
+template <typename R>
+__device__ __forceinline__ QuartetHdr<R> quartet_header(const PrimPairD& bp, const PrimPairD& kp,
+                                                        double omega) {
+  QuartetHdr<R> h;
+  const R p = R(bp.zeta), q = R(kp.zeta);
+  R r, inv;
+  inv_and_rsqrt(p + q, r, inv);
+  h.hpq = R(0.5) * inv;
+  h.qpq = q * inv;
+  h.ppq = p * inv;
+  const R rho = p * h.qpq;
+  // centre differences in double first: absolute coordinates would lose
+  // the separation to cancellation in FP32
+  h.pqx = R(bp.px - kp.px);
+  h.pqy = R(bp.py - kp.py);
+  h.pqz = R(bp.pz - kp.pz);
+  h.T = rho * (h.pqx * h.pqx + h.pqy * h.pqy + h.pqz * h.pqz);
+  h.pref = R(bp.ez) * R(kp.ez) * r;
+  h.inv2p = R(bp.inv2z);
+  h.inv2q = R(kp.inv2z);
+  h.pax = R(bp.pax);
+  h.pay = R(bp.pay);
+  h.paz = R(bp.paz);
+  h.qcx = R(kp.pax);
+  h.qcy = R(kp.pay);
+  h.qcz = R(kp.paz);
+  erf_scale(h, rho, omega);
   return h;
 }
 
@@ -322,28 +356,9 @@ __device__ __forceinline__ double quartet_T64(const PrimPairD& bp, const PrimPai
   return T;
 }
 
-// Root r of the N-point quadrature at T, evaluated in FP64 from the double
-// tables (the FP32 launches take this path for large T and high l).
-template <int N>
-__device__ __forceinline__ void rys_root_fp64(double T, int r, double& x, double& w) {
-  const RysMeta m = c_rys[N];
-  if (T >= m.t_hi) {
-    x = c_lag_x[N - 1][r] / T;
-    w = c_lag_w[N - 1][r] * 0.5 * rsqrt(T);
-    return;
-  }
-  int s = (int)(T / m.width);
-  s = s < 0 ? 0 : (s >= m.n_sub ? m.n_sub - 1 : s);
-  const double a = (double)s * m.width, b = a + m.width;
-  const double xi = (2.0 * T - (a + b)) / (b - a);
-  const double* base = c_rys_tab + m.off + ((size_t)s * N + r) * 2 * RYS_NC;
-  x = chebev<double>(base, xi);
-  w = chebev<double>(base + RYS_NC, xi);
-}
-
 // The FP32 launches generate roots and weights in FP64 for every quadrature
 // of five or more roots (high angular momentum, l_a + l_b + l_c + l_d >= 8):
-// the n where Clenshaw sums lose digits just below the asymptotic crossover
+// the n where weights lose digits just below the asymptotic crossover
 // (the reference's own FP64 weights lose three to four there at n = 9, 11,
 // 13, src/math/rys.rs:80-89) are all among them.  Above the crossover the
 // roots and weights are the closed forms c_i / T and w_i T^{-1/2}, exact to
@@ -361,29 +376,26 @@ __device__ __forceinline__ QuartetHdr<float> quartet_header_f(const PrimPairF& b
                                                               float acy, float acz, double omega) {
   QuartetHdr<float> h;
   const float p = bp.zeta, q = kp.zeta;
-  h.p = p;
-  h.q = q;
-  h.pq = p + q;
-  const float rho = p * q / h.pq;
+  float r, inv;
+  inv_and_rsqrt(p + q, r, inv);
+  h.hpq = 0.5f * inv;
+  h.qpq = q * inv;
+  h.ppq = p * inv;
+  const float rho = p * h.qpq;
   h.pqx = acx + (bp.pax - kp.pax);
   h.pqy = acy + (bp.pay - kp.pay);
   h.pqz = acz + (bp.paz - kp.paz);
   h.T = rho * (h.pqx * h.pqx + h.pqy * h.pqy + h.pqz * h.pqz);
-  h.pref = 34.98683665524972f / (p * q * sqrtf(h.pq)) * bp.e * kp.e;
+  h.pref = bp.ez * kp.ez * r;
+  h.inv2p = bp.inv2z;
+  h.inv2q = kp.inv2z;
   h.pax = bp.pax;
   h.pay = bp.pay;
   h.paz = bp.paz;
   h.qcx = kp.pax;
   h.qcy = kp.pay;
   h.qcz = kp.paz;
-  h.xs = 1.f;
-  if (omega > 0.0) {
-    const float w2 = float(omega) * float(omega);
-    const float sc = w2 / (rho + w2);
-    h.T *= sc;
-    h.pref *= sqrtf(sc);
-    h.xs = sc;
-  }
+  erf_scale(h, rho, omega);
   return h;
 }
 

@@ -175,7 +175,8 @@ struct GradShape {
   static constexpr int GT = (NEV + 1) * (NFV + 1);
   // per primitive quartet in shared memory: roots, weights*prefactor, the
   // three raise factors 2*alpha_A, 2*alpha_B, 2*alpha_C, and 3*NR 2D tables
-  static constexpr int PRIM_TAB = 2 * NR + 3 + 3 * NR * GT;
+  // (an odd number: its lanes' stores then spread over the banks)
+  static constexpr int PRIM_TAB = (2 * NR + 3 + 3 * NR * GT) | 1;
   static constexpr int BUDGET = (48 * 1024 / 128) * (T == 1 ? 1 : T) / (int)sizeof(R);
   static constexpr int BP0 = BUDGET / PRIM_TAB;
   static constexpr int BP = BP0 >= T ? T : (BP0 >= 16 ? 16 : (BP0 >= 8 ? 8 : (BP0 >= 4 ? 4 : (BP0 >= 2 ? 2 : 1))));
@@ -186,7 +187,7 @@ struct GradShape {
 // --------------------------------------------------- phase 1, one thread
 
 template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void grad_tables_thread(const KernelArgs& A, const R* s_tab, const PairD& pb,
+__device__ __forceinline__ void grad_tables_thread(const KernelArgs& A, const R* rys, const PairD& pb,
                                                    const PairD& pk, double* tab) {
   using GS = GradShape<LA, LB, LC, LD, R>;
   constexpr int NEV = GS::NEV, NFV = GS::NFV, NR = GS::NR;
@@ -212,17 +213,14 @@ __device__ __forceinline__ void grad_tables_thread(const KernelArgs& A, const R*
       const R wC = R(2) * R(kp.alpha);
       const QuartetHdr<R> h = quartet_header<R>(bp, kp, A.omega);
       R x[NR], w[NR];
-      rys_roots_s<NR, R>(s_tab, h.T, x, w);
-      const R inv_pq = R(1) / h.pq;
-      const R qpq = h.q * inv_pq, ppq = h.p * inv_pq;
-      const R inv2pq = R(0.5) * inv_pq, inv2p = R(0.5) / h.p, inv2q = R(0.5) / h.q;
+      rys_roots_s<NR, !rys_staged<NR, R>(1)>(rys, h.T, x, w);
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const R xr = x[r] * h.xs;
-        const R b00 = xr * inv2pq;
-        const R b10 = (R(1) - xr * qpq) * inv2p;
-        const R b01 = (R(1) - xr * ppq) * inv2q;
-        const R cq = xr * qpq, cp = xr * ppq;
+        const R cq = xr * h.qpq, cp = xr * h.ppq;
+        const R b00 = xr * h.hpq;
+        const R b10 = (R(1) - cq) * h.inv2p;
+        const R b01 = (R(1) - cp) * h.inv2q;
         R gx[NEV + 1][NFV + 1], gy[NEV + 1][NFV + 1], gz[NEV + 1][NFV + 1];
         vrr_axis<NEV, NFV, R>(R(1), h.pax - cq * h.pqx, h.qcx + cp * h.pqx, b10, b01, b00, gx);
         vrr_axis<NEV, NFV, R>(R(1), h.pay - cq * h.pqy, h.qcy + cp * h.pqy, b10, b01, b00, gy);
@@ -279,7 +277,7 @@ __device__ __forceinline__ void grad_tables_thread(const KernelArgs& A, const R*
 // -------------------------------------------------------- phase 1, team
 
 template <int LA, int LB, int LC, int LD, typename R, int PASS>
-__device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* s_tab, const PairD& pb, const PairD& pk,
+__device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* rys, const PairD& pb, const PairD& pk,
                                                R* sm, int lane, unsigned tmask, double* tab) {
   using GS = GradShape<LA, LB, LC, LD, R>;
   constexpr int NEV = GS::NEV, NFV = GS::NFV, NR = GS::NR, T = GS::T, GT = GS::GT;
@@ -322,7 +320,7 @@ __device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* s_t
       h = quartet_header<R>(bp, kp, A.omega);
       for (int r = sub; r < NR; r += SUB) {
         R xr, wr;
-        rys_root_one<NR, R>(s_tab, h.T, r, xr, wr);
+        rys_root_one<NR, !rys_staged<NR, R>(T)>(rys, h.T, r, xr, wr);
         mys[r] = xr * h.xs;
         mys[NR + r] = wr * h.pref;
       }
@@ -334,21 +332,18 @@ __device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* s_t
     }
     __syncwarp(tmask);
     if (active) {
-      const R inv_pq = R(1) / h.pq;
-      const R qpq = h.q * inv_pq, ppq = h.p * inv_pq;
-      const R inv2p = R(0.5) / h.p, inv2q = R(0.5) / h.q;
       for (int t = sub; t < 3 * NR; t += SUB) {
         const int axis = t / NR, r = t - axis * NR;
         const R xr = mys[r];
-        const R b00 = xr * R(0.5) * inv_pq;
-        const R b10 = (R(1) - xr * qpq) * inv2p;
-        const R b01 = (R(1) - xr * ppq) * inv2q;
+        const R cq = xr * h.qpq, cp = xr * h.ppq;
+        const R b00 = xr * h.hpq;
+        const R b10 = (R(1) - cq) * h.inv2p;
+        const R b01 = (R(1) - cp) * h.inv2q;
         const R pqa = axis == 0 ? h.pqx : (axis == 1 ? h.pqy : h.pqz);
         const R paa = axis == 0 ? h.pax : (axis == 1 ? h.pay : h.paz);
         const R qca = axis == 0 ? h.qcx : (axis == 1 ? h.qcy : h.qcz);
         R g[NEV + 1][NFV + 1];
-        vrr_axis<NEV, NFV, R>(axis == 2 ? mys[NR + r] : R(1), paa - xr * qpq * pqa, qca + xr * ppq * pqa, b10, b01,
-                              b00, g);
+        vrr_axis<NEV, NFV, R>(axis == 2 ? mys[NR + r] : R(1), paa - cq * pqa, qca + cp * pqa, b10, b01, b00, g);
         R* dst = mys + 2 * NR + 3 + (axis * NR + r) * GT;
 #pragma unroll
         for (int n = 0; n <= NEV; ++n)
@@ -429,13 +424,13 @@ __device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* s_t
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int PASS>
-__device__ __forceinline__ void grad_team_passes(const KernelArgs& A, const R* s_tab, const PairD& pb,
+__device__ __forceinline__ void grad_team_passes(const KernelArgs& A, const R* rys, const PairD& pb,
                                                  const PairD& pk, R* sm, int lane, unsigned tmask, double* tab) {
   using GS = GradShape<LA, LB, LC, LD, R>;
   if constexpr (PASS < GS::PL.npass) {
-    grad_team_pass<LA, LB, LC, LD, R, PASS>(A, s_tab, pb, pk, sm, lane, tmask, tab);
+    grad_team_pass<LA, LB, LC, LD, R, PASS>(A, rys, pb, pk, sm, lane, tmask, tab);
     __syncwarp(tmask);
-    grad_team_passes<LA, LB, LC, LD, R, PASS + 1>(A, s_tab, pb, pk, sm, lane, tmask, tab);
+    grad_team_passes<LA, LB, LC, LD, R, PASS + 1>(A, rys, pb, pk, sm, lane, tmask, tab);
   }
 }
 
@@ -559,13 +554,13 @@ __device__ __forceinline__ void grad_dot(const double* W, const double* blk, con
 
 // One shifted block: copy its [e0|f0] slice into the first HRR buffer, run
 // the bra and ket recurrences, dot with W.
-__device__ __forceinline__ void grad_shifted(const double* tabp, int tab_cols, int row_off, int nrows, int col_off,
+__device__ __forceinline__ void grad_shifted(const double* tabp, int ryscols, int row_off, int nrows, int col_off,
                                              int ncols, const int bls[4], const int ls[4], int pos, bool raised,
                                              const double* W, double* buf[3], double* blk, const double ab[3],
                                              const double cd[3], double g[3], int lane, int T, unsigned tmask) {
   for (int q = lane; q < nrows * ncols; q += T) {
     const int r = q / ncols, c = q % ncols;
-    buf[0][q] = tabp[(size_t)(row_off + r) * tab_cols + col_off + c];
+    buf[0][q] = tabp[(size_t)(row_off + r) * ryscols + col_off + c];
   }
   __syncwarp(tmask);
   int cur = 0;
@@ -709,13 +704,13 @@ __device__ __forceinline__ void grad_dot_ct(const double* W, const double* blk, 
 }
 
 template <int L0, int L1, int L2, int L3, int POS, bool RAISED, int T>
-__device__ __forceinline__ void grad_shifted_ct(const double* tabp, int tab_cols, int row_off, int nrows, int col_off,
+__device__ __forceinline__ void grad_shifted_ct(const double* tabp, int ryscols, int row_off, int nrows, int col_off,
                                                 const double* W, double* buf[3], double* blk, const double ab[3],
                                                 const double cd[3], double g[3], int lane, unsigned tmask) {
   constexpr int NCOLS = nrange(L2, L2 + L3);
   for (int q = lane; q < nrows * NCOLS; q += T) {
     const int r = q / NCOLS, c = q - (q / NCOLS) * NCOLS;
-    buf[0][q] = tabp[(size_t)(row_off + r) * tab_cols + col_off + c];
+    buf[0][q] = tabp[(size_t)(row_off + r) * ryscols + col_off + c];
   }
   __syncwarp(tmask);
   int cur = 0;
@@ -773,8 +768,9 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
   using GS = GradShape<LA, LB, LC, LD, R>;
   constexpr int T = GS::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ R s_tab[GS::NR * RYS_MAX_SUB * 2 * RYS_NC];
-  stage_rys_table<GS::NR, R>(s_tab);
+  __shared__ __align__(16) R s_tab[rys_smem<GS::NR, R>(T)];
+  const R* rys = rys_staged<GS::NR, R>(T) ? s_tab : rys_global<GS::NR, R>();
+  stage_rys_table<GS::NR, R, T>(s_tab);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int team = tid / T;
   const int lane = threadIdx.x % T;
@@ -816,9 +812,9 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
       if (!sc.keep) continue;
       if (lane == 0) cnt.add(sc, pb, pk, A.fp32);
       if constexpr (T == 1)
-        grad_tables_thread<LA, LB, LC, LD, R>(A, s_tab, pb, pk, slot);
+        grad_tables_thread<LA, LB, LC, LD, R>(A, rys, pb, pk, slot);
       else
-        grad_team_passes<LA, LB, LC, LD, R, 0>(A, s_tab, pb, pk, sm, lane, tmask, slot);
+        grad_team_passes<LA, LB, LC, LD, R, 0>(A, rys, pb, pk, sm, lane, tmask, slot);
       __syncwarp(tmask);
       double g[9];
       if (A.kinds == 0)

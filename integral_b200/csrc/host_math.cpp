@@ -1,6 +1,6 @@
 // Host-side math of the plan: primitive normalisation, the Cartesian ->
-// real-solid-harmonic matrices, and the Rys Chebyshev tables the device
-// interpolates.  These are plan-construction steps (the reference also builds
+// real-solid-harmonic matrices, and the Rys polynomial tables the device
+// evaluates.  These are plan-construction steps (the reference also builds
 // its tables lazily at first use, src/math/boys.rs:122-136); no quartet is
 // evaluated here.
 #include "host_math.hpp"
@@ -135,9 +135,10 @@ std::vector<double> c2s_effective(int l) {
 //
 // Gauss quadrature for d mu(x) = x^{-1/2} exp(-T x) dx / 2 on [0,1] by the
 // discretised Stieltjes procedure on a 128-point Gauss-Legendre rule in
-// u = sqrt(x) plus Golub-Welsch, fitted per T-subinterval by degree-16
-// Chebyshev series (the method of src/math/rys.rs:230-515 and
-// xtask/src/gen_rys_tables.rs); above asymptotic_boundary(2n-1) the
+// u = sqrt(x) plus Golub-Welsch, fitted per unit interval of T by
+// polynomials through Chebyshev nodes (the quadrature is the method of
+// src/math/rys.rs:230-515 and xtask/src/gen_rys_tables.rs; the intervals and
+// the power basis are this build's); above asymptotic_boundary(2n-1) the
 // generalized Gauss-Laguerre(-1/2) nodes scaled by 1/T.
 
 namespace {
@@ -269,36 +270,27 @@ void finite_quadrature(const GL& gl, int n, double T, double* x, double* w) {
   gauss_from_jacobi(al, be, n, x, w);
 }
 
-double clenshaw(const double* c, double xi) {
-  double d = 0.0, dd = 0.0;
-  for (int k = RYS_NC - 1; k >= 1; --k) {
-    const double sv = d;
-    d = 2.0 * xi * d - dd + c[k];
-    dd = sv;
-  }
-  return xi * d - dd + 0.5 * c[0];
-}
-
-// degree-16 Chebyshev fits of the n roots and n weights on [a, b]:
-// out[(i*2 + {0,1}) * 17 + k]
-void fit(const GL& gl, int n, double a, double b, double* out) {
-  const int NC = RYS_NC;
-  double vx[RYS_NC][MAX_ROOTS], vw[RYS_NC][MAX_ROOTS];
-  for (int j = 0; j < NC; ++j) {
-    const double y = std::cos(PI * ((double)j + 0.5) / (double)NC);
-    finite_quadrature(gl, n, y * 0.5 * (b - a) + 0.5 * (b + a), vx[j], vw[j]);
-  }
-  for (int i = 0; i < n; ++i)
-    for (int k = 0; k < NC; ++k) {
-      double sx = 0.0, sw = 0.0;
-      for (int j = 0; j < NC; ++j) {
-        const double ck = std::cos(PI * (double)k * ((double)j + 0.5) / (double)NC);
-        sx += vx[j][i] * ck;
-        sw += vw[j][i] * ck;
-      }
-      out[(i * 2 + 0) * NC + k] = 2.0 / NC * sx;
-      out[(i * 2 + 1) * NC + k] = 2.0 / NC * sw;
+// Interpolating polynomial of degree nc - 1 through the values v[0..nc-1] at
+// the Chebyshev nodes node(j, nc), as coefficients of the powers of xi
+// (ascending): the Chebyshev sums by discrete orthogonality, expanded in long
+// double.  Their terms fall by 4^-k / k!, so the power basis on [-1, 1] is as
+// accurate as the Chebyshev one.
+double node(int j, int nc) { return std::cos(PI * ((double)j + 0.5) / (double)nc); }
+void power_fit(const double* v, int nc, double* out) {
+  long double mono[16] = {0}, t0[16] = {0}, t1[16] = {0}, t2[16];
+  t0[0] = 1.0L;  // T_k and T_{k-1} as powers
+  for (int k = 0; k < nc; ++k) {
+    long double s = 0.0L;
+    for (int j = 0; j < nc; ++j) s += (long double)v[j] * std::cos((long double)PI * k * (j + 0.5L) / nc);
+    s *= (k ? 2.0L : 1.0L) / nc;
+    for (int m = 0; m < nc; ++m) mono[m] += s * t0[m];
+    for (int m = 0; m < nc; ++m) t2[m] = (k == 0 ? 1.0L : 2.0L) * (m ? t0[m - 1] : 0.0L) - (k == 0 ? 0.0L : t1[m]);
+    for (int m = 0; m < nc; ++m) {
+      t1[m] = t0[m];
+      t0[m] = t2[m];
     }
+  }
+  for (int m = 0; m < nc; ++m) out[m] = (double)mono[m];
 }
 }  // namespace
 
@@ -307,40 +299,26 @@ const RysTables& rys_tables() {
   static std::once_flag once;
   std::call_once(once, [] {
     GL gl;
-    T.meta.assign(MAX_ROOTS + 1, RysMeta{0, 0, 0.0, 0.0});
-    std::vector<double> cell((size_t)MAX_ROOTS * 2 * RYS_NC);
+    constexpr int NC = rys_nc<double>(), NF = rys_nc<float>();
+    T.coef.assign(rys_off<double>(MAX_ROOTS + 1), 0.0);
+    T.coef_f.assign(rys_off<float>(MAX_ROOTS + 1), 0.0f);
     for (int n = 1; n <= MAX_ROOTS; ++n) {
-      const double t_hi = 33.0 + 2.5 * (double)(2 * n - 1);
-      // smallest equal-width subdivision whose fits stay within 2e-14
-      int n_sub = 1;
-      for (;; ++n_sub) {
-        const double width = t_hi / n_sub;
-        double worst = 0.0;
-        for (int s = 0; s < n_sub && worst <= 2e-14; ++s) {
-          const double a = s * width, b = a + width;
-          fit(gl, n, a, b, cell.data());
-          for (int j = 0; j < 33; ++j) {
-            const double t = a + (double)j / 32.0 * (b - a);
-            double rx[MAX_ROOTS], rw[MAX_ROOTS];
-            finite_quadrature(gl, n, t, rx, rw);
-            const double xi = (2.0 * t - (a + b)) / (b - a);
-            for (int i = 0; i < n; ++i) {
-              worst = std::max(worst, std::fabs(clenshaw(&cell[(i * 2) * RYS_NC], xi) - rx[i]));
-              worst = std::max(worst, std::fabs(clenshaw(&cell[(i * 2 + 1) * RYS_NC], xi) - rw[i]));
-            }
+      for (int s = 0; s < rys_nsub(n); ++s) {
+        double vx[NC][MAX_ROOTS], vw[NC][MAX_ROOTS];
+        for (int j = 0; j < NC; ++j) finite_quadrature(gl, n, s + 0.5 * (node(j, NC) + 1.0), vx[j], vw[j]);
+        for (int q = 0; q < 2 * n; ++q) {
+          double v[NC], vf[NF], c[NC], cf[NF];
+          for (int j = 0; j < NC; ++j) v[j] = q % 2 ? vw[j][q / 2] : vx[j][q / 2];
+          power_fit(v, NC, c);
+          // the FP32 polynomial through the FP64 one's values
+          for (int j = 0; j < NF; ++j) {
+            vf[j] = 0.0;
+            for (int m = NC - 1; m >= 0; --m) vf[j] = vf[j] * node(j, NF) + c[m];
           }
+          power_fit(vf, NF, cf);
+          std::copy(c, c + NC, &T.coef[rys_off<double>(n) + (size_t)s * rys_row<double>(n) + q * NC]);
+          std::copy(cf, cf + NF, &T.coef_f[rys_off<float>(n) + (size_t)s * rys_row<float>(n) + q * NF]);
         }
-        if (worst <= 2e-14 || n_sub >= 256) break;
-      }
-      RysMeta m;
-      m.n_sub = n_sub;
-      m.off = (int)T.coef.size();
-      m.width = t_hi / n_sub;
-      m.t_hi = t_hi;
-      T.meta[n] = m;
-      for (int s = 0; s < n_sub; ++s) {
-        fit(gl, n, s * m.width, s * m.width + m.width, cell.data());
-        T.coef.insert(T.coef.end(), cell.begin(), cell.begin() + (size_t)n * 2 * RYS_NC);
       }
       // generalized Gauss-Laguerre(-1/2): a_k = 2k + 1/2, b_k = k(k - 1/2), b_0 = sqrt(pi)
       double a[MAX_ROOTS], b[MAX_ROOTS];

@@ -14,8 +14,8 @@ std::vector<std::array<int, 3>> cart_comps(int l);
 std::vector<double> c2s_effective(int l);
 
 struct RysTables {
-  std::vector<RysMeta> meta;     // index n = 1..MAX_ROOTS
-  std::vector<double> coef;      // per n at meta[n].off: [(sub*n + i)*2 + {0,1}][17]
+  std::vector<double> coef;   // FP64 tables of n = 1..MAX_ROOTS (rys_off<double>, rys_row<double>)
+  std::vector<float> coef_f;  // FP32 tables
   double lag_x[MAX_ROOTS * MAX_ROOTS] = {0};
   double lag_w[MAX_ROOTS * MAX_ROOTS] = {0};
 };

@@ -4,13 +4,18 @@
 #include <cstddef>
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define IGPU_HD __host__ __device__
+#else
+#define IGPU_HD
+#endif
+
 namespace igpu {
 
 constexpr int MAX_L = 6;             // reference engine cap (src/engine/os.rs:34)
 constexpr int MAX_GRAD_L = MAX_L - 1;
 constexpr int GPU_MAX_L = 4;         // highest shell l with compiled quartet kernels
 constexpr int MAX_ROOTS = 13;
-constexpr int RYS_NC = 17;           // degree-16 Chebyshev series per root/weight
 constexpr int MAX_DENS = 64;
 constexpr int ADDR_TAB_DEG_HOST = 20;  // degrees of the device triple table
 
@@ -30,25 +35,30 @@ struct DevShell {
 // One primitive pair of a shell pair in evaluation orientation (first shell
 // A, second shell B, l_A >= l_B), surviving the 1e-32 pair screen of the
 // reference (src/engine/os_eri.rs:211-244).
-struct PrimPairD {
+// The quartet kernels form every per-quartet factor from products of these
+// and one rsqrt of zeta_bra + zeta_ket: no division per primitive quartet.
+struct alignas(16) PrimPairD {
   double zeta;       // alpha + beta
-  double alpha;      // exponent on A (gradient raise on A)
-  double beta;       // exponent on B
+  double inv2z;      // 1 / (2 zeta)
+  double ez;         // kappa * c_A * c_B (effective coefficients) * sqrt(2 pi^{5/2}) / zeta
   double px, py, pz; // Gaussian product centre
   double pax, pay, paz;  // P - A
-  double e;          // kappa * c_A * c_B (effective coefficients)
+  double alpha;      // exponent on A (gradient raise on A)
+  double beta;       // exponent on B
+  double pad;
 };
+// sqrt(2 pi^{5/2}): the product of two pairs' ez carries the Coulomb prefactor.
+constexpr double SQRT_TWO_PI_2_5 = 5.914967172795613;
 
 // FP32 copy of one primitive pair for the FP32 launches, rounded once at
 // plan creation: the FP32 header then needs no double loads or conversions.
 // P - Q of a quartet is formed as (A - C) + (PA - QC), with A - C (the
 // evaluation shells' centres) rounded once per quartet, so no absolute
 // coordinate enters an FP32 difference.
-struct PrimPairF {
-  float zeta, e;
+struct alignas(16) PrimPairF {
+  float zeta, inv2z, ez;
   float pax, pay, paz;
   float alpha, beta;
-  float pad;
 };
 
 // One canonical shell pair (i >= j in the reference's sense) with its
@@ -66,15 +76,30 @@ struct PairD {
   double q;       // Schwarz bound Q[i][j]
 };
 
-// Rys table metadata for n roots: finite branch T < t_hi uses n_sub equal
-// subintervals of width `width`; coefficients at `off` laid out as
-// [(sub*n + i)*2 + {0 root, 1 weight}][RYS_NC].
-struct RysMeta {
-  int n_sub;
-  int off;
-  double width;
-  double t_hi;
-};
+// Rys tables of the n-point quadrature: below rys_t_hi(n) the roots and
+// weights are polynomials on unit intervals of T, in xi = 2 (T - s) - 1 on
+// [s, s + 1] (exact in both precisions), 12 coefficients in FP64 (within
+// 3e-15 of the quadrature for every n) and 8 in FP32 (4e-11, below its
+// rounding), ascending.  Row s holds root 0, weight 0, root 1, ...; its stride
+// is an odd multiple of 16 bytes, so that the 16-byte reads of lanes in
+// different intervals start in different shared-memory banks.  Above it the
+// generalised Gauss-Laguerre limit holds.
+template <typename R>
+IGPU_HD constexpr int rys_nc() {
+  return sizeof(R) == 8 ? 12 : 8;
+}
+IGPU_HD constexpr double rys_t_hi(int n) { return 30.5 + 5.0 * n; }
+IGPU_HD constexpr int rys_nsub(int n) { return 31 + 5 * n; }
+template <typename R>
+IGPU_HD constexpr int rys_row(int n) {
+  return 2 * n * rys_nc<R>() + 16 / (int)sizeof(R);
+}
+template <typename R>
+IGPU_HD constexpr int rys_off(int n) {
+  int o = 0;
+  for (int k = 1; k < n; ++k) o += rys_nsub(k) * rys_row<R>(k);
+  return o;
+}
 
 // Task list of one class-pair launch: for each listed bra (position in the
 // bra class' Q-sorted pair list) kets 0..nket-1 of the ket class' sorted
@@ -92,12 +117,11 @@ struct TaskList {
 struct ConstData {
   const int* addr_lxyz;
   int n_addr;
-  const RysMeta* meta;   // MAX_ROOTS + 1 entries
   const double* lag_x;   // MAX_ROOTS x MAX_ROOTS
   const double* lag_w;
   const float* lag_xf;
   const float* lag_wf;
-  const double* tab;     // device Chebyshev tables
+  const double* tab;     // device Rys tables (rys_off, rys_row)
   const float* tab_f;
 };
 

@@ -33,10 +33,9 @@ int ensure_constants(int dev) {
   double* d_tab = nullptr;
   float* d_tab_f = nullptr;
   CK(cudaMalloc(&d_tab, T.coef.size() * sizeof(double)));
-  CK(cudaMalloc(&d_tab_f, T.coef.size() * sizeof(float)));
-  std::vector<float> tf(T.coef.begin(), T.coef.end());
+  CK(cudaMalloc(&d_tab_f, T.coef_f.size() * sizeof(float)));
   CK(cudaMemcpy(d_tab, T.coef.data(), T.coef.size() * sizeof(double), cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d_tab_f, tf.data(), tf.size() * sizeof(float), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(d_tab_f, T.coef_f.data(), T.coef_f.size() * sizeof(float), cudaMemcpyHostToDevice));
   float lxf[MAX_ROOTS * MAX_ROOTS], lwf[MAX_ROOTS * MAX_ROOTS];
   for (int i = 0; i < MAX_ROOTS * MAX_ROOTS; ++i) {
     lxf[i] = (float)T.lag_x[i];
@@ -45,7 +44,6 @@ int ensure_constants(int dev) {
   ConstData c;
   c.addr_lxyz = lxyz.data();
   c.n_addr = (int)lxyz.size();
-  c.meta = T.meta.data();
   c.lag_x = T.lag_x;
   c.lag_w = T.lag_w;
   c.lag_xf = lxf;
@@ -816,8 +814,8 @@ cudaError_t upload_prims(igpu_plan* P) {
   std::vector<PrimPairF> f(P->prims.size());
   for (size_t k = 0; k < f.size(); ++k) {
     const PrimPairD& d = P->prims[k];
-    f[k] = PrimPairF{(float)d.zeta, (float)d.e, (float)d.pax, (float)d.pay, (float)d.paz,
-                     (float)d.alpha, (float)d.beta, 0.f};
+    f[k] = PrimPairF{(float)d.zeta, (float)d.inv2z, (float)d.ez, (float)d.pax, (float)d.pay, (float)d.paz,
+                     (float)d.alpha, (float)d.beta};
   }
   cudaError_t e = P->d_prims.upload(P->prims, P->stream);
   if (e != cudaSuccess) return e;
@@ -973,7 +971,7 @@ int igpu_plan_create(const igpu_shell* sh, size_t nsh, int engine, igpu_plan** o
           q.pax = q.px - A.cx;
           q.pay = q.py - A.cy;
           q.paz = q.pz - A.cz;
-          q.e = kappa * ca * cb;
+          set_pair_factors(q, kappa * ca * cb);
           P->prims.push_back(q);
         }
       pr.nprim = (int)P->prims.size() - pr.prim_off;

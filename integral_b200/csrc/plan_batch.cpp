@@ -276,7 +276,7 @@ int igpu_batch_create(const igpu_shell* sh, const size_t* mol_nsh, size_t nmol, 
             q.pax = q.px - A.cx;
             q.pay = q.py - A.cy;
             q.paz = q.pz - A.cz;
-            q.e = kappa * ca * cb;
+            set_pair_factors(q, kappa * ca * cb);
             P->prims.push_back(q);
           }
         pr.nprim = (int)P->prims.size() - pr.prim_off;

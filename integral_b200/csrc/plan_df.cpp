@@ -108,7 +108,7 @@ int igpu_plan_attach_aux(igpu_plan* P, const igpu_shell* aux, size_t naux_sh) {
       q.px = a.cx;
       q.py = a.cy;
       q.pz = a.cz;
-      q.e = ca;
+      set_pair_factors(q, ca);
       P->prims.push_back(q);
     }
     pr.nprim = (int)P->prims.size() - pr.prim_off;

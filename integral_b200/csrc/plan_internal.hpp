@@ -52,6 +52,13 @@ inline int pc_la_host(int pc) {
   return la;
 }
 
+// The factors of a primitive pair that the kernels multiply, from its zeta
+// and its prefactor e = kappa * c_A * c_B.
+inline void set_pair_factors(PrimPairD& q, double e) {
+  q.inv2z = 0.5 / q.zeta;
+  q.ez = e * SQRT_TWO_PI_2_5 / q.zeta;
+}
+
 template <typename T>
 struct DevBuf {
   T* p = nullptr;

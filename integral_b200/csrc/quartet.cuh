@@ -16,7 +16,7 @@
 //               per-axis tables are built cooperatively in shared memory and
 //               every lane accumulates its own rows e of G (register tiles
 //               of FCH columns, the f range walked in chunks).
-// The class's Rys Chebyshev table is staged in shared memory per block.
+// The class's Rys table is staged in shared memory where rys_staged says so.
 // Phase 2 (post.cuh) runs the horizontal recurrences, the Cartesian ->
 // spherical transform and the mode-specific consumer on the team.
 #pragma once
@@ -67,7 +67,11 @@ struct TeamShape {
   // Primitive quartets set up per round: as many as fit a shared-memory
   // budget of 48 KB per 128-thread block (power of two, at most T).
   static constexpr int GTAB = (S::NE + 1) * (S::NF + 1);
-  static constexpr int PRIM_TAB = 2 * S::NR + 3 * S::NR * GTAB;  // x, w, g[3][NR][GTAB]
+  // x, w, g[3][NR][GTAB] of one primitive quartet, an odd number of values:
+  // the lanes that build different quartets' tables store at this stride, and
+  // an even one shares few banks (it was 96 for (22|10): every lane of a store
+  // in one bank)
+  static constexpr int PRIM_TAB = (2 * S::NR + 3 * S::NR * GTAB) | 1;
   static constexpr int BUDGET = (48 * 1024 / 128) * (T == 1 ? 1 : T) / (int)sizeof(R);
   static constexpr int BP0 = BUDGET / PRIM_TAB;
   static constexpr int BP = BP0 >= T ? T : (BP0 >= 16 ? 16 : (BP0 >= 8 ? 8 : (BP0 >= 4 ? 4 : (BP0 >= 2 ? 2 : 1))));
@@ -89,7 +93,7 @@ struct TeamShape {
 // and Boys value is <= 1); evaluated in FP32 for the primitive screen of the
 // FP32 launches.
 __device__ __forceinline__ float prim_bound(const PrimPairF& b, const PrimPairF& k) {
-  return fabsf(b.e * k.e) * (34.98683665f / (b.zeta * k.zeta * sqrtf(b.zeta + k.zeta)));
+  return fabsf(b.ez * k.ez) * rsqrtf(b.zeta + k.zeta);
 }
 
 // Largest primitive-quartet count the team screen compacts (16 x 16 primitive
@@ -99,7 +103,7 @@ constexpr int MAX_SURV = 256;
 // ------------------------------------------------------------- TEAM == 1
 
 template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* s_tab, const PairD& pb,
+__device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* tab, const PairD& pb,
                                                   const PairD& pk, R (&G)[ClassShape<LA, LB, LC, LD>::NG]) {
   using S = ClassShape<LA, LB, LC, LD>;
   constexpr int NE = S::NE, NF = S::NF, NR = S::NR;
@@ -134,26 +138,23 @@ __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* 
 #pragma unroll
           for (int r = 0; r < NR; ++r) {
             double xd, wd;
-            rys_root_fp64<NR>(T64, r, xd, wd);
+            rys_root_one<NR, true>(rys_global<NR, double>(), T64, r, xd, wd);
             x[r] = R(xd);
             w[r] = R(wd);
           }
         } else {
-          rys_roots_s<NR, R>(s_tab, h.T, x, w);
+          rys_roots_s<NR, !rys_staged<NR, R>(1)>(tab, h.T, x, w);
         }
       } else {
-        rys_roots_s<NR, R>(s_tab, h.T, x, w);
+        rys_roots_s<NR, !rys_staged<NR, R>(1)>(tab, h.T, x, w);
       }
-      const R inv_pq = R(1) / h.pq;
-      const R qpq = h.q * inv_pq, ppq = h.p * inv_pq;
-      const R inv2pq = R(0.5) * inv_pq, inv2p = R(0.5) / h.p, inv2q = R(0.5) / h.q;
 #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const R xr = x[r] * h.xs;
-        const R b00 = xr * inv2pq;
-        const R b10 = (R(1) - xr * qpq) * inv2p;
-        const R b01 = (R(1) - xr * ppq) * inv2q;
-        const R cq = xr * qpq, cp = xr * ppq;
+        const R cq = xr * h.qpq, cp = xr * h.ppq;
+        const R b00 = xr * h.hpq;
+        const R b10 = (R(1) - cq) * h.inv2p;
+        const R b01 = (R(1) - cp) * h.inv2q;
         R gx[NE + 1][NF + 1], gy[NE + 1][NF + 1], gz[NE + 1][NF + 1];
         vrr_axis<NE, NF, R>(R(1), h.pax - cq * h.pqx, h.qcx + cp * h.pqx, b10, b01, b00, gx);
         vrr_axis<NE, NF, R>(R(1), h.pay - cq * h.pqy, h.qcy + cp * h.pqy, b10, b01, b00, gy);
@@ -176,35 +177,10 @@ __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* 
 
 // --------------------------------------------------------------- TEAM > 1
 
-// Root r of the N-point quadrature from the shared-memory table.
-template <int N, typename R>
-__device__ __forceinline__ void rys_root_one(const R* s_tab, R T, int r, R& x, R& w) {
-  const RysMeta m = c_rys[N];
-  if (T >= R(m.t_hi)) {
-    if constexpr (sizeof(R) == 8) {
-      x = c_lag_x[N - 1][r] / T;
-      w = c_lag_w[N - 1][r] * R(0.5) * rsqrt(T);
-    } else {
-      x = c_lag_xf[N - 1][r] / T;
-      w = c_lag_wf[N - 1][r] * R(0.5) * rsqrt(T);
-    }
-    return;
-  }
-  R width = R(m.width);
-  int s = (int)(T / width);
-  s = s < 0 ? 0 : (s >= m.n_sub ? m.n_sub - 1 : s);
-  R a = R(s) * width;
-  R b = a + width;
-  R xi = (R(2) * T - (a + b)) / (b - a);
-  const R* base = s_tab + ((size_t)s * N + r) * 2 * RYS_NC;
-  x = chebev_s<R>(base, xi);
-  w = chebev_s<R>(base + RYS_NC, xi);
-}
-
 // One pass over all primitive quartets accumulating the columns
 // [F0, F0 + FCH) of this lane's rows.
 template <int LA, int LB, int LC, int LD, typename R, int F0>
-__device__ __forceinline__ void team_pass(const KernelArgs& A, const R* s_tab, const PairD& pb, const PairD& pk,
+__device__ __forceinline__ void team_pass(const KernelArgs& A, const R* tab, const PairD& pb, const PairD& pk,
                                           R* sm, int lane, unsigned tmask, double* G, const unsigned short* surv,
                                           int npr, bool g32) {
   using S = ClassShape<LA, LB, LC, LD>;
@@ -261,11 +237,11 @@ __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* s_tab, c
         R xr, wr;
         if (r64) {
           double xd, wd;
-          rys_root_fp64<NR>(T64, r, xd, wd);
+          rys_root_one<NR, true>(rys_global<NR, double>(), T64, r, xd, wd);
           xr = R(xd);
           wr = R(wd);
         } else {
-          rys_root_one<NR, R>(s_tab, h.T, r, xr, wr);
+          rys_root_one<NR, !rys_staged<NR, R>(T)>(tab, h.T, r, xr, wr);
         }
         mys[r] = xr * h.xs;
         mys[NR + r] = wr * h.pref;
@@ -273,21 +249,18 @@ __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* s_tab, c
     }
     __syncwarp(tmask);
     if (active) {
-      const R inv_pq = R(1) / h.pq;
-      const R qpq = h.q * inv_pq, ppq = h.p * inv_pq;
-      const R inv2p = R(0.5) / h.p, inv2q = R(0.5) / h.q;
       for (int t = sub; t < 3 * NR; t += SUB) {
         const int axis = t / NR, r = t - axis * NR;
         const R xr = mys[r];
-        const R b00 = xr * R(0.5) * inv_pq;
-        const R b10 = (R(1) - xr * qpq) * inv2p;
-        const R b01 = (R(1) - xr * ppq) * inv2q;
+        const R cq = xr * h.qpq, cp = xr * h.ppq;
+        const R b00 = xr * h.hpq;
+        const R b10 = (R(1) - cq) * h.inv2p;
+        const R b01 = (R(1) - cp) * h.inv2q;
         const R pqa = axis == 0 ? h.pqx : (axis == 1 ? h.pqy : h.pqz);
         const R paa = axis == 0 ? h.pax : (axis == 1 ? h.pay : h.paz);
         const R qca = axis == 0 ? h.qcx : (axis == 1 ? h.qcy : h.qcz);
         R g[NE + 1][NF + 1];
-        vrr_axis<NE, NF, R>(axis == 2 ? mys[NR + r] : R(1), paa - xr * qpq * pqa, qca + xr * ppq * pqa, b10, b01,
-                            b00, g);
+        vrr_axis<NE, NF, R>(axis == 2 ? mys[NR + r] : R(1), paa - cq * pqa, qca + cp * pqa, b10, b01, b00, g);
         R* dst = mys + 2 * NR + (axis * NR + r) * GT;
 #pragma unroll
         for (int n = 0; n <= NE; ++n)
@@ -341,14 +314,14 @@ __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* s_tab, c
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int C>
-__device__ __forceinline__ void team_chunks(const KernelArgs& A, const R* s_tab, const PairD& pb, const PairD& pk,
+__device__ __forceinline__ void team_chunks(const KernelArgs& A, const R* tab, const PairD& pb, const PairD& pk,
                                             R* sm, int lane, unsigned tmask, double* G, const unsigned short* surv,
                                             int npr, bool g32) {
   using TS = TeamShape<LA, LB, LC, LD, R>;
   if constexpr (C < TS::NCHUNK) {
-    team_pass<LA, LB, LC, LD, R, C * TS::FCH>(A, s_tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
+    team_pass<LA, LB, LC, LD, R, C * TS::FCH>(A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
     __syncwarp(tmask);
-    team_chunks<LA, LB, LC, LD, R, C + 1>(A, s_tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
+    team_chunks<LA, LB, LC, LD, R, C + 1>(A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
   }
 }
 
@@ -399,7 +372,7 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
   using TS = TeamShape<LA, LB, LC, LD, R>;
   constexpr int T = TS::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ R s_tab[S::NR * RYS_MAX_SUB * 2 * RYS_NC];
+  __shared__ __align__(16) R s_tab[rys_smem<S::NR, R>(T)];
   constexpr bool SCREEN = sizeof(R) == 4 && T > 1;
   __shared__ unsigned short s_surv[SCREEN ? (128 / T) * MAX_SURV : 1];
   constexpr bool CT_POST = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 10000;
@@ -409,7 +382,8 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
     build_hrr_tab<LA, LB, LC, LD>(s_hrr);
     stage_c2s<LA, LB, LC, LD, R>(A, s_c2s);
   }
-  stage_rys_table<S::NR, R>(s_tab);  // its __syncthreads also publishes s_hrr, s_c2s
+  const R* tab = rys_staged<S::NR, R>(T) ? s_tab : rys_global<S::NR, R>();
+  stage_rys_table<S::NR, R, T>(s_tab);  // its __syncthreads also publishes s_hrr, s_c2s
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int team = tid / T;
   const int lane = threadIdx.x % T;
@@ -457,7 +431,7 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
       if (lane == 0) cnt.add(sc, pb, pk, A.fp32);
       if constexpr (T == 1) {
         R G[S::NG];
-        accumulate_thread<LA, LB, LC, LD, R>(A, s_tab, pb, pk, G);
+        accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, G);
         if (use_acc && A.kinds != 2) {
           // the post phase runs in the launch's arithmetic (FP32 launches
           // read the FP32 densities); J/K accumulate in FP64
@@ -480,7 +454,7 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
             if (npr == 0) continue;  // the whole quartet is below the screen
           }
         }
-        team_chunks<LA, LB, LC, LD, R, 0>(A, s_tab, pb, pk, sm, lane, tmask, slot, surv, npr,
+        team_chunks<LA, LB, LC, LD, R, 0>(A, tab, pb, pk, sm, lane, tmask, slot, surv, npr,
                                           CT_POST && use_acc && A.kinds != 2);
       }
       __syncwarp(tmask);
