@@ -19,7 +19,8 @@
 //   A  2*alpha_A      e in [la+1, la+lb+1] f in [lc, lc+ld]
 //   B  2*alpha_B      e in [la, la+lb+1]   f in [lc, lc+ld]
 //   C  2*alpha_C      e in [la, la+lb]     f in [lc+1, lc+ld+1]
-// (A and B share their rows: one product feeds both).  Phase 2 runs the
+// (one product of the 2D integrals feeds every table that has its row and
+// column).  Phase 2 runs the
 // horizontal recurrences of the six shifted blocks from these tables and
 // dots each with W, so the gradient is the adjoint of the value path with
 // the intermediates recomputed instead of kept.
@@ -90,76 +91,103 @@ __host__ __device__ inline GradSlot grad_slot_layout(int la, int lb, int lc, int
   return L;
 }
 
-// Lanes per quartet: one thread while all accumulators fit in registers,
-// else the smallest team of 8, 16 or 32 lanes giving each lane at most one
-// row of every segment (32 beyond that).  Measured against at most two rows
-// per lane: fewer columns per lane means fewer passes, each of which
-// recomputes the 2D tables of every primitive quartet.
-__host__ __device__ constexpr int grad_team_for(int la, int lb, int lc, int ld) {
-  if (g_acc_total(la, lb, lc, ld) <= 40) return 1;
-  int mr = 0;
-  for (int s = 0; s < 3; ++s)
-    if (g_nacc(la, lb, lc, ld, s) > 0 && g_rows(la, lb, lc, ld, s) > mr) mr = g_rows(la, lb, lc, ld, s);
-  for (int t = 8; t < 32; t *= 2)
-    if ((mr + t - 1) / t <= 1) return t;
-  return 32;
+// Main rows of the team sweep: e of degree la .. la+lb+1, one per lane and
+// row slot, each with every column f of degree max(lc-1, 0) .. lc+ld+1.  A
+// lane loads the 3 (NFV + 1) axis values of its row once per primitive
+// quartet and root and forms each product once for all the tables that take
+// it: the loads, not the arithmetic, bound the sweep (a warp's FP64 shared
+// load takes four times its fused multiply-add), and the tables' own row
+// sets, swept one after another, loaded them up to three times.  The rows of
+// degree la-1 that the lowered A block alone needs go one element a lane.
+__host__ __device__ constexpr int g_main_rows(int la, int lb) { return nrange(la, la + lb + 1); }
+__host__ __device__ constexpr int g_col_lo(int lc) { return lc > 0 ? lc - 1 : 0; }
+__host__ __device__ constexpr int g_main_cols(int lc, int ld) { return nrange(g_col_lo(lc), lc + ld + 1); }
+// which tables column degree df of a main row feeds
+__host__ __device__ constexpr bool g_feeds_p(int, int lb, int lc, int ld, int df) {
+  return (lc > 0 && df <= lc + ld - 1) || (lb > 0 && df >= lc && df <= lc + ld);
+}
+__host__ __device__ constexpr bool g_feeds_ab(int lc, int ld, int df) { return df >= lc && df <= lc + ld; }
+__host__ __device__ constexpr bool g_feeds_c(int lc, int, int df) { return df >= lc + 1; }
+__host__ __device__ constexpr int g_col_acc(int la, int lb, int lc, int ld, int df) {
+  return (g_feeds_p(la, lb, lc, ld, df) ? 1 : 0) + (g_feeds_ab(lc, ld, df) ? 2 : 0) + (g_feeds_c(lc, ld, df) ? 1 : 0);
+}
+// accumulators of the columns before column c
+__host__ __device__ constexpr int g_acc_before(int la, int lb, int lc, int ld, int c) {
+  int n = 0;
+  for (int k = 0; k < c; ++k) n += g_col_acc(la, lb, lc, ld, range_deg(g_col_lo(lc), k));
+  return n;
+}
+__host__ __device__ constexpr int g_low_elems(int la, int lc, int ld) {
+  return la > 0 ? ncart(la - 1) * nrange(lc, lc + ld) : 0;
 }
 
-// Compile-time plan of the team sweep: items = (segment, column chunk);
-// consecutive items are packed into passes of at most BUD accumulators per
-// lane.  Every pass recomputes the Rys 2D tables of all primitive quartets.
-constexpr int GPLAN_MAX = 96;
+// Passes of the sweep: `rows` row slots and a run of columns each, at most
+// `bud` accumulators a lane where one row slot and one column allow it.  Every
+// pass recomputes the 2D tables, so rows are split first (a row's loads then
+// stay in one pass), columns only when one row slot exceeds the budget.
+constexpr int GPLAN_MAX = 256;
 struct GradPassPlan {
-  int nitems;
-  int seg[GPLAN_MAX], f0[GPLAN_MAX], fw[GPLAN_MAX], off[GPLAN_MAX], rslot[GPLAN_MAX];
   int npass;
-  int pbeg[GPLAN_MAX + 1];
-  int pacc[GPLAN_MAX];
-  int prows[GPLAN_MAX];
+  int rows;                 // row slots per pass
+  int slot[GPLAN_MAX];      // first row slot of the pass
+  int c0[GPLAN_MAX], c1[GPLAN_MAX];
 };
 __host__ __device__ constexpr GradPassPlan make_grad_plan(int la, int lb, int lc, int ld, int T, int bud) {
   GradPassPlan p{};
-  int n = 0;
-  for (int s = 0; s < 3; ++s) {
-    const int na = g_nacc(la, lb, lc, ld, s);
-    if (na == 0) continue;
-    const int rl = (g_rows(la, lb, lc, ld, s) + T - 1) / T;
-    const int cols = g_cols(la, lb, lc, ld, s);
-    int fch = bud / (rl * na);
-    fch = fch < 1 ? 1 : (fch > cols ? cols : fch);
-    for (int f0 = 0; f0 < cols; f0 += fch) {
-      p.seg[n] = s;
-      p.f0[n] = f0;
-      p.fw[n] = cols - f0 < fch ? cols - f0 : fch;
-      ++n;
+  const int rl = (g_main_rows(la, lb) + T - 1) / T;
+  const int cols = g_main_cols(lc, ld);
+  const int ca = g_acc_before(la, lb, lc, ld, cols);
+  if (ca <= bud) {
+    int rp = bud / ca < rl ? bud / ca : rl;
+    const int np = (rl + rp - 1) / rp;
+    rp = (rl + np - 1) / np;
+    p.rows = rp;
+    for (int s = 0; s < rl; s += rp) {
+      p.slot[p.npass] = s;
+      p.c0[p.npass] = 0;
+      p.c1[p.npass] = cols;
+      ++p.npass;
     }
+    return p;
   }
-  p.nitems = n;
-  int np = 0, cur = 0, rows = 0;
-  p.pbeg[0] = 0;
-  for (int i = 0; i < n; ++i) {
-    const int s = p.seg[i];
-    const int rl = (g_rows(la, lb, lc, ld, s) + T - 1) / T;
-    const int acc = rl * p.fw[i] * g_nacc(la, lb, lc, ld, s);
-    if (cur > 0 && cur + acc > bud) {
-      p.pacc[np] = cur;
-      p.prows[np] = rows;
-      ++np;
-      p.pbeg[np] = i;
-      cur = 0;
-      rows = 0;
+  p.rows = 1;
+  for (int s = 0; s < rl; ++s)
+    for (int c = 0; c < cols;) {
+      int e = c, acc = 0;
+      while (e < cols && (e == c || acc + g_col_acc(la, lb, lc, ld, range_deg(g_col_lo(lc), e)) <= bud)) {
+        acc += g_col_acc(la, lb, lc, ld, range_deg(g_col_lo(lc), e));
+        ++e;
+      }
+      p.slot[p.npass] = s;
+      p.c0[p.npass] = c;
+      p.c1[p.npass] = e;
+      ++p.npass;
+      c = e;
     }
-    p.off[i] = cur;
-    p.rslot[i] = rows;
-    cur += acc;
-    rows += rl;
-  }
-  p.pacc[np] = cur;
-  p.prows[np] = rows;
-  ++np;
-  p.pbeg[np] = n;
-  p.npass = np;
   return p;
+}
+
+// Lanes per quartet: one thread while all accumulators fit in registers,
+// else the team of 8, 16 or 32 lanes with the least lane time per root by a
+// count of issue slots: the 2D tables of each pass (recurrences and their
+// shared-memory stores) and, per row slot, the row's loads and the columns'
+// products and sums, idle lanes of the last row slot included.
+__host__ __device__ constexpr int grad_team_for(int la, int lb, int lc, int ld) {
+  if (g_acc_total(la, lb, lc, ld) <= 40) return 1;
+  const int nev = la + lb + 1, nfv = lc + ld + 1;
+  int best = 32, cost = 1 << 30;
+  for (int t = 32; t >= 8; t /= 2) {
+    const int rl = (g_main_rows(la, lb) + t - 1) / t;
+    const GradPassPlan p = make_grad_plan(la, lb, lc, ld, t, 80);
+    const int cols = g_main_cols(lc, ld);
+    const int c = p.npass * 12 * (nev + 1) * (nfv + 1) +
+                  rl * t * (6 * (nfv + 1) + cols + g_acc_before(la, lb, lc, ld, cols) / 2);
+    if (c < cost) {
+      cost = c;
+      best = t;
+    }
+  }
+  return best;
 }
 
 template <int LA, int LB, int LC, int LD, typename R>
@@ -169,7 +197,7 @@ struct GradShape {
   static constexpr int NR = (NE + NF + 1) / 2 + 1;
   static constexpr bool LOW = g_low(LA, LC);
   static constexpr int T = grad_team_for(LA, LB, LC, LD);
-  // accumulators per lane per pass (measured: 80/112 beat 48/72 and 64/96)
+  // accumulators per lane per pass
   static constexpr int BUD = sizeof(R) == 8 ? 80 : 112;
   static constexpr GradPassPlan PL = make_grad_plan(LA, LB, LC, LD, T, BUD);
   static constexpr int GT = (NEV + 1) * (NFV + 1);
@@ -281,27 +309,40 @@ __device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* rys
                                                R* sm, int lane, unsigned tmask, double* tab) {
   using GS = GradShape<LA, LB, LC, LD, R>;
   constexpr int NEV = GS::NEV, NFV = GS::NFV, NR = GS::NR, T = GS::T, GT = GS::GT;
-  constexpr int I0 = GS::PL.pbeg[PASS], I1 = GS::PL.pbeg[PASS + 1];
-  constexpr int NACC = GS::PL.pacc[PASS], NROW = GS::PL.prows[PASS];
-  R acc[NACC];
+  constexpr int ROWS = g_main_rows(LA, LB), RL = (ROWS + T - 1) / T;
+  constexpr int S0 = GS::PL.slot[PASS];
+  constexpr int NS = RL - S0 < GS::PL.rows ? RL - S0 : GS::PL.rows;
+  constexpr int C0 = GS::PL.c0[PASS], C1 = GS::PL.c1[PASS];
+  constexpr int A0 = g_acc_before(LA, LB, LC, LD, C0);
+  constexpr int CA = g_acc_before(LA, LB, LC, LD, C1) - A0;
+  constexpr int CLO = g_col_lo(LC);
+  // the last pass also takes the elements of degree la-1
+  constexpr int NLOW = PASS + 1 == GS::PL.npass ? g_low_elems(LA, LC, LD) : 0;
+  constexpr int XS = (NLOW + T - 1) / T, XCOLS = nrange(LC, LC + LD);
+  R acc[NS * CA], low[XS > 0 ? XS : 1];
 #pragma unroll
-  for (int q = 0; q < NACC; ++q) acc[q] = R(0);
-  // row offsets into the per-axis tables: e components of every row slot
-  int ox[NROW], oy[NROW], oz[NROW];
-  static_for<I1 - I0>([&](auto ii) {
-    constexpr int I = I0 + decltype(ii)::value;
-    constexpr int s = GS::PL.seg[I];
-    constexpr int EA = g_ea(LA, LB, LC, LD, s), ROWS = g_rows(LA, LB, LC, LD, s);
-    constexpr int RL = (ROWS + T - 1) / T, RS = GS::PL.rslot[I];
+  for (int q = 0; q < NS * CA; ++q) acc[q] = R(0);
 #pragma unroll
-    for (int k = 0; k < RL; ++k) {
-      const int row = lane + T * k;
-      const int a = tri_below(EA) + (row < ROWS ? row : 0);
-      ox[RS + k] = addr_lx(a) * (NFV + 1);
-      oy[RS + k] = addr_ly(a) * (NFV + 1);
-      oz[RS + k] = addr_lz(a) * (NFV + 1);
-    }
-  });
+  for (int q = 0; q < (XS > 0 ? XS : 1); ++q) low[q] = R(0);
+  // row offsets into the per-axis tables (lanes beyond the rows sum row 0,
+  // which is not stored)
+  int ox[NS], oy[NS], oz[NS];
+#pragma unroll
+  for (int k = 0; k < NS; ++k) {
+    const int row = lane + T * (S0 + k);
+    const int a = tri_below(LA) + (row < ROWS ? row : 0);
+    ox[k] = addr_lx(a) * (NFV + 1);
+    oy[k] = addr_ly(a) * (NFV + 1);
+    oz[k] = addr_lz(a) * (NFV + 1);
+  }
+  int xo[XS > 0 ? XS : 1];  // packed element offsets, 10 bits an axis
+#pragma unroll
+  for (int q = 0; q < XS; ++q) {
+    const int el = lane + T * q < NLOW ? lane + T * q : 0;
+    const int e = tri_below(LA > 0 ? LA - 1 : 0) + el / XCOLS, f = tri_below(LC) + el % XCOLS;
+    xo[q] = (addr_lx(e) * (NFV + 1) + addr_lx(f)) | (addr_ly(e) * (NFV + 1) + addr_ly(f)) << 10 |
+            (addr_lz(e) * (NFV + 1) + addr_lz(f)) << 20;
+  }
   constexpr int BP = GS::BP, SUB = GS::SUB, PT = GS::PRIM_TAB;
   const int npk = pk.nprim;
   const int npr = pb.nprim * npk;
@@ -361,66 +402,66 @@ __device__ __forceinline__ void grad_team_pass(const KernelArgs& A, const R* rys
         const R* tx = gt + (0 * NR + r) * GT;
         const R* ty = gt + (1 * NR + r) * GT;
         const R* tz = gt + (2 * NR + r) * GT;
-        static_for<I1 - I0>([&](auto ii) {
-          constexpr int I = I0 + decltype(ii)::value;
-          constexpr int s = GS::PL.seg[I], FF = GS::PL.f0[I], FW = GS::PL.fw[I], OFF = GS::PL.off[I];
-          constexpr int FA = g_fa(LA, LB, LC, LD, s), ROWS = g_rows(LA, LB, LC, LD, s);
-          constexpr int RL = (ROWS + T - 1) / T, RS = GS::PL.rslot[I];
 #pragma unroll
-          for (int k = 0; k < RL; ++k) {
-            if (RL * T > ROWS && lane + T * k >= ROWS) continue;
-            R rx[NFV + 1], ry[NFV + 1], rz[NFV + 1];
+        for (int k = 0; k < NS; ++k) {
+          R rx[NFV + 1], ry[NFV + 1], rz[NFV + 1];
 #pragma unroll
-            for (int m = 0; m <= NFV; ++m) {
-              rx[m] = tx[ox[RS + k] + m];
-              ry[m] = ty[oy[RS + k] + m];
-              rz[m] = tz[oz[RS + k] + m];
-            }
-            if constexpr (s == 2) {
-#pragma unroll
-              for (int m = 0; m <= NFV; ++m) rz[m] *= wC;
-            }
-            static_for<FW>([&](auto f) {
-              constexpr int fi = FF + decltype(f)::value;
-              constexpr int fx = range_x(FA, fi), fy = range_y(FA, fi), fz = range_z(FA, fi);
-              const R v = rx[fx] * ry[fy] * rz[fz];
-              if constexpr (s == 1) {
-                acc[OFF + (k * FW + decltype(f)::value) * 2] += wA * v;
-                acc[OFF + (k * FW + decltype(f)::value) * 2 + 1] += wB * v;
-              } else {
-                acc[OFF + k * FW + decltype(f)::value] += v;
-              }
-            });
+          for (int m = 0; m <= NFV; ++m) {
+            rx[m] = tx[ox[k] + m];
+            ry[m] = ty[oy[k] + m];
+            rz[m] = tz[oz[k] + m];
           }
-        });
+          static_for<C1 - C0>([&](auto c) {
+            constexpr int ci = C0 + decltype(c)::value;
+            constexpr int df = range_deg(CLO, ci);
+            constexpr int fx = range_x(CLO, ci), fy = range_y(CLO, ci), fz = range_z(CLO, ci);
+            constexpr bool P = g_feeds_p(LA, LB, LC, LD, df), AB = g_feeds_ab(LC, LD, df);
+            constexpr int o = g_acc_before(LA, LB, LC, LD, ci) - A0;
+            const R v = rx[fx] * ry[fy] * rz[fz];
+            R* q = acc + k * CA + o;
+            if constexpr (P) q[0] += v;
+            if constexpr (AB) {
+              q[P] += wA * v;
+              q[P + 1] += wB * v;
+            }
+            if constexpr (g_feeds_c(LC, LD, df)) q[P + 2 * AB] += wC * v;
+          });
+        }
+#pragma unroll
+        for (int q = 0; q < XS; ++q) low[q] += tx[xo[q] & 1023] * ty[xo[q] >> 10 & 1023] * tz[xo[q] >> 20];
       }
     }
     __syncwarp(tmask);
   }
   const GradSlot L = grad_slot_layout(LA, LB, LC, LD);
-  static_for<I1 - I0>([&](auto ii) {
-    constexpr int I = I0 + decltype(ii)::value;
-    constexpr int s = GS::PL.seg[I], FF = GS::PL.f0[I], FW = GS::PL.fw[I], OFF = GS::PL.off[I];
-    constexpr int ROWS = g_rows(LA, LB, LC, LD, s), COLS = g_cols(LA, LB, LC, LD, s);
-    constexpr int RL = (ROWS + T - 1) / T;
+  constexpr int COLSP = g_cols(LA, LB, LC, LD, 0), COLS1 = g_cols(LA, LB, LC, LD, 1), COLS2 = g_cols(LA, LB, LC, LD, 2);
+  constexpr int ROWP0 = tri_below(LA) - tri_below(g_ea(LA, LB, LC, LD, 0));  // P rows before degree la
+  constexpr int F1 = tri_below(LC) - tri_below(CLO), F2 = tri_below(LC + 1) - tri_below(CLO);
 #pragma unroll
-    for (int k = 0; k < RL; ++k) {
-      const int row = lane + T * k;
-      if (row >= ROWS) continue;
-#pragma unroll
-      for (int f = 0; f < FW; ++f) {
-        if constexpr (s == 0) {
-          tab[L.off_p + (size_t)row * COLS + FF + f] = (double)acc[OFF + k * FW + f];
-        } else if constexpr (s == 1) {
-          tab[L.off_b + (size_t)row * COLS + FF + f] = (double)acc[OFF + (k * FW + f) * 2 + 1];
-          if (row >= ncart(LA))
-            tab[L.off_a + (size_t)(row - ncart(LA)) * COLS + FF + f] = (double)acc[OFF + (k * FW + f) * 2];
-        } else {
-          tab[L.off_c + (size_t)row * COLS + FF + f] = (double)acc[OFF + k * FW + f];
-        }
+  for (int k = 0; k < NS; ++k) {
+    const int row = lane + T * (S0 + k);
+    if (row >= ROWS) continue;
+    static_for<C1 - C0>([&](auto c) {
+      constexpr int ci = C0 + decltype(c)::value;
+      constexpr int df = range_deg(CLO, ci);
+      constexpr bool P = g_feeds_p(LA, LB, LC, LD, df), AB = g_feeds_ab(LC, LD, df);
+      constexpr int o = g_acc_before(LA, LB, LC, LD, ci) - A0;
+      const R* q = acc + k * CA + o;
+      if constexpr (P)
+        if (row < nrange(LA, LA + LB)) tab[L.off_p + (size_t)(ROWP0 + row) * COLSP + ci] = (double)q[0];
+      if constexpr (AB) {
+        tab[L.off_b + (size_t)row * COLS1 + ci - F1] = (double)q[P + 1];
+        if (row >= ncart(LA)) tab[L.off_a + (size_t)(row - ncart(LA)) * COLS1 + ci - F1] = (double)q[P];
       }
-    }
-  });
+      if constexpr (g_feeds_c(LC, LD, df))
+        if (row < nrange(LA, LA + LB)) tab[L.off_c + (size_t)row * COLS2 + ci - F2] = (double)q[P + 2 * AB];
+    });
+  }
+#pragma unroll
+  for (int q = 0; q < XS; ++q) {
+    const int el = lane + T * q;
+    if (el < NLOW) tab[L.off_p + (size_t)(el / XCOLS) * COLSP + F1 + el % XCOLS] = (double)low[q];
+  }
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int PASS>
@@ -703,62 +744,92 @@ __device__ __forceinline__ void grad_dot_ct(const double* W, const double* blk, 
   }
 }
 
-template <int L0, int L1, int L2, int L3, int POS, bool RAISED, int T>
-__device__ __forceinline__ void grad_shifted_ct(const double* tabp, int ryscols, int row_off, int nrows, int col_off,
-                                                const double* W, double* buf[3], double* blk, const double ab[3],
-                                                const double cd[3], double g[3], int lane, unsigned tmask) {
-  constexpr int NCOLS = nrange(L2, L2 + L3);
-  for (int q = lane; q < nrows * NCOLS; q += T) {
-    const int r = q / NCOLS, c = q - (q / NCOLS) * NCOLS;
-    buf[0][q] = tabp[(size_t)(row_off + r) * ryscols + col_off + c];
-  }
-  __syncwarp(tmask);
-  int cur = 0;
-  hrr_bra(buf, cur, L0, L1, NCOLS, ab, lane, T, tmask);
-  hrr_ket(buf, cur, blk, L0, L1, L2, L3, NCOLS, cd, lane, T, tmask);
-  constexpr int LS[4] = {L0, L1, L2, L3};
+// Where the recurrence tables (HrrTab, post.cuh) of the six shifted blocks
+// lie in the block's shared memory, as ints; a class whose tables exceed
+// GRAD_HRR_MAX (g shells) runs the component arithmetic of grad_post instead.
+constexpr int GRAD_HRR_MAX = 6144;
+template <int LA, int LB, int LC, int LD>
+struct GradHrr {
+  static constexpr int RA = 0;
+  static constexpr int FA = RA + HrrTab<LA + 1, LB, LC, LD>::TOTAL;
+  static constexpr int RB = FA + (LA > 0 ? HrrTab<(LA > 0 ? LA - 1 : 0), LB, LC, LD>::TOTAL : 0);
+  static constexpr int FB = RB + HrrTab<LA, LB + 1, LC, LD>::TOTAL;
+  static constexpr int RC = FB + (LB > 0 ? HrrTab<LA, (LB > 0 ? LB - 1 : 0), LC, LD>::TOTAL : 0);
+  static constexpr int FC = RC + HrrTab<LA, LB, LC + 1, LD>::TOTAL;
+  static constexpr int TOTAL = FC + (LC > 0 ? HrrTab<LA, LB, (LC > 0 ? LC - 1 : 0), LD>::TOTAL : 0);
+  static constexpr bool USE = TOTAL <= GRAD_HRR_MAX;
+};
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void build_grad_hrr(int* tab) {
+  using G = GradHrr<LA, LB, LC, LD>;
+  build_hrr_tab<LA + 1, LB, LC, LD>(tab + G::RA);
+  if constexpr (LA > 0) build_hrr_tab<LA - 1, LB, LC, LD>(tab + G::FA);
+  build_hrr_tab<LA, LB + 1, LC, LD>(tab + G::RB);
+  if constexpr (LB > 0) build_hrr_tab<LA, LB - 1, LC, LD>(tab + G::FB);
+  build_hrr_tab<LA, LB, LC + 1, LD>(tab + G::RC);
+  if constexpr (LC > 0) build_hrr_tab<LA, LB, LC - 1, LD>(tab + G::FC);
+}
+
+// The shifted block (L0, L1 | L2, L3) of its [e0|f0] slice, rows from `src` at
+// stride SC, table driven (team_hrr, post.cuh), and its dot with W.
+template <int L0, int L1, int L2, int L3, int POS, bool RAISED, int SC, int T>
+__device__ __forceinline__ void grad_shifted_ct(const double* src, const int* tab, const double* W, double* buf[3],
+                                                double* blk, const double ab[3], const double cd[3], double g[3],
+                                                int lane, unsigned tmask) {
+  team_hrr<L0, L1, L2, L3, T, double, SC>(src, buf, tab, blk, ab, cd, lane, tmask);
   constexpr int D0 = POS == 0 ? (RAISED ? -1 : 1) : 0, D1 = POS == 1 ? (RAISED ? -1 : 1) : 0;
   constexpr int D2 = POS == 2 ? (RAISED ? -1 : 1) : 0;
   // W and the dot use the unshifted shells
   grad_dot_ct<L0 + D0, L1 + D1, L2 + D2, L3, POS, RAISED, T>(W, blk, g, lane);
-  (void)LS;
   __syncwarp(tmask);
 }
 
-// Phase 2 of an all-Cartesian quartet (grad_post with compile-time shapes).
+// Phase 2 with compile-time shapes and table-driven recurrences.  The
+// component arithmetic of grad_post spends most of its time in index
+// divisions and in constant-memory lookups that serialise when the lanes
+// diverge.
 template <int LA, int LB, int LC, int LD, int T>
-__device__ __forceinline__ void grad_post_cart(const KernelArgs& A, const PairD& pb, const PairD& pk, const Screen& sc,
-                                               double* slot, double g[9], int lane, unsigned tmask) {
+__device__ __forceinline__ void grad_post_ct(const KernelArgs& A, const PairD& pb, const PairD& pk, const Screen& sc,
+                                             const int* tab, double* slot, double g[9], int lane, unsigned tmask) {
+  using G = GradHrr<LA, LB, LC, LD>;
   const GradSlot L = grad_slot_layout(LA, LB, LC, LD);
-  double* W = slot + L.ntab;
-  double* buf[3] = {W + 2 * L.W, W + 2 * L.W + L.S, W + 2 * L.W + 2 * L.S};
-  double* blk = W + 2 * L.W + 3 * L.S;
-  grad_weight_block_cart<LA, LB, LC, LD, T>(A, pb, pk, sc, W, lane);
-  __syncwarp(tmask);
+  double* W0 = slot + L.ntab;
+  double* W1 = W0 + L.W;
+  double* buf[3] = {W1 + L.W, W1 + L.W + L.S, W1 + L.W + 2 * L.S};
+  double* blk = W1 + L.W + 3 * L.S;
+  const double* W = W0;
+  if (A.kinds == 0) {
+    grad_weight_block_cart<LA, LB, LC, LD, T>(A, pb, pk, sc, W0, lane);
+    __syncwarp(tmask);
+  } else {
+    W = grad_weight_block(A, pb, pk, sc, W0, W1, lane, T, tmask);
+  }
   const double ab[3] = {pb.abx, pb.aby, pb.abz};
   const double cd[3] = {pk.abx, pk.aby, pk.abz};
-  constexpr int NE = LA + LB, NF = LC + LD;
-  constexpr int EA0 = LA > 0 ? LA - 1 : 0, FA0 = LC > 0 ? LC - 1 : 0;
+  constexpr int NF = LC + LD;
+  constexpr int FA0 = LC > 0 ? LC - 1 : 0;
   constexpr int COLSP = nrange(FA0, NF), COLS1 = nrange(LC, NF), COLS2 = nrange(LC + 1, NF + 1);
+  // the lowered blocks' slices of the plain table: rows from degree la-1 or
+  // la, columns from degree lc or lc-1
+  constexpr int ROWA = (LA > 0 ? ncart(LA - 1) : 0) * COLSP;
+  constexpr int COLL = tri_below(LC) - tri_below(FA0);
 #pragma unroll 1
   for (int q = 0; q < 9; ++q) g[q] = 0.0;
-  grad_shifted_ct<LA + 1, LB, LC, LD, 0, true, T>(slot + L.off_a, COLS1, 0, nrange(LA + 1, NE + 1), 0, W, buf, blk,
-                                                  ab, cd, g, lane, tmask);
+  grad_shifted_ct<LA + 1, LB, LC, LD, 0, true, COLS1, T>(slot + L.off_a, tab + G::RA, W, buf, blk, ab, cd, g, lane,
+                                                         tmask);
   if constexpr (LA > 0)
-    grad_shifted_ct<LA - 1, LB, LC, LD, 0, false, T>(slot + L.off_p, COLSP, 0, nrange(LA - 1, NE - 1),
-                                                     tri_below(LC) - tri_below(FA0), W, buf, blk, ab, cd, g, lane,
-                                                     tmask);
-  grad_shifted_ct<LA, LB + 1, LC, LD, 1, true, T>(slot + L.off_b, COLS1, 0, nrange(LA, NE + 1), 0, W, buf, blk, ab,
-                                                  cd, g + 3, lane, tmask);
+    grad_shifted_ct<LA - 1, LB, LC, LD, 0, false, COLSP, T>(slot + L.off_p + COLL, tab + G::FA, W, buf, blk, ab, cd, g,
+                                                            lane, tmask);
+  grad_shifted_ct<LA, LB + 1, LC, LD, 1, true, COLS1, T>(slot + L.off_b, tab + G::RB, W, buf, blk, ab, cd, g + 3,
+                                                         lane, tmask);
   if constexpr (LB > 0)
-    grad_shifted_ct<LA, LB - 1, LC, LD, 1, false, T>(slot + L.off_p, COLSP, tri_below(LA) - tri_below(EA0),
-                                                     nrange(LA, NE - 1), tri_below(LC) - tri_below(FA0), W, buf, blk,
-                                                     ab, cd, g + 3, lane, tmask);
-  grad_shifted_ct<LA, LB, LC + 1, LD, 2, true, T>(slot + L.off_c, COLS2, 0, nrange(LA, NE), 0, W, buf, blk, ab, cd,
-                                                  g + 6, lane, tmask);
+    grad_shifted_ct<LA, LB - 1, LC, LD, 1, false, COLSP, T>(slot + L.off_p + ROWA + COLL, tab + G::FB, W, buf, blk, ab,
+                                                            cd, g + 3, lane, tmask);
+  grad_shifted_ct<LA, LB, LC + 1, LD, 2, true, COLS2, T>(slot + L.off_c, tab + G::RC, W, buf, blk, ab, cd, g + 6,
+                                                         lane, tmask);
   if constexpr (LC > 0)
-    grad_shifted_ct<LA, LB, LC - 1, LD, 2, false, T>(slot + L.off_p, COLSP, tri_below(LA) - tri_below(EA0),
-                                                     nrange(LA, NE), 0, W, buf, blk, ab, cd, g + 6, lane, tmask);
+    grad_shifted_ct<LA, LB, LC - 1, LD, 2, false, COLSP, T>(slot + L.off_p + ROWA, tab + G::FC, W, buf, blk, ab, cd,
+                                                            g + 6, lane, tmask);
 }
 
 // --------------------------------------------------------------- kernel
@@ -769,6 +840,9 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
   constexpr int T = GS::T;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(16) R s_tab[rys_smem<GS::NR, R>(T)];
+  constexpr bool TAB = GradHrr<LA, LB, LC, LD>::USE;
+  __shared__ int s_hrr[TAB ? GradHrr<LA, LB, LC, LD>::TOTAL : 1];
+  if constexpr (TAB) build_grad_hrr<LA, LB, LC, LD>(s_hrr);
   const R* rys = rys_staged<GS::NR, R>(T) ? s_tab : rys_global<GS::NR, R>();
   stage_rys_table<GS::NR, R, T>(s_tab);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -817,8 +891,8 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
         grad_team_passes<LA, LB, LC, LD, R, 0>(A, rys, pb, pk, sm, lane, tmask, slot);
       __syncwarp(tmask);
       double g[9];
-      if (A.kinds == 0)
-        grad_post_cart<LA, LB, LC, LD, T>(A, pb, pk, sc, slot, g, lane, tmask);
+      if constexpr (TAB)
+        grad_post_ct<LA, LB, LC, LD, T>(A, pb, pk, sc, s_hrr, slot, g, lane, tmask);
       else
         grad_post(A, LA, LB, LC, LD, pb, pk, sc, slot, g, lane, T, tmask);
       if constexpr (T > 1) {

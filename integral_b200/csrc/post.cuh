@@ -922,11 +922,12 @@ __device__ __forceinline__ X pick_axis(int ax, const X v[3]) {
 }
 
 // The horizontal recurrences of one quartet on a team, table driven (same
-// recurrences and order as hrr_bra / hrr_ket): the [e0|f0] table in buf[0]
-// ([e][f]) becomes the Cartesian block [a][b][c][d] in `out`.
-template <int LA, int LB, int LC, int LD, int T, typename X>
-__device__ __forceinline__ void team_hrr(X* buf[3], const int* tab, X* out, const double ab[3], const double cd[3],
-                                         int lane, unsigned tmask) {
+// recurrences and order as hrr_bra / hrr_ket): the [e0|f0] table at `in`
+// ([e][f], rows SC values apart; it may be buf[0]) becomes the Cartesian block
+// [a][b][c][d] in `out`.
+template <int LA, int LB, int LC, int LD, int T, typename X, int SC = nrange(LC, LC + LD)>
+__device__ __forceinline__ void team_hrr(const X* in, X* buf[3], const int* tab, X* out, const double ab[3],
+                                         const double cd[3], int lane, unsigned tmask) {
   using H = HrrTab<LA, LB, LC, LD>;
   constexpr int NE = H::NE, NF = H::NF;
   constexpr int NFP = nrange(LC, NF);
@@ -939,22 +940,24 @@ __device__ __forceinline__ void team_hrr(X* buf[3], const int* tab, X* out, cons
     constexpr int KB = decltype(k_)::value + 1;
     constexpr int N = ncart(KB) * nrange(LA, NE - KB) * NFP;
     constexpr int OFF = H::bra_off(KB);
-    const X* src = buf[cur];
+    constexpr int ST = KB == 1 ? SC : NFP;
+    const X* src = KB == 1 ? in : buf[cur];
     X* dst = buf[(cur + 1) % 3];
     for (int q = lane; q < N; q += T) {
       const int row = q / NFP, f = q - row * NFP;
       const int e = tab[OFF + row];
-      dst[q] = src[(e & 0x7ff) * NFP + f] + pick_axis(e >> 22 & 3, abv) * src[((e >> 11) & 0x7ff) * NFP + f];
+      dst[q] = src[(e & 0x7ff) * ST + f] + pick_axis(e >> 22 & 3, abv) * src[((e >> 11) & 0x7ff) * ST + f];
     }
     __syncwarp(tmask);
     cur = (cur + 1) % 3;
   });
-  const X* Hb = buf[cur];  // [b][a][f]
+  const X* Hb = LB == 0 ? in : buf[cur];  // [b][a][f]
+  constexpr int HS = LB == 0 ? SC : NFP;
   if constexpr (LD == 0) {
     for (int q = lane; q < NAB * NC; q += T) {
       const int abr = q / NC, ic = q - abr * NC;
       const int ia = abr / NB, ib = abr - ia * NB;
-      out[q] = Hb[(ib * NA + ia) * NFP + ic];
+      out[q] = Hb[(ib * NA + ia) * HS + ic];
     }
   } else {
     const int w0 = (cur + 1) % 3, w1 = (cur + 2) % 3;
@@ -971,7 +974,7 @@ __device__ __forceinline__ void team_hrr(X* buf[3], const int* tab, X* out, cons
         int base;
         if constexpr (KD == 1) {
           const int ia = abr / NB, ib = abr - ia * NB;
-          base = (ib * NA + ia) * NFP;
+          base = (ib * NA + ia) * HS;
         } else {
           base = abr * NELP;
         }
@@ -1040,7 +1043,7 @@ __device__ __forceinline__ void post_quartet_jk_cart(const KernelArgs& A, const 
   const double cdv[3] = {pk.abx, pk.aby, pk.abz};
   // the block goes straight to the team's shared memory when it has room
   X* B = stage ? stage : xs + 3 * L.S;
-  team_hrr<LA, LB, LC, LD, T, X>(buf, hrr_tab, B, ab, cdv, lane, tmask);
+  team_hrr<LA, LB, LC, LD, T, X>(xs, buf, hrr_tab, B, ab, cdv, lane, tmask);
   const int shl[4] = {pb.a, pb.b, pk.a, pk.b};
   const int offs[4] = {A.shells[shl[0]].off, A.shells[shl[1]].off, A.shells[shl[2]].off, A.shells[shl[3]].off};
   double* acc = slot + A.acc_offset;
@@ -1087,7 +1090,7 @@ __device__ __forceinline__ void post_quartet_jk_sph(const KernelArgs& A, const P
   X* tmp = blk + L.blk;
   const double ab[3] = {pb.abx, pb.aby, pb.abz};
   const double cdv[3] = {pk.abx, pk.aby, pk.abz};
-  team_hrr<LA, LB, LC, LD, T, X>(buf, hrr_tab, blk, ab, cdv, lane, tmask);
+  team_hrr<LA, LB, LC, LD, T, X>(xs, buf, hrr_tab, blk, ab, cdv, lane, tmask);
   team_c2s_axis<0, N0, N1, N2, N3, F0, T, X>(blk, tmp, s_m + 0 * C2S_TILE, lane);
   __syncwarp(tmask);
   team_c2s_axis<1, F0, N1, N2, N3, F1, T, X>(tmp, blk, s_m + 1 * C2S_TILE, lane);
