@@ -399,6 +399,38 @@ __device__ __forceinline__ QuartetHdr<float> quartet_header_f(const PrimPairF& b
   return h;
 }
 
+// Primitive pair q of a lane's ket: from the class's interleaved copy when
+// the launch has one, else from the pair list.
+__device__ __forceinline__ PrimPairD load_ket(const KernelArgs& A, int prim_off, int kpos, int q, double) {
+  if (!A.kets) return A.prims[prim_off + q];
+  const size_t st = A.ket_stride;
+  const double* p = A.kets + (size_t)q * KET_VALS * st + kpos;
+  PrimPairD k;
+  k.zeta = __ldg(p);
+  k.inv2z = __ldg(p + st);
+  k.ez = __ldg(p + 2 * st);
+  k.px = __ldg(p + 3 * st);
+  k.py = __ldg(p + 4 * st);
+  k.pz = __ldg(p + 5 * st);
+  k.pax = __ldg(p + 6 * st);
+  k.pay = __ldg(p + 7 * st);
+  k.paz = __ldg(p + 8 * st);
+  return k;
+}
+__device__ __forceinline__ PrimPairF load_ket(const KernelArgs& A, int prim_off, int kpos, int q, float) {
+  if (!A.ketsf) return A.primsf[prim_off + q];
+  const size_t st = A.ket_stride;
+  const float* p = A.ketsf + (size_t)q * KET_VALS_F * st + kpos;
+  PrimPairF k;
+  k.zeta = __ldg(p);
+  k.inv2z = __ldg(p + st);
+  k.ez = __ldg(p + 2 * st);
+  k.pax = __ldg(p + 3 * st);
+  k.pay = __ldg(p + 4 * st);
+  k.paz = __ldg(p + 5 * st);
+  return k;
+}
+
 // ----------------------------------------------------------- misc device
 
 __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {

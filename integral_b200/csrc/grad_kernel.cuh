@@ -878,8 +878,8 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
     TaskCursor cur;
     if (base + tw < end) cursor_seek(A.task, base + tw, cur);
     for (unsigned long long t = base + tw; t < end; t += TPW) {
-      int pbi, pki;
-      cursor_decode(A.task, t, cur, pbi, pki);
+      int pbi, pki, kpos;
+      cursor_decode(A.task, t, cur, pbi, pki, kpos);
       const PairD pb = A.pairs[pbi];
       const PairD pk = A.pairs[pki];
       const Screen sc = screen_quartet(A, pb, pk);

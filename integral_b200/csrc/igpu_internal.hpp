@@ -61,6 +61,15 @@ struct alignas(16) PrimPairF {
   float alpha, beta;
 };
 
+// Lane-interleaved copy of a ket class's primitive pairs for the kernels that
+// run one quartet per lane: value v of primitive pair q of the ket at position
+// k of the class list lies at (q * KET_VALS + v) * stride + k, so that lanes
+// on consecutive kets read consecutive values.  From PrimPairD each such read
+// of a warp takes one L1 wavefront per lane (96 bytes apart), which bound
+// those kernels: 85-92% of the L1 rate in FP64.
+constexpr int KET_VALS = 9;    // zeta, inv2z, ez, px, py, pz, pax, pay, paz
+constexpr int KET_VALS_F = 6;  // zeta, inv2z, ez, pax, pay, paz
+
 // One canonical shell pair (i >= j in the reference's sense) with its
 // evaluation orientation.  An auxiliary pair of density fitting (an aux shell
 // with the unit s dummy, src/df.rs:1-37) has i = the aux shell's position in
@@ -186,6 +195,9 @@ struct KernelArgs {
   const PairD* pairs;
   const PrimPairD* prims;
   const PrimPairF* primsf;  // FP32 copy of prims (same order)
+  const double* kets;       // this ket class's interleaved copies (nullptr: none)
+  const float* ketsf;
+  size_t ket_stride;
   const double* c2s;     // c2s matrices (ratio folded), c2s_off[l] into it
   int c2s_off[GPU_MAX_L + 3];
   int nsh;

@@ -31,6 +31,34 @@ int add_class_unit(bool grad, ClassRegFn reg, ConstUpFn up) {
   return (int)class_units().size();
 }
 
+namespace {
+struct WideUnit {
+  WideRegFn reg;
+  ConstUpFn up;
+};
+std::vector<WideUnit>& wide_units() {
+  static std::vector<WideUnit> v;
+  return v;
+}
+}  // namespace
+
+int add_wide_unit(WideRegFn reg, ConstUpFn up) {
+  wide_units().push_back({reg, up});
+  return (int)wide_units().size();
+}
+
+static WideEntry g_wide_table[NPC * NPC];
+static std::once_flag g_wide_once;
+
+const WideEntry* wide_entry(int pcb, int pck, bool fp32) {
+  std::call_once(g_wide_once, [] {
+    for (const WideUnit& u : wide_units()) u.reg(g_wide_table, NPC);
+  });
+  if (pcb < 0 || pck < 0 || pcb >= NPC || pck >= NPC || pcb < pck) return nullptr;
+  const WideEntry* e = &g_wide_table[pcb * NPC + pck];
+  return (fp32 ? e->k32 : e->k64) ? e : nullptr;
+}
+
 static KernelEntry g_table[NPC * NPC];
 static KernelEntry g_grad_table[GNPC * GNPC];
 static std::once_flag g_once, g_grad_once;
@@ -73,6 +101,10 @@ cudaError_t upload_all_constants(const ConstData& c) {
     cudaError_t e = u.up(c);
     if (e != cudaSuccess) return e;
   }
+  for (const WideUnit& u : wide_units()) {
+    cudaError_t e = u.up(c);
+    if (e != cudaSuccess) return e;
+  }
   return cudaSuccess;
 }
 
@@ -81,6 +113,18 @@ int blocks_per_sm(const KernelEntry* e, bool fp32) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void*>(fp32 ? e->k32 : e->k64), 128,
                                                 fp32 ? e->smem32 : e->smem64);
   return n < 1 ? 1 : n;
+}
+
+int blocks_per_sm(const WideEntry* e, bool fp32) {
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, reinterpret_cast<const void*>(fp32 ? e->k32 : e->k64), 128, 0);
+  return n < 1 ? 1 : n;
+}
+
+cudaError_t launch_wide(const WideEntry* e, bool fp32, int grid, const KernelArgs& args, cudaStream_t stream) {
+  auto k = fp32 ? e->k32 : e->k64;
+  k<<<grid, 128, 0, stream>>>(args);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_quartets(const KernelEntry* e, bool fp32, int grid, const KernelArgs& args,
@@ -151,6 +195,31 @@ __global__ void to_float_kernel(const double* __restrict__ in, float* __restrict
 cudaError_t launch_to_float(const double* in, float* out, size_t n, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   to_float_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, out, n);
+  return cudaGetLastError();
+}
+
+// The lane-interleaved copies of one ket class (KET_VALS): one thread per
+// (position, primitive pair).
+__global__ void ket_copy_kernel(const PairD* __restrict__ pairs, const PrimPairD* __restrict__ prims,
+                                const int* __restrict__ list, int n, int maxprim, double* __restrict__ out,
+                                float* __restrict__ outf) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (size_t)n * maxprim) return;
+  const int k = (int)(t % n), q = (int)(t / n);
+  const PairD p = pairs[list[k]];
+  if (q >= p.nprim) return;
+  const PrimPairD d = prims[p.prim_off + q];
+  const double v[KET_VALS] = {d.zeta, d.inv2z, d.ez, d.px, d.py, d.pz, d.pax, d.pay, d.paz};
+  const float f[KET_VALS_F] = {(float)d.zeta, (float)d.inv2z, (float)d.ez, (float)d.pax, (float)d.pay, (float)d.paz};
+  for (int i = 0; i < KET_VALS; ++i) out[((size_t)q * KET_VALS + i) * n + k] = v[i];
+  for (int i = 0; i < KET_VALS_F; ++i) outf[((size_t)q * KET_VALS_F + i) * n + k] = f[i];
+}
+
+cudaError_t launch_ket_copy(const PairD* pairs, const PrimPairD* prims, const int* list, int n, int maxprim,
+                            double* out, float* outf, cudaStream_t s) {
+  const size_t t = (size_t)n * maxprim;
+  if (t == 0) return cudaSuccess;
+  ket_copy_kernel<<<(unsigned)((t + 127) / 128), 128, 0, s>>>(pairs, prims, list, n, maxprim, out, outf);
   return cudaGetLastError();
 }
 

@@ -21,6 +21,17 @@ struct KernelEntry {
   bool valid = false;
 };
 
+// One-thread-per-quartet kernels of the larger Cartesian classes (wide.cuh),
+// for symmetric J/K launches of many quartets; absent where nullptr.
+struct WideEntry {
+  void (*k64)(KernelArgs) = nullptr;
+  void (*k32)(KernelArgs) = nullptr;
+  size_t tab64 = 0, tab32 = 0;  // scratch doubles per block before the J sums
+};
+using WideRegFn = void (*)(WideEntry* tab, int npc);
+int add_wide_unit(WideRegFn reg, cudaError_t (*up)(const ConstData&));
+const WideEntry* wide_entry(int pcb, int pck, bool fp32);
+
 // Highest shell l of the compiled gradient classes.
 #ifndef GRAD_KERNEL_MAX_L
 #define GRAD_KERNEL_MAX_L 3
@@ -43,12 +54,16 @@ const KernelEntry* grad_entry(int pcb, int pck);
 const KernelEntry* kernel_entry(int pcb, int pck);
 cudaError_t upload_all_constants(const ConstData& c);
 int blocks_per_sm(const KernelEntry* e, bool fp32);
+int blocks_per_sm(const WideEntry* e, bool fp32);
 cudaError_t launch_quartets(const KernelEntry* e, bool fp32, int grid, const KernelArgs& args,
                             cudaStream_t stream);
+cudaError_t launch_wide(const WideEntry* e, bool fp32, int grid, const KernelArgs& args, cudaStream_t stream);
 cudaError_t launch_shell_block_max(const double* D, int nmat, const DevShell* sh, int nsh, int nao,
                                    int symmetrise, double* out, cudaStream_t s);
 cudaError_t launch_symmetrize_add(const double* H, double* out, int nmat, int nao, cudaStream_t s);
 cudaError_t launch_to_float(const double* in, float* out, size_t n, cudaStream_t s);
+cudaError_t launch_ket_copy(const PairD* pairs, const PrimPairD* prims, const int* list, int n, int maxprim,
+                            double* out, float* outf, cudaStream_t s);
 cudaError_t launch_asym_count(const double* D, int nmat, int nao, unsigned long long* flag, cudaStream_t s);
 // Molecule batches (plan_batch.cpp): matrices of molecule m at m*P*(P+1),
 // row stride P; shell blocks at m*S*(S+1), row stride S.

@@ -71,15 +71,21 @@ static int sm_count() {
   return count[dev];
 }
 
-size_t grid_for(const KernelEntry* e, bool fp32, unsigned long long total, int bps_cap) {
-  const int nsm = sm_count();
-  const int teams_per_block = 128 / e->team;
-  const unsigned long long need = (total + teams_per_block - 1) / teams_per_block;
-  int bps = blocks_per_sm(e, fp32);
+// Blocks for `total` quartets, `per_block` at a time, at `bps` blocks per SM.
+static size_t grid_blocks(unsigned long long total, int per_block, int bps, int bps_cap) {
+  const unsigned long long need = (total + per_block - 1) / per_block;
   if (bps_cap > 0 && bps_cap < bps) bps = bps_cap;
-  const unsigned long long cap = (unsigned long long)bps * nsm;
+  const unsigned long long cap = (unsigned long long)bps * sm_count();
   return (size_t)std::max<unsigned long long>(1, std::min(need, cap));
 }
+
+size_t grid_for(const KernelEntry* e, bool fp32, unsigned long long total, int bps_cap) {
+  return grid_blocks(total, 128 / e->team, blocks_per_sm(e, fp32), bps_cap);
+}
+
+// Quartets from which a class's launch takes its one-thread-per-quartet
+// kernel (wide.cuh).
+static unsigned long long wide_min_tasks() { return (unsigned long long)kWideRounds * 128 * sm_count(); }
 
 KernelArgs base_args(igpu_plan* P) {
   KernelArgs A;
@@ -254,6 +260,33 @@ static int ensure_side_streams(igpu_plan* P, size_t n) {
   return IGPU_OK;
 }
 
+// The lane-interleaved ket copies (KET_VALS) of every main class that a
+// one-thread launch can have as its ket: shells up to d.
+static int ensure_kets(igpu_plan* P) {
+  if (!P->ket_off.empty()) return IGPU_OK;
+  const int npc = std::min<int>((int)P->class_pairs.size(), pair_class(2, 2) + 1);
+  std::vector<size_t> off, offf;
+  std::vector<int> maxprim(npc, 0);
+  size_t n = 0, nf = 0;
+  for (int c = 0; c < npc; ++c) {
+    for (int p : P->class_pairs[c]) maxprim[c] = std::max(maxprim[c], P->pairs[p].nprim);
+    off.push_back(n);
+    offf.push_back(nf);
+    n += P->class_pairs[c].size() * (size_t)maxprim[c] * KET_VALS;
+    nf += P->class_pairs[c].size() * (size_t)maxprim[c] * KET_VALS_F;
+  }
+  CK(P->d_kets.ensure(n));
+  CK(P->d_ketsf.ensure(nf));
+  for (int c = 0; c < npc; ++c)
+    CK(launch_ket_copy(P->d_pairs.p, P->d_prims.p, P->d_class_lists.p + P->class_list_off[c],
+                       (int)P->class_pairs[c].size(), maxprim[c], P->d_kets.p + off[c], P->d_ketsf.p + offf[c],
+                       P->stream));
+  CK(cudaStreamSynchronize(P->stream));
+  P->ket_off = off;
+  P->ketf_off = offf;
+  return IGPU_OK;
+}
+
 // Run every launch of a task set; quartet kernels only.  Per-launch device
 // time and counters are kept for igpu_last_profile.
 //
@@ -273,8 +306,11 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   auto entry = [grad](int pcb, int pck) { return grad ? grad_entry(pcb, pck) : kernel_entry(pcb, pck); };
   const size_t nl = ts.launches.size();
   struct Planned {
-    size_t li, grid, slot, stream;
+    size_t li, grid, stream;
+    size_t slot, acc;         // scratch doubles per unit, and before its J sums
+    size_t units;             // teams (wide kernels: blocks) in the grid
     const KernelEntry* e;
+    const WideEntry* wide;    // its one-thread-per-quartet kernel runs instead
     double load;
     bool full;  // enough rounds to fill the device by itself
   };
@@ -296,17 +332,34 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     Planned r{};
     r.li = li;
     r.e = e;
-    r.grid = grid_for(e, L->fp32, L->total, bps_cap);
-    r.slot = slot_with_acc(e, L->pcb, A);
+    if (A.mode == MODE_JK && A.jk.symmetric && A.kinds == 0 && L->total >= wide_min_tasks())
+      r.wide = wide_entry(L->pcb, L->pck, L->fp32);
+    const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
+    if (r.wide) {
+      r.grid = grid_blocks(L->total, 128, blocks_per_sm(r.wide, L->fp32), bps_cap);
+      r.units = r.grid;
+      r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
+      r.slot = r.acc + 128 * sums;
+    } else {
+      r.grid = grid_for(e, L->fp32, L->total, bps_cap);
+      r.units = r.grid * (128 / e->team);
+      // one-thread classes finish symmetric J/K of one shell kind in registers
+      r.acc = e->team == 1 && A.mode == MODE_JK && A.jk.symmetric && A.kinds != 2 ? 0 : e->slot;
+      r.slot = r.acc + sums;
+    }
     // rounds of quartets over the resident teams times one quartet's work on
     // a team's lanes
     const int la = pc_la_host(L->pcb), lb = L->pcb - la * (la + 1) / 2;
     const int lc = pc_la_host(L->pck), ld = L->pck - lc * (lc + 1) / 2;
-    const double teams = (double)r.grid * (128 / e->team);
+    const double teams = r.wide ? (double)r.grid * 128 : (double)r.units;
     const double np = (double)L->prim_pairs * L->prim_pairs;
     r.full = (double)L->total >= kFullRounds * teams;
     r.load = std::ceil((double)L->total / teams) * np *
-             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / e->team;
+             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / (r.wide ? 1 : e->team);
+    if (!grad && (r.wide || e->team == 1) && L->ket_class >= 0) {
+      const int rc = ensure_kets(P);
+      if (rc) return rc;
+    }
     run.push_back(r);
   }
   // longest first; fewer streams while the scratch regions exceed the budget
@@ -315,7 +368,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
     return run[x].full != run[y].full ? run[x].full : run[x].load > run[y].load;
   });
-  auto doubles = [](const Planned& r) { return r.grid * (128 / r.e->team) * r.slot; };
+  auto doubles = [](const Planned& r) { return r.units * r.slot; };
   size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(kRunStreams, run.size()));
   std::vector<size_t> region;  // scratch doubles per stream
   size_t largest = 0;
@@ -386,7 +439,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     const cudaStream_t st = stream_of(pl.stream);
     A.scratch = base[pl.stream];
     A.slot_doubles = pl.slot;
-    A.acc_offset = e->slot;
+    A.acc_offset = pl.acc;
     A.work_counter = lg.work.p + li;
     // tasks a warp claims per grab: (32 / team) x mult.  Untuned, mult is 16,
     // or less when the launch has so few tasks that 16 would leave warps of
@@ -403,6 +456,8 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       if (t != P->tuned_mult.end()) mult = t->second;
     }
     A.chunk = (unsigned long long)(32 / e->team) * mult;
+    // a wide block takes 128 quartets at a time
+    if (pl.wide) A.chunk = 128 * std::max<unsigned long long>(1, std::min<unsigned long long>(4, L->total / (512 * grid)));
     A.counters = counters ? counters + li : nullptr;
     A.task.bra_pair = L->bra_pair.p;
     A.task.ket_pairs = L->ket_list;
@@ -410,11 +465,15 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     A.task.ket_start = L->ket_start.n ? L->ket_start.p : nullptr;
     A.task.nbra = L->nbra;
     A.task.total = L->total;
+    const bool copies = !grad && (pl.wide || e->team == 1) && L->ket_class >= 0 && L->ket_class < (int)P->ket_off.size();
+    A.kets = copies ? P->d_kets.p + P->ket_off[L->ket_class] : nullptr;
+    A.ketsf = copies ? P->d_ketsf.p + P->ketf_off[L->ket_class] : nullptr;
+    A.ket_stride = copies ? P->class_pairs[L->ket_class].size() : 0;
     A.fp32 = L->fp32 ? 1 : 0;
     A.prim_cut = prim_cut0 / fp32_class_scale(class_lmax(L->pcb, L->pck));
     A.builder_swap = L->builder_swap;
     CK(record(lg.events[2 * li], st));
-    CK(launch_quartets(e, L->fp32, (int)grid, A, st));
+    CK(pl.wide ? launch_wide(pl.wide, L->fp32, (int)grid, A, st) : launch_quartets(e, L->fp32, (int)grid, A, st));
     CK(record(lg.events[2 * li + 1], st));
     ++launches;
     igpu_launch_record& r = lg.profile[x];
@@ -423,7 +482,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     r.lc = pc_la_host(L->pck);
     r.ld = L->pck - r.lc * (r.lc + 1) / 2;
     r.fp32 = L->fp32 ? 1 : 0;
-    r.team = e->team;
+    r.team = pl.wide ? 1 : e->team;
     r.grid = (uint32_t)grid;
     r.tasks = L->total;
     r.chunk = (uint32_t)A.chunk;
@@ -601,10 +660,12 @@ int build_jk_tasks(igpu_plan* P, double tau, double fp64_cut, TaskSet& ts) {
       int rc;
       auto L64 = make_launch(P, ca, cb, false, bras, n64, st64, klist, 0, P->stream, rc);
       if (!L64) return rc;
+      L64->ket_class = cb;
       ts.launches.push_back(std::move(L64));
       if (fp64_cut > 0.0) {
         auto L32 = make_launch(P, ca, cb, true, bras, n32, st32, klist, 0, P->stream, rc);
         if (!L32) return rc;
+        L32->ket_class = cb;
         ts.launches.push_back(std::move(L32));
       }
     }

@@ -93,6 +93,7 @@ struct Launch {
   DevBuf<int> bra_pair, ket_start, own_kets;
   DevBuf<unsigned long long> prefix;
   const int* ket_list = nullptr;  // device Q-sorted pair list of the ket class
+  int ket_class = -1;             // the main class whose list that is (-1: another list)
 };
 
 struct TaskSet {
@@ -119,6 +120,8 @@ constexpr size_t kRunStreams = 8;
 // Scratch doubles (256 MiB, or twice the largest launch's) above which a run
 // uses fewer streams, each of which needs a scratch region of its own.
 constexpr size_t kScratchBudget = (size_t)1 << 25;
+// Rounds of 128 quartets per SM from which a launch takes the wide kernels.
+constexpr double kWideRounds = 3.0;
 // Quartets per resident team from which a launch fills the device by itself:
 // its last round is then at most a sixteenth of it.
 constexpr double kFullRounds = 16.0;
@@ -179,6 +182,11 @@ struct igpu_plan {
   DevBuf<double> d_c2s;
   DevBuf<int> d_class_lists;
   std::vector<int> class_list_off;
+  // lane-interleaved primitive pairs of the main ket classes up to d shells
+  // (KET_VALS), made by the first run with one-thread launches
+  DevBuf<double> d_kets;
+  DevBuf<float> d_ketsf;
+  std::vector<size_t> ket_off, ketf_off;
   DevBuf<double> d_scratch;
   DevBuf<Counters> d_counters;
   DevBuf<double> d_schwarz_pair;

@@ -61,13 +61,13 @@ __device__ __forceinline__ void cursor_seek(const TaskList& t, unsigned long lon
   c.hi = t.prefix[lo + 1];
 }
 __device__ __forceinline__ void cursor_decode(const TaskList& t, unsigned long long g, TaskCursor& c, int& pbi,
-                                              int& pki) {
+                                              int& pki, int& kpos) {
   while (g >= c.hi) {  // g < prefix[nbra] = total, so seg stays below nbra
     ++c.seg;
     c.lo = c.hi;
     c.hi = t.prefix[c.seg + 1];
   }
-  const int kpos = (int)(g - c.lo) + (t.ket_start ? t.ket_start[c.seg] : 0);
+  kpos = (int)(g - c.lo) + (t.ket_start ? t.ket_start[c.seg] : 0);
   pbi = t.bra_pair[c.seg];
   pki = t.ket_pairs[kpos];
 }
@@ -398,8 +398,11 @@ __device__ __forceinline__ void jk_term(const double* B, const int dims[4], cons
 
 // Atomically add a team's running bra-block accumulators to J' and clear
 // them.  acc layout: [0] = evaluation bra pair index (or -1), then
-// ndens blocks of n_func(A) x n_func(B).
-__device__ __forceinline__ void flush_bra_acc(const KernelArgs& A, double* acc, int lane, int T, unsigned tmask) {
+// ndens blocks of n_func(A) x n_func(B); consecutive values lie `as` doubles
+// apart (32 where every lane of a warp has its own: the lanes' accesses then
+// coalesce).
+__device__ __forceinline__ void flush_bra_acc(const KernelArgs& A, double* acc, int as, int lane, int T,
+                                              unsigned tmask) {
   const int bra = (int)acc[0];
   if (bra >= 0) {
     const PairD pb = A.pairs[bra];
@@ -407,13 +410,13 @@ __device__ __forceinline__ void flush_bra_acc(const KernelArgs& A, double* acc, 
     const int nab = sa.nfunc * sb.nfunc;
     const size_t n2 = (size_t)A.nao * A.nao;
     for (int d = 0; d < A.jk.ndens; ++d) {
-      double* a = acc + 1 + (size_t)d * nab;
+      double* a = acc + (1 + (size_t)d * nab) * as;
       for (int q = lane; q < nab; q += T) {
-        const double v = a[q];
+        const double v = a[q * as];
         if (v != 0.0) {
           const int ia = q / sb.nfunc, ib = q % sb.nfunc;
           atomicAdd(A.jk.J + d * n2 + (size_t)(sa.off + ia) * A.nao + sb.off + ib, v);
-          a[q] = 0.0;
+          a[q * as] = 0.0;
         }
       }
     }
@@ -439,7 +442,7 @@ constexpr int JK_DCH = 4;
 template <int DCH>
 __device__ __forceinline__ void jk_sym_chunk(const KernelArgs& A, const double* B, const int dims[4],
                                              const int offs[4], const double wt[6], int nterm, int d0, unsigned m,
-                                             double* acc, int lane, int T) {
+                                             double* acc, int as, int lane, int T) {
   // (u, v) output axes and (s, t) summed axes of term t, one nibble per term
   // (no dynamically indexed local arrays); D block rows on s, columns on t
   constexpr unsigned PU = 0x101020u, PV = 0x332231u, PS = 0x010102u, PT = 0x223313u;
@@ -481,7 +484,7 @@ __device__ __forceinline__ void jk_sym_chunk(const KernelArgs& A, const double* 
     if (t == 0) {
 #pragma unroll
       for (int k = 0; k < DCH; ++k)
-        if ((m >> k) & 1u) acc[1 + (size_t)(d0 + k) * nab + r] += w * sum[k];
+        if ((m >> k) & 1u) acc[(1 + (size_t)(d0 + k) * nab + r) * as] += w * sum[k];
     } else {
       double* out = t == 1 ? A.jk.J : A.jk.K;
       const size_t o = (size_t)(off(u) + iu) * nao + off(v) + iv;
@@ -499,14 +502,14 @@ __host__ __device__ constexpr int jk_stage_doubles(int la, int lb, int lc, int l
 
 __device__ __forceinline__ void consume_jk(const KernelArgs& A, const double* B, const int dims[4],
                                            const int offs[4], const int sh[4], uint64_t mask, int lane, int T,
-                                           double* acc, int pbi, unsigned tmask, double* stage) {
+                                           double* acc, int as, int pbi, unsigned tmask, double* stage) {
   const unsigned w = distinct_perms(sh);
   auto W = [&](int p) { return (double)((w >> p) & 1u); };
   const int nao = A.nao;
   const size_t n2 = (size_t)nao * nao;
   if (A.jk.symmetric) {
     if ((int)acc[0] != pbi) {
-      flush_bra_acc(A, acc, lane, T, tmask);
+      flush_bra_acc(A, acc, as, lane, T, tmask);
       if (lane == 0) acc[0] = (double)pbi;
       __syncwarp(tmask);
     }
@@ -525,7 +528,7 @@ __device__ __forceinline__ void consume_jk(const KernelArgs& A, const double* B,
     const unsigned long long live = A.jk.ndens >= 64 ? ~0ull : ((1ull << A.jk.ndens) - 1ull);
     for (int d0 = 0; d0 < A.jk.ndens; d0 += JK_DCH) {
       const unsigned m = (unsigned)(((mask & live) >> d0) & ((1u << JK_DCH) - 1u));
-      if (m) jk_sym_chunk<JK_DCH>(A, Bs, dims, offs, wt, nterm, d0, m, acc, lane, T);
+      if (m) jk_sym_chunk<JK_DCH>(A, Bs, dims, offs, wt, nterm, d0, m, acc, as, lane, T);
     }
     __syncwarp(tmask);
     return;
@@ -759,7 +762,7 @@ __device__ __forceinline__ void consume_schwarz(const KernelArgs& A, const doubl
 // block -> consumer.
 __device__ __forceinline__ void post_quartet(const KernelArgs& A, const ClassDims& cd_, const PairD& pb,
                                              const PairD& pk, const Screen& sc, double* slot, int lane, int T,
-                                             unsigned tmask, int pb_index, double* stage) {
+                                             unsigned tmask, int pb_index, double* stage, double* acc, int as) {
   const int la = cd_.la, lb = cd_.lb, lc = cd_.lc, ld = cd_.ld;
   const SlotLayout L = slot_layout(la, lb, lc, ld);
   double* buf[3] = {slot, slot + L.S, slot + 2 * L.S};
@@ -780,7 +783,7 @@ __device__ __forceinline__ void post_quartet(const KernelArgs& A, const ClassDim
   const int offs[4] = {s0.off, s1.off, s2.off, s3.off};
   switch (A.mode) {
     case MODE_JK:
-      consume_jk(A, B, dims, offs, shl, sc.mask, lane, T, slot + A.acc_offset, pb_index, tmask, stage);
+      consume_jk(A, B, dims, offs, shl, sc.mask, lane, T, acc, as, pb_index, tmask, stage);
       break;
     case MODE_DENSE:
       consume_dense(A, B, dims, offs, shl, lane, T);
@@ -1048,7 +1051,7 @@ __device__ __forceinline__ void post_quartet_jk_cart(const KernelArgs& A, const 
   const int offs[4] = {A.shells[shl[0]].off, A.shells[shl[1]].off, A.shells[shl[2]].off, A.shells[shl[3]].off};
   double* acc = slot + A.acc_offset;
   if ((int)acc[0] != pbi) {
-    flush_bra_acc(A, acc, lane, T, tmask);
+    flush_bra_acc(A, acc, 1, lane, T, tmask);
     if (lane == 0) acc[0] = (double)pbi;
     __syncwarp(tmask);
   }
@@ -1104,7 +1107,7 @@ __device__ __forceinline__ void post_quartet_jk_sph(const KernelArgs& A, const P
   const int offs[4] = {A.shells[shl[0]].off, A.shells[shl[1]].off, A.shells[shl[2]].off, A.shells[shl[3]].off};
   double* acc = slot + A.acc_offset;
   if ((int)acc[0] != pbi) {
-    flush_bra_acc(A, acc, lane, T, tmask);
+    flush_bra_acc(A, acc, 1, lane, T, tmask);
     if (lane == 0) acc[0] = (double)pbi;
     __syncwarp(tmask);
   }

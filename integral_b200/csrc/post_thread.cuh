@@ -144,7 +144,7 @@ __device__ __forceinline__ void thread_block(const V* G, V* blk, const PairD& pb
 // Symmetric-density J/K of one function-space block [N0][N1][N2][N3] in
 // value type V (double, or float for the FP32 launches of the mixed path,
 // which read the FP32 copy of the densities): bra-block J term into the
-// running FP64 accumulators `acc`, the other five one-orientation terms
+// running FP64 accumulators `acc` (values 32 doubles apart), the other five one-orientation terms
 // atomically into the FP64 J', K'.
 template <int N0, int N1, int N2, int N3, typename V>
 __device__ __forceinline__ void thread_jk(const KernelArgs& A, const V* B, const int offs[4], unsigned w,
@@ -166,7 +166,7 @@ __device__ __forceinline__ void thread_jk(const KernelArgs& A, const V* B, const
       for (int c = 0; c < N2; ++c)
 #pragma unroll
         for (int e = 0; e < N3; ++e) dcd[c * N3 + e] = __ldg(Dm + (size_t)(offs[2] + c) * nao + offs[3] + e);
-      double* a = acc + 1 + (size_t)d * N0 * N1;
+      double* a = acc + (1 + (size_t)d * N0 * N1) * 32;
 #pragma unroll
       for (int i = 0; i < N0; ++i)
 #pragma unroll
@@ -174,7 +174,7 @@ __device__ __forceinline__ void thread_jk(const KernelArgs& A, const V* B, const
           V s = V(0);
 #pragma unroll
           for (int q = 0; q < N2 * N3; ++q) s += B[i * S0 + j * S1 + q] * dcd[q];
-          a[i * N1 + j] += (double)(wab * s);
+          a[(i * N1 + j) * 32] += (double)(wab * s);
         }
     }
     // J'[C c][D d]
@@ -288,7 +288,7 @@ __device__ __forceinline__ void thread_post_jk(const KernelArgs& A, const V* G, 
   const int offs[4] = {A.shells[shl[0]].off, A.shells[shl[1]].off, A.shells[shl[2]].off, A.shells[shl[3]].off};
   const unsigned w = distinct_perms(shl);
   if ((int)acc[0] != pbi) {
-    flush_bra_acc(A, acc, 0, 1, 1u << (threadIdx.x & 31));
+    flush_bra_acc(A, acc, 32, 0, 1, 1u << (threadIdx.x & 31));
     acc[0] = (double)pbi;
   }
   if constexpr (!SPH) {

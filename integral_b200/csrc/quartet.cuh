@@ -104,7 +104,7 @@ constexpr int MAX_SURV = 256;
 
 template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* tab, const PairD& pb,
-                                                  const PairD& pk, R (&G)[ClassShape<LA, LB, LC, LD>::NG]) {
+                                                  const PairD& pk, int kpos, R (&G)[ClassShape<LA, LB, LC, LD>::NG]) {
   using S = ClassShape<LA, LB, LC, LD>;
   constexpr int NE = S::NE, NF = S::NF, NR = S::NR;
 #pragma unroll
@@ -123,11 +123,11 @@ __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* 
       QuartetHdr<R> h;
       if constexpr (sizeof(R) == 4) {
         const PrimPairF bp = A.primsf[pb.prim_off + ip];
-        const PrimPairF kp = A.primsf[pk.prim_off + kq];
+        const PrimPairF kp = load_ket(A, pk.prim_off, kpos, kq, 0.f);
         if (cut > 0.f && prim_bound(bp, kp) < cut) continue;
         h = quartet_header_f(bp, kp, acx, acy, acz, A.omega);
       } else {
-        h = quartet_header<R>(A.prims[pb.prim_off + ip], A.prims[pk.prim_off + kq], A.omega);
+        h = quartet_header<R>(A.prims[pb.prim_off + ip], load_ket(A, pk.prim_off, kpos, kq, 0.0), A.omega);
       }
       R x[NR], w[NR];
       if constexpr (sizeof(R) == 4) {
@@ -393,7 +393,16 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
   R* sm = reinterpret_cast<R*>(team_smem);
   double* stage = TS::STAGE ? reinterpret_cast<double*>(team_smem) : nullptr;
   R* stage_r = TS::STAGE ? reinterpret_cast<R*>(team_smem) : nullptr;
+  // a team's slot, then its running bra-block accumulators; one-thread teams
+  // keep a warp's accumulators together, interleaved by lane
+  constexpr int AS = T == 1 ? 32 : 1;
   double* slot = A.scratch + (size_t)team * A.slot_doubles;
+  double* acc = slot + A.acc_offset;
+  if constexpr (T == 1) {
+    double* warp = A.scratch + (size_t)(team & ~31) * A.slot_doubles;
+    slot = warp + (size_t)(team & 31) * A.acc_offset;
+    acc = warp + 32 * A.acc_offset + (team & 31);
+  }
   QuartetCounters cnt;
   const ClassDims dims{LA, LB, LC, LD};
   (void)nteams;
@@ -401,9 +410,8 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
   if (use_acc) {
     // the scratch slot is shared with earlier launches: clear the running
     // bra-block accumulators before first use
-    double* acc = slot + A.acc_offset;
     const int nacc = A.jk.ndens * ncart(LA) * ncart(LB);
-    for (int q = lane; q < nacc; q += T) acc[1 + q] = 0.0;
+    for (int q = lane; q < nacc; q += T) acc[(1 + q) * AS] = 0.0;
     if (lane == 0) acc[0] = -1.0;
   }
   __syncwarp(tmask);
@@ -422,8 +430,8 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
     TaskCursor cur;
     if (base + tw < end) cursor_seek(A.task, base + tw, cur);
     for (unsigned long long g = base + tw; g < end; g += TPW) {
-      int pbi, pki;
-      cursor_decode(A.task, g, cur, pbi, pki);
+      int pbi, pki, kpos;
+      cursor_decode(A.task, g, cur, pbi, pki, kpos);
       const PairD pb = A.pairs[pbi];
       const PairD pk = A.pairs[pki];
       Screen sc = screen_quartet(A, pb, pk);
@@ -431,14 +439,14 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
       if (lane == 0) cnt.add(sc, pb, pk, A.fp32);
       if constexpr (T == 1) {
         R G[S::NG];
-        accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, G);
+        accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, kpos, G);
         if (use_acc && A.kinds != 2) {
           // the post phase runs in the launch's arithmetic (FP32 launches
           // read the FP32 densities); J/K accumulate in FP64
           if (A.kinds == 0)
-            thread_post_jk<LA, LB, LC, LD, false, R>(A, G, pb, pk, sc, slot + A.acc_offset, pbi);
+            thread_post_jk<LA, LB, LC, LD, false, R>(A, G, pb, pk, sc, acc, pbi);
           else
-            thread_post_jk<LA, LB, LC, LD, true, R>(A, G, pb, pk, sc, slot + A.acc_offset, pbi);
+            thread_post_jk<LA, LB, LC, LD, true, R>(A, G, pb, pk, sc, acc, pbi);
           continue;
         }
 #pragma unroll
@@ -471,11 +479,11 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
           continue;
         }
       }
-      post_quartet(A, dims, pb, pk, sc, slot, lane, T, tmask, pbi, stage);
+      post_quartet(A, dims, pb, pk, sc, slot, lane, T, tmask, pbi, stage, acc, AS);
       __syncwarp(tmask);
     }
   }
-  if (use_acc) flush_bra_acc(A, slot + A.acc_offset, lane, T, tmask);
+  if (use_acc) flush_bra_acc(A, acc, AS, lane, T, tmask);
   cnt.flush(A.counters);
 }
 
