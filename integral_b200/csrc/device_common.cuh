@@ -1,10 +1,11 @@
 // Device helpers shared by the quartet kernels: compile-time angular-momentum
-// tables, Rys roots/weights from the Chebyshev tables, the per-axis Rys
+// tables, Rys roots/weights from the polynomial tables, the per-axis Rys
 // vertical recurrence, and small warp utilities.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include "igpu_internal.hpp"

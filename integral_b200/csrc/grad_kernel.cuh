@@ -671,13 +671,14 @@ __device__ __forceinline__ void grad_post(const KernelArgs& A, int la, int lb, i
 
 __host__ __device__ constexpr int cidx(int lx, int ly, int lz) { return (ly + lz) * (ly + lz + 1) / 2 + lz; }
 
-// Weight block of an all-Cartesian quartet with compile-time dims (same
-// values as grad_weight_block).  The reference-orientation AO index of each
+// Function-space weight block of an all-Cartesian (or, SPH, all-spherical)
+// quartet with compile-time dims (same values as grad_weight_block).  The reference-orientation AO index of each
 // element is picked by selects, not by indexing a local array.
-template <int LA, int LB, int LC, int LD, int T>
-__device__ __forceinline__ void grad_weight_block_cart(const KernelArgs& A, const PairD& pb, const PairD& pk,
+template <int LA, int LB, int LC, int LD, int T, bool SPH>
+__device__ __forceinline__ void grad_weight_block_ct(const KernelArgs& A, const PairD& pb, const PairD& pk,
                                                        const Screen& sc, double* W, int lane) {
-  constexpr int N0 = ncart(LA), N1 = ncart(LB), N2 = ncart(LC), N3 = ncart(LD);
+  constexpr int N0 = SPH ? 2 * LA + 1 : ncart(LA), N1 = SPH ? 2 * LB + 1 : ncart(LB);
+  constexpr int N2 = SPH ? 2 * LC + 1 : ncart(LC), N3 = SPH ? 2 * LD + 1 : ncart(LD);
   const int o0 = A.shells[pb.a].off, o1 = A.shells[pb.b].off, o2 = A.shells[pk.a].off, o3 = A.shells[pk.b].off;
   // evaluation position of reference positions 0..3
   const int bb = sc.swapped ? 2 : 0, kb = sc.swapped ? 0 : 2;
@@ -709,6 +710,26 @@ __device__ __forceinline__ void grad_weight_block_cart(const KernelArgs& A, cons
                   __ldg(Lm + m0 * n + m3) * __ldg(Rm + m1 * n + m2) + __ldg(Lm + m1 * n + m3) * __ldg(Rm + m0 * n + m2));
     }
     W[q] = w;
+  }
+}
+
+// One axis of the pull-back of a function-space weight block to Cartesian
+// components, the transpose of team_c2s_axis: M is (2l+1) x NOUT in shared
+// memory, the block [D0][D1][D2][D3].
+template <int AXIS, int D0, int D1, int D2, int D3, int NOUT, int T>
+__device__ __forceinline__ void team_c2s_back(const double* in, double* out, const double* M, int lane) {
+  constexpr int dims[4] = {D0, D1, D2, D3};
+  constexpr int NIN = dims[AXIS];
+  constexpr int outer = AXIS == 0 ? 1 : (AXIS == 1 ? D0 : (AXIS == 2 ? D0 * D1 : D0 * D1 * D2));
+  constexpr int inner = AXIS == 0 ? D1 * D2 * D3 : (AXIS == 1 ? D2 * D3 : (AXIS == 2 ? D3 : 1));
+  for (int q = lane; q < outer * NOUT * inner; q += T) {
+    const int sidx = q % inner, t = q / inner;
+    const int qo = t % NOUT, o = t / NOUT;
+    const double* src = in + (o * NIN) * inner + sidx;
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < NIN; ++j) acc += M[j * NOUT + qo] * src[j * inner];
+    out[q] = acc;
   }
 }
 
@@ -790,7 +811,8 @@ __device__ __forceinline__ void grad_shifted_ct(const double* src, const int* ta
 // diverge.
 template <int LA, int LB, int LC, int LD, int T>
 __device__ __forceinline__ void grad_post_ct(const KernelArgs& A, const PairD& pb, const PairD& pk, const Screen& sc,
-                                             const int* tab, double* slot, double g[9], int lane, unsigned tmask) {
+                                             const int* tab, const double* s_c2s, double* slot, double g[9], int lane,
+                                             unsigned tmask) {
   using G = GradHrr<LA, LB, LC, LD>;
   const GradSlot L = grad_slot_layout(LA, LB, LC, LD);
   double* W0 = slot + L.ntab;
@@ -799,7 +821,20 @@ __device__ __forceinline__ void grad_post_ct(const KernelArgs& A, const PairD& p
   double* blk = W1 + L.W + 3 * L.S;
   const double* W = W0;
   if (A.kinds == 0) {
-    grad_weight_block_cart<LA, LB, LC, LD, T>(A, pb, pk, sc, W0, lane);
+    grad_weight_block_ct<LA, LB, LC, LD, T, false>(A, pb, pk, sc, W0, lane);
+    __syncwarp(tmask);
+  } else if (A.kinds == 1) {
+    constexpr int F0 = 2 * LA + 1, F1 = 2 * LB + 1, F2 = 2 * LC + 1, F3 = 2 * LD + 1;
+    constexpr int N0 = ncart(LA), N1 = ncart(LB), N2 = ncart(LC), N3 = ncart(LD);
+    grad_weight_block_ct<LA, LB, LC, LD, T, true>(A, pb, pk, sc, W0, lane);
+    __syncwarp(tmask);
+    team_c2s_back<3, F0, F1, F2, F3, N3, T>(W0, W1, s_c2s + 3 * C2S_TILE, lane);
+    __syncwarp(tmask);
+    team_c2s_back<2, F0, F1, F2, N3, N2, T>(W1, W0, s_c2s + 2 * C2S_TILE, lane);
+    __syncwarp(tmask);
+    team_c2s_back<1, F0, F1, N2, N3, N1, T>(W0, W1, s_c2s + 1 * C2S_TILE, lane);
+    __syncwarp(tmask);
+    team_c2s_back<0, F0, N1, N2, N3, N0, T>(W1, W0, s_c2s + 0 * C2S_TILE, lane);
     __syncwarp(tmask);
   } else {
     W = grad_weight_block(A, pb, pk, sc, W0, W1, lane, T, tmask);
@@ -842,7 +877,11 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
   __shared__ __align__(16) R s_tab[rys_smem<GS::NR, R>(T)];
   constexpr bool TAB = GradHrr<LA, LB, LC, LD>::USE;
   __shared__ int s_hrr[TAB ? GradHrr<LA, LB, LC, LD>::TOTAL : 1];
-  if constexpr (TAB) build_grad_hrr<LA, LB, LC, LD>(s_hrr);
+  __shared__ double s_c2s[TAB ? 4 * C2S_TILE : 1];
+  if constexpr (TAB) {
+    build_grad_hrr<LA, LB, LC, LD>(s_hrr);
+    stage_c2s<LA, LB, LC, LD, double>(A, s_c2s);
+  }
   const R* rys = rys_staged<GS::NR, R>(T) ? s_tab : rys_global<GS::NR, R>();
   stage_rys_table<GS::NR, R, T>(s_tab);
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -892,7 +931,7 @@ __global__ void __launch_bounds__(128) grad_kernel(KernelArgs A) {
       __syncwarp(tmask);
       double g[9];
       if constexpr (TAB)
-        grad_post_ct<LA, LB, LC, LD, T>(A, pb, pk, sc, s_hrr, slot, g, lane, tmask);
+        grad_post_ct<LA, LB, LC, LD, T>(A, pb, pk, sc, s_hrr, s_c2s, slot, g, lane, tmask);
       else
         grad_post(A, LA, LB, LC, LD, pb, pk, sc, slot, g, lane, T, tmask);
       if constexpr (T > 1) {

@@ -8,10 +8,6 @@
 
 namespace igpu {
 
-struct ClassDims {
-  int la, lb, lc, ld;
-};
-
 // Scratch-slot layout of one quartet (in doubles): three level buffers of S
 // doubles (the first holds G on entry), then the Cartesian block and its
 // transform partner.
@@ -758,65 +754,12 @@ __device__ __forceinline__ void consume_schwarz(const KernelArgs& A, const doubl
   if (lane == 0) A.schwarz_out[pair_index] = sqrt(mx);
 }
 
-// Post phase of one quartet: G (in slot) -> Cartesian block -> function
-// block -> consumer.
-__device__ __forceinline__ void post_quartet(const KernelArgs& A, const ClassDims& cd_, const PairD& pb,
-                                             const PairD& pk, const Screen& sc, double* slot, int lane, int T,
-                                             unsigned tmask, int pb_index, double* stage, double* acc, int as) {
-  const int la = cd_.la, lb = cd_.lb, lc = cd_.lc, ld = cd_.ld;
-  const SlotLayout L = slot_layout(la, lb, lc, ld);
-  double* buf[3] = {slot, slot + L.S, slot + 2 * L.S};
-  double* blk = slot + 3 * L.S;
-  double* tmp = blk + L.blk;
-  const int nfp = nrange(lc, lc + ld);
-  const double ab[3] = {pb.abx, pb.aby, pb.abz};
-  const double cdv[3] = {pk.abx, pk.aby, pk.abz};
-  int cur = 0;
-  hrr_bra(buf, cur, la, lb, nfp, ab, lane, T, tmask);
-  hrr_ket(buf, cur, blk, la, lb, lc, ld, nfp, cdv, lane, T, tmask);
-  const int shl[4] = {pb.a, pb.b, pk.a, pk.b};
-  const DevShell s0 = A.shells[shl[0]], s1 = A.shells[shl[1]], s2 = A.shells[shl[2]], s3 = A.shells[shl[3]];
-  int dims[4] = {ncart(la), ncart(lb), ncart(lc), ncart(ld)};
-  const int ls[4] = {la, lb, lc, ld};
-  const int sph[4] = {s0.spherical, s1.spherical, s2.spherical, s3.spherical};
-  const double* B = c2s_block(A, blk, tmp, dims, ls, sph, lane, T, tmask);
-  const int offs[4] = {s0.off, s1.off, s2.off, s3.off};
-  switch (A.mode) {
-    case MODE_JK:
-      consume_jk(A, B, dims, offs, shl, sc.mask, lane, T, acc, as, pb_index, tmask, stage);
-      break;
-    case MODE_DENSE:
-      consume_dense(A, B, dims, offs, shl, lane, T);
-      break;
-    case MODE_BUILDER:
-      consume_builder(A, B, dims, offs, shl, A.builder_swap != 0, lane, T);
-      break;
-    case MODE_PACKED:
-      consume_packed(A, B, dims, pb, pk, sc, lane, T);
-      break;
-    case MODE_SCHWARZ:
-      consume_schwarz(A, B, dims, pb_index, lane, T, tmask);
-      break;
-    case MODE_DF3:
-      consume_df3(A, B, dims, offs, shl, pb.j < 0, lane, T);
-      break;
-    case MODE_DF2:
-      consume_df2(A, B, dims, offs, shl, lane, T);
-      break;
-    case MODE_BLOCK:
-      consume_block(A, B, dims, shl, lane, T);
-      break;
-    default:
-      break;
-  }
-}
-
 // ----------------------------------------- J/K post phase, Cartesian classes
 
 // One contraction term of the symmetric J/K images with the block shape
 // known at compile time: output (u, v), summed (s, t), D block rows on s and
-// columns on t.  Every sum is fully unrolled, so its block and density loads
-// are independent and in flight together.
+// columns on t.  The sums are unrolled, so their block and density loads are
+// independent and in flight together.
 template <int U, int V, int S, int TT, int N0, int N1, int N2, int N3, int T, bool ACC, typename X>
 __device__ __forceinline__ void jk_term_ct(const KernelArgs& A, const X* B, const int offs[4], X w, int d0, unsigned m,
                                            double* out, int lane) {
@@ -824,6 +767,7 @@ __device__ __forceinline__ void jk_term_ct(const KernelArgs& A, const X* B, cons
   constexpr int ST[4] = {N1 * N2 * N3, N2 * N3, N3, 1};
   constexpr int NU = N[U], NV = N[V], NS = N[S], NT = N[TT];
   constexpr int DCH = JK_DCH;
+  constexpr int UNROLL = NS * NT <= 50 ? NS : 1;  // whole sums up to f shells, rows of g sums
   const int nao = A.nao;
   const size_t n2 = (size_t)nao * nao;
   const X* Dp = dens_of<X>(A.jk) + (size_t)d0 * n2 + (size_t)offs[S] * nao + offs[TT];
@@ -833,7 +777,7 @@ __device__ __forceinline__ void jk_term_ct(const KernelArgs& A, const X* B, cons
     X sum[DCH];
 #pragma unroll
     for (int k = 0; k < DCH; ++k) sum[k] = X(0);
-#pragma unroll
+#pragma unroll UNROLL
     for (int is = 0; is < NS; ++is)
 #pragma unroll
       for (int it = 0; it < NT; ++it) {
@@ -991,6 +935,64 @@ __device__ __forceinline__ void team_hrr(const X* in, X* buf[3], const int* tab,
     });
   }
   __syncwarp(tmask);
+}
+
+// Post phase of one quartet: G (in slot) -> Cartesian block -> function
+// block -> consumer.
+template <int LA, int LB, int LC, int LD, int TEAM>
+__device__ __forceinline__ void post_quartet(const KernelArgs& A, const int* hrr_tab, const PairD& pb,
+                                             const PairD& pk, const Screen& sc, double* slot, int lane, int T,
+                                             unsigned tmask, int pb_index, double* stage, double* acc, int as) {
+  constexpr int la = LA, lb = LB, lc = LC, ld = LD;
+  const SlotLayout L = slot_layout(la, lb, lc, ld);
+  double* buf[3] = {slot, slot + L.S, slot + 2 * L.S};
+  double* blk = slot + 3 * L.S;
+  double* tmp = blk + L.blk;
+  const double ab[3] = {pb.abx, pb.aby, pb.abz};
+  const double cdv[3] = {pk.abx, pk.aby, pk.abz};
+  if constexpr (TEAM > 1) {
+    team_hrr<LA, LB, LC, LD, TEAM, double>(slot, buf, hrr_tab, blk, ab, cdv, lane, tmask);
+  } else {
+    constexpr int nfp = nrange(lc, lc + ld);
+    int cur = 0;
+    hrr_bra(buf, cur, la, lb, nfp, ab, lane, T, tmask);
+    hrr_ket(buf, cur, blk, la, lb, lc, ld, nfp, cdv, lane, T, tmask);
+  }
+  const int shl[4] = {pb.a, pb.b, pk.a, pk.b};
+  const DevShell s0 = A.shells[shl[0]], s1 = A.shells[shl[1]], s2 = A.shells[shl[2]], s3 = A.shells[shl[3]];
+  int dims[4] = {ncart(la), ncart(lb), ncart(lc), ncart(ld)};
+  const int ls[4] = {la, lb, lc, ld};
+  const int sph[4] = {s0.spherical, s1.spherical, s2.spherical, s3.spherical};
+  const double* B = c2s_block(A, blk, tmp, dims, ls, sph, lane, T, tmask);
+  const int offs[4] = {s0.off, s1.off, s2.off, s3.off};
+  switch (A.mode) {
+    case MODE_JK:
+      consume_jk(A, B, dims, offs, shl, sc.mask, lane, T, acc, as, pb_index, tmask, stage);
+      break;
+    case MODE_DENSE:
+      consume_dense(A, B, dims, offs, shl, lane, T);
+      break;
+    case MODE_BUILDER:
+      consume_builder(A, B, dims, offs, shl, A.builder_swap != 0, lane, T);
+      break;
+    case MODE_PACKED:
+      consume_packed(A, B, dims, pb, pk, sc, lane, T);
+      break;
+    case MODE_SCHWARZ:
+      consume_schwarz(A, B, dims, pb_index, lane, T, tmask);
+      break;
+    case MODE_DF3:
+      consume_df3(A, B, dims, offs, shl, pb.j < 0, lane, T);
+      break;
+    case MODE_DF2:
+      consume_df2(A, B, dims, offs, shl, lane, T);
+      break;
+    case MODE_BLOCK:
+      consume_block(A, B, dims, shl, lane, T);
+      break;
+    default:
+      break;
+  }
 }
 
 // One axis of the Cartesian -> spherical transform of a [D0][D1][D2][D3]

@@ -14,8 +14,8 @@
 //   TEAM == 1 : one thread per quartet, everything in registers.
 //   TEAM >= 2 : a team of TEAM lanes per quartet; roots and the 3*nroots
 //               per-axis tables are built cooperatively in shared memory and
-//               every lane accumulates its own rows e of G (register tiles
-//               of FCH columns, the f range walked in chunks).
+//               every lane accumulates its own rows of G, of the bra or the
+//               ket side (register tiles walked in passes, TeamSweep).
 // The class's Rys table is staged in shared memory where rys_staged says so.
 // Phase 2 (post.cuh) runs the horizontal recurrences, the Cartesian ->
 // spherical transform and the mode-specific consumer on the team.
@@ -52,31 +52,72 @@ __host__ __device__ constexpr int team_size() {
   return team_for(nrange(LA, LA + LB), nrange(LC, LC + LD));
 }
 
-// Phase-1 register footprint per lane: rows x FCH accumulators.
+// Accumulators per lane and pass.
 template <typename R>
 __host__ __device__ constexpr int max_acc() { return sizeof(R) == 8 ? 64 : 96; }
+
+// How a team sums its table.  Rows of one side (e of the bra, or f of the ket
+// when `ket`) go one to a lane over groups of `gp` lanes, the other side's
+// components are the columns; the team's T / gp groups take different primitive
+// quartets of a round.  A pass holds rp row slots and fch columns per lane and
+// recomputes the 2D tables.
+struct TeamSweep {
+  bool ket;
+  int gp, rl, nchunk, fch, rp, npass;
+  long cost;
+};
+// The cheapest of the lane-rows, by a count of SM cycles per root (times 32):
+// a row slot loads 3 (N + 1) axis values, N the columns' side, once per column
+// chunk, and spends two operations per column; a warp's FP64 shared load takes
+// four times its multiply-add (likewise in FP32).  Rows on the bra side alone
+// cost (33|21) 2.7 times as much: 74 rows of 21 loads for 16 columns against 16
+// rows of 21 for 74.
+__host__ __device__ constexpr TeamSweep team_sweep(int la, int lb, int lc, int ld, int T, int bp, int max_acc) {
+  const int ne = la + lb, nf = lc + ld;
+  const int nep = nrange(la, ne), nfp = nrange(lc, nf);
+  TeamSweep best{};
+  best.cost = 1L << 60;
+  for (int side = 0; side < 2; ++side)
+    for (int gp = T; gp >= 4; gp /= 2) {
+      TeamSweep w{};
+      w.ket = side == 1;
+      const int rows = w.ket ? nfp : nep, cols = w.ket ? nep : nfp;
+      const int loads = 3 * ((w.ket ? ne : nf) + 1);
+      w.gp = gp;
+      w.rl = (rows + gp - 1) / gp;
+      w.nchunk = (cols + max_acc - 1) / max_acc;
+      w.fch = (cols + w.nchunk - 1) / w.nchunk;
+      int rp = w.nchunk > 1 ? 1 : max_acc / cols;
+      rp = rp < w.rl ? rp : w.rl;
+      rp = rp < 6 ? rp : 6;  // three offsets a row slot
+      const int rpass = (w.rl + rp - 1) / rp;
+      w.rp = (w.rl + rpass - 1) / rpass;
+      w.npass = ((w.rl + w.rp - 1) / w.rp) * w.nchunk;
+      const int groups = T / gp < bp ? T / gp : bp;
+      w.cost = (long)w.npass * 10 * (ne + 1) * (nf + 1) + (long)(T / groups) * w.rl * (2 * w.nchunk * loads + cols);
+      if (w.cost < best.cost) best = w;
+    }
+  return best;
+}
 
 template <int LA, int LB, int LC, int LD, typename R>
 struct TeamShape {
   using S = ClassShape<LA, LB, LC, LD>;
   static constexpr int T = team_size<LA, LB, LC, LD>();
-  static constexpr int ROWS = (S::NEP + T - 1) / T;
-  static constexpr int FCH0 = max_acc<R>() / ROWS;
-  static constexpr int FCH = FCH0 < 1 ? 1 : (FCH0 > S::NFP ? S::NFP : FCH0);
-  static constexpr int NCHUNK = (S::NFP + FCH - 1) / FCH;
   // Primitive quartets set up per round: as many as fit a shared-memory
-  // budget of 48 KB per 128-thread block (power of two, at most T).
+  // budget of 56 KB (FP32: 48) per 128-thread block (power of two, at most T).
   static constexpr int GTAB = (S::NE + 1) * (S::NF + 1);
   // x, w, g[3][NR][GTAB] of one primitive quartet, an odd number of values:
   // the lanes that build different quartets' tables store at this stride, and
   // an even one shares few banks (it was 96 for (22|10): every lane of a store
   // in one bank)
   static constexpr int PRIM_TAB = (2 * S::NR + 3 * S::NR * GTAB) | 1;
-  static constexpr int BUDGET = (48 * 1024 / 128) * (T == 1 ? 1 : T) / (int)sizeof(R);
+  static constexpr int BUDGET = ((sizeof(R) == 8 ? 56 : 48) * 1024 / 128) * (T == 1 ? 1 : T) / (int)sizeof(R);
   static constexpr int BP0 = BUDGET / PRIM_TAB;
   static constexpr int BP = BP0 >= T ? T : (BP0 >= 16 ? 16 : (BP0 >= 8 ? 8 : (BP0 >= 4 ? 4 : (BP0 >= 2 ? 2 : 1))));
   static constexpr int SUB = T / BP;  // lanes sharing one primitive quartet in a round
   static constexpr int SMEM_PER_TEAM = T == 1 ? 0 : BP * PRIM_TAB;  // in R units
+  static constexpr TeamSweep SW = team_sweep(LA, LB, LC, LD, T < 4 ? 4 : T, BP, max_acc<R>());
   // Per-team shared memory: the primitive tables of phase 1, reused by the
   // post phase for the team's copy of the Cartesian block (16-byte multiple).
   // Classes whose copies would need more than 96 KB per 128-thread block
@@ -178,29 +219,41 @@ __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* 
 // --------------------------------------------------------------- TEAM > 1
 
 // One pass over all primitive quartets accumulating the columns
-// [F0, F0 + FCH) of this lane's rows.
-template <int LA, int LB, int LC, int LD, typename R, int F0>
+// [C0, C0 + fch) of this lane's rows in row slots [K0, K0 + rp).
+template <int LA, int LB, int LC, int LD, typename R, int K0, int C0>
 __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* tab, const PairD& pb, const PairD& pk,
                                           R* sm, int lane, unsigned tmask, double* G, const unsigned short* surv,
                                           int npr, bool g32) {
   using S = ClassShape<LA, LB, LC, LD>;
   using TS = TeamShape<LA, LB, LC, LD, R>;
+  constexpr TeamSweep SW = TS::SW;
   constexpr int NE = S::NE, NF = S::NF, NR = S::NR, T = TS::T;
-  constexpr int FW = (F0 + TS::FCH <= S::NFP) ? TS::FCH : (S::NFP - F0);
+  constexpr bool KET = SW.ket;
+  constexpr int GP = SW.gp, GROUPS = T / GP;
+  constexpr int NROW = KET ? S::NFP : S::NEP, NCOL = KET ? S::NEP : S::NFP;
+  constexpr int RLO = KET ? LC : LA, CLO = KET ? LA : LC;  // lowest degrees
+  constexpr int NL = KET ? NE : NF;                        // axis power of the columns' side
+  constexpr int RST = KET ? 1 : NF + 1, CST = KET ? NF + 1 : 1;
+  constexpr int CW = C0 + SW.fch <= NCOL ? SW.fch : NCOL - C0;
   constexpr int GT = TS::GTAB;
-  R acc[TS::ROWS][FW];
+  constexpr int ROWS = SW.rl - K0 < SW.rp ? SW.rl - K0 : SW.rp;
+  // unrolled, the loads of later roots are hoisted into registers that large
+  // tiles do not leave
+  constexpr int ROOTS_UNROLL = ROWS * CW * (int)sizeof(R) / 4 <= 40 ? NR : 1;
+  const int gl = lane % GP, grp = lane / GP;
+  R acc[ROWS][CW];
 #pragma unroll
-  for (int k = 0; k < TS::ROWS; ++k)
+  for (int k = 0; k < ROWS; ++k)
 #pragma unroll
-    for (int f = 0; f < FW; ++f) acc[k][f] = R(0);
-  int ex[TS::ROWS], ey[TS::ROWS], ez[TS::ROWS];
+    for (int c = 0; c < CW; ++c) acc[k][c] = R(0);
+  int rx0[ROWS], ry0[ROWS], rz0[ROWS];
 #pragma unroll
-  for (int k = 0; k < TS::ROWS; ++k) {
-    int e = lane + T * k;
-    int a = tri_below(LA) + (e < S::NEP ? e : 0);
-    ex[k] = addr_lx(a);
-    ey[k] = addr_ly(a);
-    ez[k] = addr_lz(a);
+  for (int k = 0; k < ROWS; ++k) {
+    const int row = gl + GP * (K0 + k);
+    const int a = tri_below(RLO) + (row < NROW ? row : 0);
+    rx0[k] = addr_lx(a) * RST;
+    ry0[k] = addr_ly(a) * RST;
+    rz0[k] = addr_lz(a) * RST;
   }
   // Rounds of BP primitive quartets: SUB lanes set up each one (roots, then
   // the 3*NR per-axis tables) into its shared-memory slot, then every lane
@@ -269,27 +322,27 @@ __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* tab, con
       }
     }
     __syncwarp(tmask);
-    for (int p = 0; p < nb; ++p) {
+    for (int p = grp; p < nb; p += GROUPS) {
       const R* gt = sm + p * PT + 2 * NR;
-#pragma unroll
+#pragma unroll ROOTS_UNROLL
       for (int r = 0; r < NR; ++r) {
         const R* tx = gt + (0 * NR + r) * GT;
         const R* ty = gt + (1 * NR + r) * GT;
         const R* tz = gt + (2 * NR + r) * GT;
 #pragma unroll
-        for (int k = 0; k < TS::ROWS; ++k) {
-          if (TS::ROWS * T > S::NEP && lane + T * k >= S::NEP) continue;
-          R rx[NF + 1], ry[NF + 1], rz[NF + 1];
+        for (int k = 0; k < ROWS; ++k) {
+          if (SW.rl * GP > NROW && gl + GP * (K0 + k) >= NROW) continue;
+          R rx[NL + 1], ry[NL + 1], rz[NL + 1];
 #pragma unroll
-          for (int m = 0; m <= NF; ++m) {
-            rx[m] = tx[ex[k] * (NF + 1) + m];
-            ry[m] = ty[ey[k] * (NF + 1) + m];
-            rz[m] = tz[ez[k] * (NF + 1) + m];
+          for (int m = 0; m <= NL; ++m) {
+            rx[m] = tx[rx0[k] + m * CST];
+            ry[m] = ty[ry0[k] + m * CST];
+            rz[m] = tz[rz0[k] + m * CST];
           }
-          static_for<FW>([&](auto f) {
-            constexpr int fi = F0 + decltype(f)::value;
-            constexpr int fx = range_x(LC, fi), fy = range_y(LC, fi), fz = range_z(LC, fi);
-            acc[k][decltype(f)::value] += rx[fx] * ry[fy] * rz[fz];
+          static_for<CW>([&](auto c) {
+            constexpr int ci = C0 + decltype(c)::value;
+            constexpr int cx = range_x(CLO, ci), cy = range_y(CLO, ci), cz = range_z(CLO, ci);
+            acc[k][decltype(c)::value] += rx[cx] * ry[cy] * rz[cz];
           });
         }
       }
@@ -297,31 +350,36 @@ __device__ __forceinline__ void team_pass(const KernelArgs& A, const R* tab, con
     __syncwarp(tmask);
   }
 #pragma unroll
-  for (int k = 0; k < TS::ROWS; ++k) {
-    int e = lane + T * k;
-    if (e < S::NEP) {
-      if (sizeof(R) == 4 && g32) {
-        // FP32 post phase: the table stays in FP32
-        float* Gf = reinterpret_cast<float*>(G);
+  for (int k = 0; k < ROWS; ++k) {
+    // the groups' sums over their primitive quartets
 #pragma unroll
-        for (int f = 0; f < FW; ++f) Gf[(size_t)e * S::NFP + F0 + f] = (float)acc[k][f];
-      } else {
+    for (int o = GP; o < T; o *= 2)
 #pragma unroll
-        for (int f = 0; f < FW; ++f) G[(size_t)e * S::NFP + F0 + f] = (double)acc[k][f];
+      for (int c = 0; c < CW; ++c) acc[k][c] += __shfl_xor_sync(tmask, acc[k][c], o);
+    const int row = gl + GP * (K0 + k);
+    if (grp == 0 && row < NROW) {
+#pragma unroll
+      for (int c = 0; c < CW; ++c) {
+        const size_t at = KET ? (size_t)(C0 + c) * S::NFP + row : (size_t)row * S::NFP + C0 + c;
+        if (sizeof(R) == 4 && g32)
+          reinterpret_cast<float*>(G)[at] = (float)acc[k][c];  // FP32 post phase: the table stays in FP32
+        else
+          G[at] = (double)acc[k][c];
       }
     }
   }
 }
 
-template <int LA, int LB, int LC, int LD, typename R, int C>
-__device__ __forceinline__ void team_chunks(const KernelArgs& A, const R* tab, const PairD& pb, const PairD& pk,
+template <int LA, int LB, int LC, int LD, typename R, int P>
+__device__ __forceinline__ void team_passes(const KernelArgs& A, const R* tab, const PairD& pb, const PairD& pk,
                                             R* sm, int lane, unsigned tmask, double* G, const unsigned short* surv,
                                             int npr, bool g32) {
   using TS = TeamShape<LA, LB, LC, LD, R>;
-  if constexpr (C < TS::NCHUNK) {
-    team_pass<LA, LB, LC, LD, R, C * TS::FCH>(A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
+  if constexpr (P < TS::SW.npass) {
+    team_pass<LA, LB, LC, LD, R, P / TS::SW.nchunk * TS::SW.rp, P % TS::SW.nchunk * TS::SW.fch>(
+        A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
     __syncwarp(tmask);
-    team_chunks<LA, LB, LC, LD, R, C + 1>(A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
+    team_passes<LA, LB, LC, LD, R, P + 1>(A, tab, pb, pk, sm, lane, tmask, G, surv, npr, g32);
   }
 }
 
@@ -375,12 +433,17 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
   __shared__ __align__(16) R s_tab[rys_smem<S::NR, R>(T)];
   constexpr bool SCREEN = sizeof(R) == 4 && T > 1;
   __shared__ unsigned short s_surv[SCREEN ? (128 / T) * MAX_SURV : 1];
-  constexpr bool CT_POST = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 10000;
-  __shared__ int s_hrr[(T > 1 && CT_POST) ? HrrTab<LA, LB, LC, LD>::TOTAL : 1];
-  __shared__ R s_c2s[(T > 1 && CT_POST) ? 4 * C2S_TILE : 1];
-  if constexpr (T > 1 && CT_POST) {
+  // compile-time shaped J/K sums: every spherical class, Cartesian blocks up
+  // to (ff|ff); the larger ones (Cartesian g shells) take the runtime sums
+  constexpr bool CT_CART = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD) <= 10000;
+  __shared__ int s_hrr[T > 1 ? HrrTab<LA, LB, LC, LD>::TOTAL : 1];
+  // the spherical post phase runs in the launch's arithmetic up to f shells,
+  // in FP64 beyond
+  using PX = std::conditional_t<CT_CART, R, double>;
+  __shared__ PX s_c2s[T > 1 ? 4 * C2S_TILE : 1];
+  if constexpr (T > 1) {
     build_hrr_tab<LA, LB, LC, LD>(s_hrr);
-    stage_c2s<LA, LB, LC, LD, R>(A, s_c2s);
+    stage_c2s<LA, LB, LC, LD, PX>(A, s_c2s);
   }
   const R* tab = rys_staged<S::NR, R>(T) ? s_tab : rys_global<S::NR, R>();
   stage_rys_table<S::NR, R, T>(s_tab);  // its __syncthreads also publishes s_hrr, s_c2s
@@ -404,7 +467,6 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
     acc = warp + 32 * A.acc_offset + (team & 31);
   }
   QuartetCounters cnt;
-  const ClassDims dims{LA, LB, LC, LD};
   (void)nteams;
   const bool use_acc = A.mode == MODE_JK && A.jk.symmetric;
   if (use_acc) {
@@ -462,24 +524,26 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
             if (npr == 0) continue;  // the whole quartet is below the screen
           }
         }
-        team_chunks<LA, LB, LC, LD, R, 0>(A, tab, pb, pk, sm, lane, tmask, slot, surv, npr,
-                                          CT_POST && use_acc && A.kinds != 2);
+        team_passes<LA, LB, LC, LD, R, 0>(A, tab, pb, pk, sm, lane, tmask, slot, surv, npr,
+                                          CT_CART && use_acc && A.kinds != 2);
       }
       __syncwarp(tmask);
-      // the compile-time shaped J/K sums unroll over the whole Cartesian
-      // block, in the launch's arithmetic; blocks beyond (ff|ff) (g shells)
-      // take the runtime post phase
-      if constexpr (T > 1 && CT_POST) {
+      // in the launch's arithmetic; everything else, and the runtime sums, in
+      // FP64
+      if constexpr (T > 1 && CT_CART) {
         if (use_acc && A.kinds == 0) {
           post_quartet_jk_cart<LA, LB, LC, LD, T, R>(A, pb, pk, sc, slot, lane, tmask, pbi, stage_r, s_hrr);
           continue;
         }
+      }
+      if constexpr (T > 1) {
         if (use_acc && A.kinds == 1) {
-          post_quartet_jk_sph<LA, LB, LC, LD, T, R>(A, pb, pk, sc, slot, lane, tmask, pbi, stage_r, s_hrr, s_c2s);
+          post_quartet_jk_sph<LA, LB, LC, LD, T, PX>(A, pb, pk, sc, slot, lane, tmask, pbi,
+                                                     reinterpret_cast<PX*>(stage), s_hrr, s_c2s);
           continue;
         }
       }
-      post_quartet(A, dims, pb, pk, sc, slot, lane, T, tmask, pbi, stage, acc, AS);
+      post_quartet<LA, LB, LC, LD, T>(A, s_hrr, pb, pk, sc, slot, lane, T, tmask, pbi, stage, acc, AS);
       __syncwarp(tmask);
     }
   }
