@@ -246,7 +246,7 @@ size_t slot_with_acc(const KernelEntry* e, int pcb, const KernelArgs& A) {
 }
 
 // The other streams of a run and their join events, made on first use.
-static int ensure_side_streams(igpu_plan* P, size_t n) {
+int ensure_side_streams(igpu_plan* P, size_t n) {
   while (P->side_ev.size() < n + 1) {  // event n forks, the others join
     cudaEvent_t ev;
     CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

@@ -1,6 +1,7 @@
 // Dense-tensor entry points: Basis::eri / eri_screened / eri_block,
 // EriBuilder fills and the packed symmetry-unique tensor
 // (src/integrals.rs, src/eri_builder.rs, src/packed_eri.rs).
+#include "host_copy.hpp"
 #include "plan_internal.hpp"
 
 extern "C" {
@@ -14,9 +15,11 @@ static int dense_like(igpu_plan* P, bool builder, const uint32_t* sub, size_t ns
   const size_t n = (size_t)P->nao;
   const size_t n4 = n * n * n * n;
   CK(P->d_dense.ensure(n4));
-  if (builder)
+  // rows of other bras keep the caller's content; a fill of every bra assigns
+  // every element
+  if (builder && sub)
     CK(cudaMemcpyAsync(P->d_dense.p, out, n4 * sizeof(double), cudaMemcpyHostToDevice, P->stream));
-  else
+  else if (!builder)
     CK(cudaMemsetAsync(P->d_dense.p, 0, n4 * sizeof(double), P->stream));
   TaskSet local;
   TaskSet* ts = &local;
@@ -84,8 +87,8 @@ static int dense_like(igpu_plan* P, bool builder, const uint32_t* sub, size_t ns
   uint32_t launches = 0;
   rc = run_tasks(P, *ts, A, P->stream, launches);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(out, P->d_dense.p, n4 * sizeof(double), cudaMemcpyDeviceToHost, P->stream));
-  CK(cudaStreamSynchronize(P->stream));
+  rc = copy_to_host(P, out, P->d_dense.p, n4 * sizeof(double), P->stream);
+  if (rc) return rc;
   // per-launch device times and quartet counts (igpu_last_stats / _profile)
   return collect_profile(P, 0, false);
 }
@@ -204,8 +207,8 @@ int igpu_eri_packed(igpu_plan* P, double threshold, const uint32_t* sub, size_t 
   uint32_t launches = 0;
   rc = run_tasks(P, *ts, A, s, launches);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(out, P->d_dense.p, len * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
+  rc = copy_to_host(P, out, P->d_dense.p, len * sizeof(double), s);
+  if (rc) return rc;
   P->last = igpu_stats{};
   P->last.launches = launches;
   return IGPU_OK;

@@ -1,6 +1,7 @@
 // Density-fitting entry points (src/df.rs): the auxiliary basis attached
 // to a plan, the 3-centre tensor, the 2-centre metric and the aux Schwarz
 // factors.
+#include "host_copy.hpp"
 #include "plan_internal.hpp"
 
 namespace {
@@ -264,9 +265,7 @@ int igpu_eri_3c(igpu_plan* P, const uint32_t* sub, size_t nsub, const uint8_t* k
   }
   int rc = run_df(P, ts, MODE_DF3, len);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(out, P->d_dense.p, len * sizeof(double), cudaMemcpyDeviceToHost, P->stream));
-  CK(cudaStreamSynchronize(P->stream));
-  return IGPU_OK;
+  return copy_to_host(P, out, P->d_dense.p, len * sizeof(double), P->stream);
 }
 
 }  // extern "C"

@@ -126,6 +126,14 @@ constexpr double kWideRounds = 3.0;
 // its last round is then at most a sixteenth of it.
 constexpr double kFullRounds = 16.0;
 
+// A plan's share in the pinned buffers of copy_to_host (host_copy.cpp).
+struct StageRef {
+  StageRef();
+  ~StageRef();
+  StageRef(const StageRef&) = delete;
+  StageRef& operator=(const StageRef&) = delete;
+};
+
 // Mixed-precision J/K task lists kept per plan (see igpu_plan::mixed_keys).
 constexpr size_t kMixedTaskSets = 4;
 
@@ -168,6 +176,7 @@ struct igpu_plan {
   // device
   cudaStream_t stream = nullptr;
   // the other streams of a run and the events that join them (run_tasks)
+  StageRef stage;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> side_ev;
   ~igpu_plan() {
@@ -256,6 +265,7 @@ void tune_record(igpu_plan* P, int m, bool grad, std::map<int, std::map<int, flo
 void tune_keep(igpu_plan* P, const std::map<int, std::map<int, float>>& best, bool bps);
 int tune_two_stage(igpu_plan* P, bool grad, const std::function<int()>& run);
 size_t slot_with_acc(const KernelEntry* e, int pcb, const KernelArgs& A);
+int ensure_side_streams(igpu_plan* P, size_t n);
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches);
 int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c = -1, int grad_terms_x = 0);
 std::unique_ptr<Launch> make_launch(igpu_plan* P, int pcb, int pck, bool fp32, const std::vector<int>& bras,
