@@ -270,28 +270,76 @@ void finite_quadrature(const GL& gl, int n, double T, double* x, double* w) {
   gauss_from_jacobi(al, be, n, x, w);
 }
 
-// Interpolating polynomial of degree nc - 1 through the values v[0..nc-1] at
-// the Chebyshev nodes node(j, nc), as coefficients of the powers of xi
+// The reference's tables, which carry its roots and weights: degree-16
+// Chebyshev fits on equal subintervals of [0, t_hi(n)], the fewest whose fits
+// stay within 2e-14 (src/math/rys.rs:230-515, xtask/src/gen_rys_tables.rs).
+// This build's polynomials pass through these fits and not through the
+// quadrature itself: the fits' own errors (up to 2e-14) reach elements with
+// cancellation, which the reference's results are compared on.
+constexpr int CHEB_NC = 17;
+constexpr int CHEB_SUB[MAX_ROOTS + 1] = {0, 9, 8, 8, 8, 9, 10, 10, 11, 12, 13, 13, 14, 15};
+
+double clenshaw(const double* c, double xi) {
+  double d = 0.0, dd = 0.0;
+  for (int k = CHEB_NC - 1; k >= 1; --k) {
+    const double sv = d;
+    d = 2.0 * xi * d - dd + c[k];
+    dd = sv;
+  }
+  return xi * d - dd + 0.5 * c[0];
+}
+
+// fits of the n roots and n weights on [a, b]: out[(i*2 + {0,1}) * CHEB_NC + k]
+void cheb_fit(const GL& gl, int n, double a, double b, double* out) {
+  double vx[CHEB_NC][MAX_ROOTS], vw[CHEB_NC][MAX_ROOTS];
+  for (int j = 0; j < CHEB_NC; ++j) {
+    const double y = std::cos(PI * ((double)j + 0.5) / (double)CHEB_NC);
+    finite_quadrature(gl, n, y * 0.5 * (b - a) + 0.5 * (b + a), vx[j], vw[j]);
+  }
+  for (int i = 0; i < n; ++i)
+    for (int k = 0; k < CHEB_NC; ++k) {
+      double sx = 0.0, sw = 0.0;
+      for (int j = 0; j < CHEB_NC; ++j) {
+        const double ck = std::cos(PI * (double)k * ((double)j + 0.5) / (double)CHEB_NC);
+        sx += vx[j][i] * ck;
+        sw += vw[j][i] * ck;
+      }
+      out[(i * 2 + 0) * CHEB_NC + k] = 2.0 / CHEB_NC * sx;
+      out[(i * 2 + 1) * CHEB_NC + k] = 2.0 / CHEB_NC * sw;
+    }
+}
+
+// Interpolating polynomial of degree NC - 1 through the values v[0..NC-1] at
+// the Chebyshev nodes node(j, NC), as coefficients of the powers of xi
 // (ascending): the Chebyshev sums by discrete orthogonality, expanded in long
 // double.  Their terms fall by 4^-k / k!, so the power basis on [-1, 1] is as
 // accurate as the Chebyshev one.
 double node(int j, int nc) { return std::cos(PI * ((double)j + 0.5) / (double)nc); }
-void power_fit(const double* v, int nc, double* out) {
-  long double mono[16] = {0}, t0[16] = {0}, t1[16] = {0}, t2[16];
-  t0[0] = 1.0L;  // T_k and T_{k-1} as powers
-  for (int k = 0; k < nc; ++k) {
-    long double s = 0.0L;
-    for (int j = 0; j < nc; ++j) s += (long double)v[j] * std::cos((long double)PI * k * (j + 0.5L) / nc);
-    s *= (k ? 2.0L : 1.0L) / nc;
-    for (int m = 0; m < nc; ++m) mono[m] += s * t0[m];
-    for (int m = 0; m < nc; ++m) t2[m] = (k == 0 ? 1.0L : 2.0L) * (m ? t0[m - 1] : 0.0L) - (k == 0 ? 0.0L : t1[m]);
-    for (int m = 0; m < nc; ++m) {
-      t1[m] = t0[m];
-      t0[m] = t2[m];
+template <int NC>
+struct PowerFit {
+  long double m[NC][NC] = {};  // coefficient = sum_j m[.][j] v[j]
+  PowerFit() {
+    long double t0[NC] = {1.0L}, t1[NC] = {0.0L}, t2[NC];  // T_k and T_{k-1} as powers
+    for (int k = 0; k < NC; ++k) {
+      for (int j = 0; j < NC; ++j) {
+        const long double ck = std::cos((long double)PI * k * (j + 0.5L) / NC) * (k ? 2.0L : 1.0L) / NC;
+        for (int p = 0; p < NC; ++p) m[p][j] += ck * t0[p];
+      }
+      for (int p = 0; p < NC; ++p) t2[p] = (k ? 2.0L : 1.0L) * (p ? t0[p - 1] : 0.0L) - (k ? t1[p] : 0.0L);
+      for (int p = 0; p < NC; ++p) {
+        t1[p] = t0[p];
+        t0[p] = t2[p];
+      }
     }
   }
-  for (int m = 0; m < nc; ++m) out[m] = (double)mono[m];
-}
+  void operator()(const double* v, double* out) const {
+    for (int p = 0; p < NC; ++p) {
+      long double s = 0.0L;
+      for (int j = 0; j < NC; ++j) s += m[p][j] * (long double)v[j];
+      out[p] = (double)s;
+    }
+  }
+};
 }  // namespace
 
 const RysTables& rys_tables() {
@@ -300,22 +348,40 @@ const RysTables& rys_tables() {
   std::call_once(once, [] {
     GL gl;
     constexpr int NC = rys_nc<double>(), NF = rys_nc<float>();
+    const PowerFit<NC> fit;
+    const PowerFit<NF> fit_f;
     T.coef.assign(rys_off<double>(MAX_ROOTS + 1), 0.0);
     T.coef_f.assign(rys_off<float>(MAX_ROOTS + 1), 0.0f);
     for (int n = 1; n <= MAX_ROOTS; ++n) {
+      const double t_hi = rys_t_hi(n), width = t_hi / CHEB_SUB[n];
+      const size_t cell = (size_t)2 * n * CHEB_NC;
+      std::vector<double> cheb(CHEB_SUB[n] * cell);
+      for (int k = 0; k < CHEB_SUB[n]; ++k) cheb_fit(gl, n, k * width, k * width + width, &cheb[k * cell]);
       for (int s = 0; s < rys_nsub(n); ++s) {
         double vx[NC][MAX_ROOTS], vw[NC][MAX_ROOTS];
-        for (int j = 0; j < NC; ++j) finite_quadrature(gl, n, s + 0.5 * (node(j, NC) + 1.0), vx[j], vw[j]);
+        for (int j = 0; j < NC; ++j) {
+          const double t = s + 0.5 * (node(j, NC) + 1.0);
+          if (t >= t_hi) {  // the end of the last interval, which no T reads
+            finite_quadrature(gl, n, t, vx[j], vw[j]);
+            continue;
+          }
+          const int k = std::min((int)(t / width), CHEB_SUB[n] - 1);
+          const double xi = (2.0 * t - (2 * k + 1) * width) / width;
+          for (int i = 0; i < n; ++i) {
+            vx[j][i] = clenshaw(&cheb[k * cell + (2 * i) * CHEB_NC], xi);
+            vw[j][i] = clenshaw(&cheb[k * cell + (2 * i + 1) * CHEB_NC], xi);
+          }
+        }
         for (int q = 0; q < 2 * n; ++q) {
           double v[NC], vf[NF], c[NC], cf[NF];
           for (int j = 0; j < NC; ++j) v[j] = q % 2 ? vw[j][q / 2] : vx[j][q / 2];
-          power_fit(v, NC, c);
+          fit(v, c);
           // the FP32 polynomial through the FP64 one's values
           for (int j = 0; j < NF; ++j) {
             vf[j] = 0.0;
             for (int m = NC - 1; m >= 0; --m) vf[j] = vf[j] * node(j, NF) + c[m];
           }
-          power_fit(vf, NF, cf);
+          fit_f(vf, cf);
           std::copy(c, c + NC, &T.coef[rys_off<double>(n) + (size_t)s * rys_row<double>(n) + q * NC]);
           std::copy(cf, cf + NF, &T.coef_f[rys_off<float>(n) + (size_t)s * rys_row<float>(n) + q * NF]);
         }
