@@ -298,9 +298,9 @@ static int ensure_kets(igpu_plan* P) {
 // fills a fraction of the device (the 120 (gg|gg) quartets of a 5-atom
 // molecule run on 30 of 148 SMs for 19 ms), and a launch of a few rounds
 // leaves it idle over its last quartets.  Longer launches gain nothing from
-// company and stay on `s`, one after another: each stream has a scratch region
-// of its own, and allocating one costs 50 us/MB.  The launch-shape tuner times
-// all launches one after another.
+// company and stay on `s`, one after another (their records then hold their own
+// times).  Each stream has a scratch region of its own.  The launch-shape tuner
+// times all launches one after another.
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches) {
   const bool grad = A.mode == MODE_GRAD;
   auto entry = [grad](int pcb, int pck) { return grad ? grad_entry(pcb, pck) : kernel_entry(pcb, pck); };
@@ -371,8 +371,6 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   auto doubles = [](const Planned& r) { return r.units * r.slot; };
   size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(kRunStreams, run.size()));
   std::vector<size_t> region;  // scratch doubles per stream
-  size_t largest = 0;
-  for (const Planned& r : run) largest = std::max(largest, doubles(r));
   for (;; ns = (ns + 1) / 2) {
     std::vector<double> load(ns, 0.0);
     region.assign(ns, 0);
@@ -382,8 +380,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       load[r.stream] += r.load;
       region[r.stream] = std::max(region[r.stream], doubles(r));
     }
-    if (ns == 1 || std::accumulate(region.begin(), region.end(), (size_t)0) <= std::max(2 * largest, kScratchBudget))
-      break;
+    if (ns == 1 || std::accumulate(region.begin(), region.end(), (size_t)0) <= kScratchBudget) break;
   }
   if (ns == 1) std::iota(order.begin(), order.end(), (size_t)0);
   CK(P->d_scratch.ensure(std::accumulate(region.begin(), region.end(), (size_t)0)));

@@ -117,9 +117,11 @@ struct LaunchLog {
 // Streams that a run's class launches are spread over, the caller's among
 // them (device connections by default: more would share one queue).
 constexpr size_t kRunStreams = 8;
-// Scratch doubles (256 MiB, or twice the largest launch's) above which a run
-// uses fewer streams, each of which needs a scratch region of its own.
-constexpr size_t kScratchBudget = (size_t)1 << 25;
+// Scratch doubles (4 GiB) above which a run uses fewer streams, each of which
+// needs a scratch region of its own.  256 MiB (or twice the largest launch's)
+// left a 5-atom g molecule two streams and cost it 52 against 35 ms, an f
+// gradient 39 against 28 ms; allocating the 4 GiB adds 3 ms to a first run.
+constexpr size_t kScratchBudget = (size_t)1 << 29;
 // Rounds of 128 quartets per SM from which a launch takes the wide kernels.
 constexpr double kWideRounds = 3.0;
 // Quartets per resident team from which a launch fills the device by itself:
