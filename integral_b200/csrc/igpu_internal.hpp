@@ -153,9 +153,11 @@ struct JKDev {
   const double* bounds;  // ndens x nsh x nsh  (density_shell_bounds)
   double* J;             // symmetric: one-orientation accumulators J', K'
   double* K;             //   (J = (J' + J'^T)/2 added by the finalize pass)
-  int ndens;
+  int ndens;             // matrices contracted: nscreen, or 2 nscreen (symmetric parts, then antisymmetric ones)
+  int nscreen;           // densities the screening sees (bounds)
+  int nj;                // first matrices that have a Coulomb part
   int want_k;
-  int symmetric;         // every density symmetric (bitwise)
+  int symmetric;         // every matrix symmetric or antisymmetric (bitwise): one-orientation sums
   double threshold;
 };
 

@@ -185,6 +185,43 @@ cudaError_t launch_symmetrize_add(const double* H, double* out, int nmat, int na
   return cudaGetLastError();
 }
 
+// The symmetric parts of nmat matrices, then (anti) their antisymmetric ones.
+__global__ void split_symmetry_kernel(const double* __restrict__ D, double* __restrict__ out, int nmat, int nao,
+                                      int anti) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t n2 = (size_t)nao * nao;
+  if (t >= n2 * nmat) return;
+  const size_t d = t / n2, r = (t % n2) / nao, c = t % nao;
+  const double x = D[t], y = D[d * n2 + c * nao + r];
+  out[t] = 0.5 * (x + y);
+  if (anti) out[n2 * nmat + t] = 0.5 * (x - y);
+}
+
+cudaError_t launch_split_symmetry(const double* D, double* out, int nmat, int nao, int anti, cudaStream_t s) {
+  const size_t n = (size_t)nao * nao * nmat;
+  if (n == 0) return cudaSuccess;
+  split_symmetry_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(D, out, nmat, nao, anti);
+  return cudaGetLastError();
+}
+
+// out[d] += (H[d] + H[d]^T) / 2 + (H[nmat + d] - H[nmat + d]^T) / 2: the exchange
+// of general densities from the one-orientation accumulators of their parts.
+__global__ void join_symmetry_add_kernel(const double* __restrict__ H, double* __restrict__ out, int nmat, int nao) {
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t n2 = (size_t)nao * nao;
+  if (t >= n2 * nmat) return;
+  const size_t d = t / n2, r = (t % n2) / nao, c = t % nao, tt = d * n2 + c * nao + r;
+  const double* HA = H + n2 * nmat;
+  out[t] += 0.5 * (H[t] + H[tt]) + 0.5 * (HA[t] - HA[tt]);
+}
+
+cudaError_t launch_join_symmetry_add(const double* H, double* out, int nmat, int nao, cudaStream_t s) {
+  const size_t n = (size_t)nao * nao * nmat;
+  if (n == 0) return cudaSuccess;
+  join_symmetry_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(H, out, nmat, nao);
+  return cudaGetLastError();
+}
+
 // out[i] = (float)in[i]: the FP32 copy of the densities read by the FP32
 // launches of the mixed J/K path.
 __global__ void to_float_kernel(const double* __restrict__ in, float* __restrict__ out, size_t n) {

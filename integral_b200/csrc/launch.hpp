@@ -61,6 +61,8 @@ cudaError_t launch_wide(const WideEntry* e, bool fp32, int grid, const KernelArg
 cudaError_t launch_shell_block_max(const double* D, int nmat, const DevShell* sh, int nsh, int nao,
                                    int symmetrise, double* out, cudaStream_t s);
 cudaError_t launch_symmetrize_add(const double* H, double* out, int nmat, int nao, cudaStream_t s);
+cudaError_t launch_split_symmetry(const double* D, double* out, int nmat, int nao, int anti, cudaStream_t s);
+cudaError_t launch_join_symmetry_add(const double* H, double* out, int nmat, int nao, cudaStream_t s);
 cudaError_t launch_to_float(const double* in, float* out, size_t n, cudaStream_t s);
 cudaError_t launch_ket_copy(const PairD* pairs, const PrimPairD* prims, const int* list, int n, int maxprim,
                             double* out, float* outf, cudaStream_t s);

@@ -57,7 +57,7 @@ int enqueue(igpu_batch* b, TaskSet& ts, double threshold, int mixed, double prim
   A.mode = MODE_JK;
   A.jk.D = b->d_D.p;
   A.jk.bounds = b->d_bounds.p;
-  A.jk.ndens = 1;
+  A.jk.ndens = A.jk.nscreen = A.jk.nj = 1;
   A.jk.want_k = want_k;
   A.jk.symmetric = sym;
   A.jk.threshold = threshold;

@@ -65,9 +65,24 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
   A.mode = MODE_JK;
   A.jk.D = d_dens;
   A.jk.bounds = P->d_bounds.p;
-  A.jk.ndens = ndens;
+  A.jk.ndens = A.jk.nscreen = A.jk.nj = ndens;
   A.jk.want_k = want_k ? 1 : 0;
   A.jk.symmetric = asym == 0 ? 1 : 0;
+  // FP64 builds of general densities run the one-orientation sums on their
+  // symmetric parts (all of J, and K's symmetric part) and antisymmetric parts
+  // (the rest of K): six sums a matrix in the specialised kernels against
+  // fourteen in the general ones (19.2 against 15.2 ms for two densities of an
+  // 11-atom molecule).  Mixed builds keep the general sums, which read the
+  // FP64 densities in every launch.
+  const int nmat = want_k ? 2 * ndens : ndens;
+  const bool parts = asym != 0 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
+  if (parts) {
+    CK(P->d_parts.ensure((size_t)P->nao * P->nao * nmat));
+    CK(launch_split_symmetry(d_dens, P->d_parts.p, ndens, P->nao, want_k ? 1 : 0, s));
+    A.jk.D = P->d_parts.p;
+    A.jk.ndens = nmat;
+    A.jk.symmetric = 1;
+  }
   A.jk.threshold = threshold;
   A.prim_cut = prim_cut;
   A.bra_bitmap = bra_subset ? P->d_bitmap.p : nullptr;
@@ -84,8 +99,9 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
     CK(cudaMemsetAsync(P->d_Jh.p, 0, n2 * sizeof(double), s));
     A.jk.J = P->d_Jh.p;
     if (want_k) {
-      CK(P->d_Kh.ensure(n2));
-      CK(cudaMemsetAsync(P->d_Kh.p, 0, n2 * sizeof(double), s));
+      const size_t nk = parts ? 2 * n2 : n2;
+      CK(P->d_Kh.ensure(nk));
+      CK(cudaMemsetAsync(P->d_Kh.p, 0, nk * sizeof(double), s));
       A.jk.K = P->d_Kh.p;
     }
   } else {
@@ -97,7 +113,9 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
   if (rc) return rc;
   if (A.jk.symmetric) {
     CK(launch_symmetrize_add(P->d_Jh.p, d_J, ndens, P->nao, s));
-    if (want_k) CK(launch_symmetrize_add(P->d_Kh.p, d_K, ndens, P->nao, s));
+    if (want_k)
+      CK(parts ? launch_join_symmetry_add(P->d_Kh.p, d_K, ndens, P->nao, s)
+               : launch_symmetrize_add(P->d_Kh.p, d_K, ndens, P->nao, s));
   }
   CK(cudaStreamSynchronize(s));
   return collect_profile(P, ndens, true);
@@ -185,7 +203,7 @@ int igpu_jk_device_static(igpu_plan* P, const double* d_dens, int ndens, double 
   A.counters = nullptr;
   A.jk.D = d_dens;
   A.jk.bounds = sb.bounds;
-  A.jk.ndens = ndens;
+  A.jk.ndens = A.jk.nscreen = A.jk.nj = ndens;
   A.jk.want_k = want_k ? 1 : 0;
   A.jk.symmetric = 0;
   A.jk.threshold = threshold;

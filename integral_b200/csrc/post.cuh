@@ -72,6 +72,7 @@ struct Screen {
   bool keep;
   bool swapped;       // reference bra is the evaluation ket pair
   uint64_t mask;      // densities this quartet contributes to
+  uint64_t dens;      // matrices contracted: mask, repeated for the antisymmetric parts
   int i, j, k, l;     // reference canonical shells
   double degeneracy;  // gradient: images of the canonical quartet
 };
@@ -114,7 +115,7 @@ __device__ __forceinline__ Screen screen_quartet(const KernelArgs& A, const Pair
   s.j = rb.j;
   s.k = rk.i;
   s.l = rk.j;
-  s.mask = 1;
+  s.mask = s.dens = 1;
   s.keep = true;
   s.degeneracy = 1.0;
   if (A.bra_bitmap && !((__ldg(A.bra_bitmap + (rb.tri >> 5)) >> (rb.tri & 31)) & 1u)) {
@@ -134,7 +135,7 @@ __device__ __forceinline__ Screen screen_quartet(const KernelArgs& A, const Pair
     }
     const int n = A.nsh;
     uint64_t mask = 0;
-    for (int d = 0; d < A.jk.ndens; ++d) {
+    for (int d = 0; d < A.jk.nscreen; ++d) {
       const double* bd = A.jk.bounds + (size_t)d * n * n;
       double db = fmax(fmax(fmax(fmax(fmax(__ldg(bd + (size_t)s.i * n + s.j), __ldg(bd + (size_t)s.k * n + s.l)),
                                       __ldg(bd + (size_t)s.i * n + s.k)),
@@ -144,6 +145,7 @@ __device__ __forceinline__ Screen screen_quartet(const KernelArgs& A, const Pair
       if (pair_bound * db >= A.jk.threshold) mask |= 1ull << d;
     }
     s.mask = mask;
+    s.dens = A.jk.ndens > A.jk.nscreen ? mask | mask << A.jk.nscreen : mask;
     s.keep = mask != 0;
   } else if (A.mode == MODE_GRAD) {
     // src/direct_grad.rs:347-370
@@ -435,6 +437,12 @@ __device__ __forceinline__ void flush_bra_acc(const KernelArgs& A, double* acc, 
 // element read feeds up to DCH products.
 constexpr int JK_DCH = 4;
 
+// Of the matrices d0 + k with bit k of m set, those with a Coulomb part.
+__device__ __forceinline__ unsigned coulomb_mask(const JKDev& jk, int d0, unsigned m) {
+  const int n = jk.nj - d0;
+  return n >= JK_DCH ? m : (n > 0 ? m & ((1u << n) - 1u) : 0u);
+}
+
 template <int DCH>
 __device__ __forceinline__ void jk_sym_chunk(const KernelArgs& A, const double* B, const int dims[4],
                                              const int offs[4], const double wt[6], int nterm, int d0, unsigned m,
@@ -456,6 +464,7 @@ __device__ __forceinline__ void jk_sym_chunk(const KernelArgs& A, const double* 
     const int t = q < e1 ? 0 : (q < e2 ? 1 : (q < e3 ? 2 : (q < e4 ? 3 : (q < e5 ? 4 : 5))));
     const int base = t == 0 ? 0 : (t == 1 ? e1 : (t == 2 ? e2 : (t == 3 ? e3 : (t == 4 ? e4 : e5))));
     const double w = t == 0 ? wt[0] : (t == 1 ? wt[1] : (t == 2 ? wt[2] : (t == 3 ? wt[3] : (t == 4 ? wt[4] : wt[5]))));
+    const unsigned mt = t < 2 ? coulomb_mask(A.jk, d0, m) : m;
     const int u = nib(PU, t), v = nib(PV, t), s = nib(PS, t), tt = nib(PT, t);
     const int r = q - base;
     const int nv = dim(v);
@@ -474,19 +483,19 @@ __device__ __forceinline__ void jk_sym_chunk(const KernelArgs& A, const double* 
         const double b = br[(size_t)it * stt];
 #pragma unroll
         for (int k = 0; k < DCH; ++k)
-          if ((m >> k) & 1u) sum[k] += b * __ldg(dr + (size_t)k * n2 + it);
+          if ((mt >> k) & 1u) sum[k] += b * __ldg(dr + (size_t)k * n2 + it);
       }
     }
     if (t == 0) {
 #pragma unroll
       for (int k = 0; k < DCH; ++k)
-        if ((m >> k) & 1u) acc[(1 + (size_t)(d0 + k) * nab + r) * as] += w * sum[k];
+        if ((mt >> k) & 1u) acc[(1 + (size_t)(d0 + k) * nab + r) * as] += w * sum[k];
     } else {
       double* out = t == 1 ? A.jk.J : A.jk.K;
       const size_t o = (size_t)(off(u) + iu) * nao + off(v) + iv;
 #pragma unroll
       for (int k = 0; k < DCH; ++k)
-        if ((m >> k) & 1u) atomicAdd(out + (size_t)(d0 + k) * n2 + o, w * sum[k]);
+        if ((mt >> k) & 1u) atomicAdd(out + (size_t)(d0 + k) * n2 + o, w * sum[k]);
     }
   }
 }
@@ -967,7 +976,7 @@ __device__ __forceinline__ void post_quartet(const KernelArgs& A, const int* hrr
   const int offs[4] = {s0.off, s1.off, s2.off, s3.off};
   switch (A.mode) {
     case MODE_JK:
-      consume_jk(A, B, dims, offs, shl, sc.mask, lane, T, acc, as, pb_index, tmask, stage);
+      consume_jk(A, B, dims, offs, shl, sc.dens, lane, T, acc, as, pb_index, tmask, stage);
       break;
     case MODE_DENSE:
       consume_dense(A, B, dims, offs, shl, lane, T);
@@ -1062,12 +1071,15 @@ __device__ __forceinline__ void post_quartet_jk_cart(const KernelArgs& A, const 
   const X w0 = W(0) + W(1) + W(2) + W(3), w1 = W(4) + W(5) + W(6) + W(7);
   const X w2 = W(0) + W(4), w3 = W(1) + W(5), w4 = W(2) + W(6), w5 = W(3) + W(7);
   const unsigned long long live = A.jk.ndens >= 64 ? ~0ull : ((1ull << A.jk.ndens) - 1ull);
-  const uint64_t mask = sc.mask & live;
+  const uint64_t mask = sc.dens & live;
   for (int d0 = 0; d0 < A.jk.ndens; d0 += JK_DCH) {
     const unsigned m = (unsigned)((mask >> d0) & ((1u << JK_DCH) - 1u));
     if (!m) continue;
-    jk_term_ct<0, 1, 2, 3, N0, N1, N2, N3, T, true, X>(A, B, offs, w0, d0, m, acc, lane);
-    if (w1 != X(0)) jk_term_ct<2, 3, 0, 1, N0, N1, N2, N3, T, false, X>(A, B, offs, w1, d0, m, A.jk.J, lane);
+    const unsigned mj = coulomb_mask(A.jk, d0, m);
+    if (mj) {
+      jk_term_ct<0, 1, 2, 3, N0, N1, N2, N3, T, true, X>(A, B, offs, w0, d0, mj, acc, lane);
+      if (w1 != X(0)) jk_term_ct<2, 3, 0, 1, N0, N1, N2, N3, T, false, X>(A, B, offs, w1, d0, mj, A.jk.J, lane);
+    }
     if (A.jk.want_k) {
       if (w2 != X(0)) jk_term_ct<0, 2, 1, 3, N0, N1, N2, N3, T, false, X>(A, B, offs, w2, d0, m, A.jk.K, lane);
       if (w3 != X(0)) jk_term_ct<1, 2, 0, 3, N0, N1, N2, N3, T, false, X>(A, B, offs, w3, d0, m, A.jk.K, lane);
@@ -1118,12 +1130,15 @@ __device__ __forceinline__ void post_quartet_jk_sph(const KernelArgs& A, const P
   const X w0 = W(0) + W(1) + W(2) + W(3), w1 = W(4) + W(5) + W(6) + W(7);
   const X w2 = W(0) + W(4), w3 = W(1) + W(5), w4 = W(2) + W(6), w5 = W(3) + W(7);
   const unsigned long long live = A.jk.ndens >= 64 ? ~0ull : ((1ull << A.jk.ndens) - 1ull);
-  const uint64_t mask = sc.mask & live;
+  const uint64_t mask = sc.dens & live;
   for (int d0 = 0; d0 < A.jk.ndens; d0 += JK_DCH) {
     const unsigned m = (unsigned)((mask >> d0) & ((1u << JK_DCH) - 1u));
     if (!m) continue;
-    jk_term_ct<0, 1, 2, 3, F0, F1, F2, F3, T, true, X>(A, B, offs, w0, d0, m, acc, lane);
-    if (w1 != X(0)) jk_term_ct<2, 3, 0, 1, F0, F1, F2, F3, T, false, X>(A, B, offs, w1, d0, m, A.jk.J, lane);
+    const unsigned mj = coulomb_mask(A.jk, d0, m);
+    if (mj) {
+      jk_term_ct<0, 1, 2, 3, F0, F1, F2, F3, T, true, X>(A, B, offs, w0, d0, mj, acc, lane);
+      if (w1 != X(0)) jk_term_ct<2, 3, 0, 1, F0, F1, F2, F3, T, false, X>(A, B, offs, w1, d0, mj, A.jk.J, lane);
+    }
     if (A.jk.want_k) {
       if (w2 != X(0)) jk_term_ct<0, 2, 1, 3, F0, F1, F2, F3, T, false, X>(A, B, offs, w2, d0, m, A.jk.K, lane);
       if (w3 != X(0)) jk_term_ct<1, 2, 0, 3, F0, F1, F2, F3, T, false, X>(A, B, offs, w3, d0, m, A.jk.K, lane);

@@ -160,7 +160,8 @@ __device__ __forceinline__ void thread_jk(const KernelArgs& A, const V* B, const
     const V* Dm = dens_of<V>(A.jk) + d * n2;
     double* J = A.jk.J + d * n2;
     // J'[A a][B b] (accumulated over the bra's quartets)
-    {
+    const bool want_j = d < A.jk.nj;
+    if (want_j) {
       V dcd[N2 * N3];
 #pragma unroll
       for (int c = 0; c < N2; ++c)
@@ -178,7 +179,7 @@ __device__ __forceinline__ void thread_jk(const KernelArgs& A, const V* B, const
         }
     }
     // J'[C c][D d]
-    if (wcd != V(0)) {
+    if (want_j && wcd != V(0)) {
       V dab[N0 * N1];
 #pragma unroll
       for (int i = 0; i < N0; ++i)
@@ -292,7 +293,7 @@ __device__ __forceinline__ void thread_post_jk(const KernelArgs& A, const V* G, 
     acc[0] = (double)pbi;
   }
   if constexpr (!SPH) {
-    thread_jk<P::NA, P::NB, P::NC, P::ND, V>(A, blk, offs, w, sc.mask, acc);
+    thread_jk<P::NA, P::NB, P::NC, P::ND, V>(A, blk, offs, w, sc.dens, acc);
   } else {
     constexpr int F0 = 2 * LA + 1, F1 = 2 * LB + 1, F2 = 2 * LC + 1, F3 = 2 * LD + 1;
     V t1[F0 * P::NB * P::NC * P::ND];
@@ -303,7 +304,7 @@ __device__ __forceinline__ void thread_post_jk(const KernelArgs& A, const V* G, 
     c2s_axis<2, F0, F1, P::NC, P::ND, F2, V>(t2, t3, A.c2s + A.c2s_off[LC]);
     V t4[F0 * F1 * F2 * F3];
     c2s_axis<3, F0, F1, F2, P::ND, F3, V>(t3, t4, A.c2s + A.c2s_off[LD]);
-    thread_jk<F0, F1, F2, F3, V>(A, t4, offs, w, sc.mask, acc);
+    thread_jk<F0, F1, F2, F3, V>(A, t4, offs, w, sc.dens, acc);
   }
 }
 

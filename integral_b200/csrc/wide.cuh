@@ -196,6 +196,7 @@ __device__ __forceinline__ void wide_post(const KernelArgs& A, const R* G, const
     const R* Dm = dens_of<R>(A.jk) + dn * n2;
     double* J = A.jk.J + dn * n2;
     double* K = want_k ? A.jk.K + dn * n2 : nullptr;
+    const bool want_j = dn < A.jk.nj;
     R jab[KEEP_AB ? NAB : 1], kad[NK][NA], kbd[NK][NB];
     double* const ja = acc + ((size_t)1 + (size_t)dn * NAB) * 32;
 #pragma unroll
@@ -224,20 +225,22 @@ __device__ __forceinline__ void wide_post(const KernelArgs& A, const R* G, const
           dbc[b] = want_k ? __ldg(Dm + (ob + b) * nao + oc + c) : R(0);
         }
         auto term = [&](int d, const R (&B)[NAB], R (&kadd)[NA], R (&kbdd)[NB]) {
-          const R dcd = __ldg(Dm + (oc + c) * nao + od + d);
-          R jcd = R(0);
+          if (want_j) {
+            const R dcd = __ldg(Dm + (oc + c) * nao + od + d);
+            R jcd = R(0);
 #pragma unroll
-          for (int a = 0; a < NA; ++a)
+            for (int a = 0; a < NA; ++a)
 #pragma unroll
-            for (int b = 0; b < NB; ++b) {
-              const R v = B[b * NA + a];
-              if constexpr (KEEP_AB)
-                jab[a * NB + b] += v * dcd;
-              else
-                ja[(a * NB + b) * 32] += (double)(wab * (v * dcd));
-              jcd += v * __ldg(Dm + (oa + a) * nao + ob + b);
-            }
-          if (wcd != R(0)) atomicAdd(J + (oc + c) * nao + od + d, (double)(wcd * jcd));
+              for (int b = 0; b < NB; ++b) {
+                const R v = B[b * NA + a];
+                if constexpr (KEEP_AB)
+                  jab[a * NB + b] += v * dcd;
+                else
+                  ja[(a * NB + b) * 32] += (double)(wab * (v * dcd));
+                jcd += v * __ldg(Dm + (oa + a) * nao + ob + b);
+              }
+            if (wcd != R(0)) atomicAdd(J + (oc + c) * nao + od + d, (double)(wcd * jcd));
+          }
           if (want_k) {
             R dad[NA], dbd[NB];
 #pragma unroll
@@ -326,9 +329,9 @@ __device__ __forceinline__ void wide_post(const KernelArgs& A, const R* G, const
             if (wbd != R(0)) atomicAdd(K + (ob + b) * nao + od + d, (double)(wbd * kbd[d][b]));
         }
     }
-    if constexpr (KEEP_AB) {
+    if (KEEP_AB && want_j) {
 #pragma unroll
-      for (int q = 0; q < NAB; ++q) ja[q * 32] += (double)(wab * jab[q]);
+      for (int q = 0; q < (KEEP_AB ? NAB : 1); ++q) ja[q * 32] += (double)(wab * jab[q]);
     }
   }
 }
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(128, 2) wide_kernel(KernelArgs A) {
         if (wi == 0) {
           s_bra[g * 32 + lane] = keep ? pbi : -1;
           s_ket[g * 32 + lane] = pki;
-          s_mask[g * 32 + lane] = sc.mask;
+          s_mask[g * 32 + lane] = sc.dens;
           if (keep) cnt.add(sc, pb, pk, A.fp32);
         }
         if (!__any_sync(0xffffffffu, keep)) continue;

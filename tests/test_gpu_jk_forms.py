@@ -1,0 +1,58 @@
+"""Branches of the J/K launches that the other parity tests do not set apart.
+
+General densities of an FP64 build run on their symmetric and antisymmetric
+parts up to 32 of them (64 matrices) and on the general eight-image sums
+beyond; jk_device_static always runs the latter.  One-thread launches of few
+quartets share each quartet among up to 16 lanes, by primitive pairs of the
+bra: molecules of one to a few atoms and contractions of 1, 3 and 5 primitives
+take every lane count, against the oracle."""
+import numpy as np
+import pytest
+
+import integral_b200 as ib
+import oracle_py as O
+from integral_b200 import systems as S
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float(abs(a - b).max() / abs(b).max())
+
+
+@pytest.mark.parametrize("spherical", [False, True, None], ids=["cart", "sph", "both"])
+@pytest.mark.parametrize("ndens, want_k", [(1, True), (3, False), (32, True), (33, True)])
+def test_general_densities(spherical, ndens, want_k):
+    import torch
+
+    shells = S.jk_system(natom=2, side=3.0, ndens=1)["shells"]
+    for k, s in enumerate(shells):
+        s["spherical"] = k % 2 == 0 if spherical is None else spherical
+    dc = ib.Basis(shells).direct_contractor()
+    n = dc.nao()
+    D = torch.tensor(np.random.default_rng(3).normal(size=(ndens, n, n)), device="cuda")
+    J, K, J0, K0 = (torch.zeros_like(D) for _ in range(4))
+    dc.jk_device(D.data_ptr(), ndens, J.data_ptr(), K.data_ptr(), 1e-13, want_exchange=want_k)
+    q = dc.last_stats()["quartets"]
+    dc.jk_device_static(D.data_ptr(), ndens, J0.data_ptr(), K0.data_ptr(), 1e-13, want_exchange=want_k)
+    torch.cuda.synchronize()
+    assert q > 0 and rel(J, J0) < 1e-12
+    if want_k:
+        assert rel(K, K0) < 1e-12
+
+
+@pytest.mark.parametrize("natom", [1, 2, 4])
+@pytest.mark.parametrize("nprim", [1, 3, 5])
+def test_shared_quartets_of_small_launches(natom, nprim):
+    rng = np.random.default_rng(10 * natom + nprim)
+    centers = S.place_atoms(rng, natom, 4.0, 1.5)
+    shells = S.build_shells(rng, centers, "ssp", nprim, 0.2, 2.5, 0.2, 1.0)
+    D = S.densities(rng, S.nao_of(shells), 2, 2)
+    dc = ib.Basis(shells).direct_contractor()
+    J, K = dc.jk(D, 1e-12)
+    st = dc.last_stats()
+    Jo, Ko, cnt, hsh = O.OracleBasis(shells).direct_jk(D, 1e-12)
+    assert st["quartets"] == cnt and st["quartet_hash"] == hsh
+    assert rel(J, Jo) < 1e-12 and rel(K, Ko) < 1e-12
+    gpu, ref = ib.Basis(shells).eri(), O.OracleBasis(shells).eri()
+    assert float(np.max(np.abs(gpu - ref))) < 1e-13 * max(1.0, float(np.max(np.abs(ref))))
