@@ -171,7 +171,10 @@ __host__ __device__ constexpr GradPassPlan make_grad_plan(int la, int lb, int lc
 // else the team of 8, 16 or 32 lanes with the least lane time per root by a
 // count of issue slots: the 2D tables of each pass (recurrences and their
 // shared-memory stores) and, per row slot, the row's loads and the columns'
-// products and sums, idle lanes of the last row slot included.
+// products and sums, idle lanes of the last row slot included.  A smaller team
+// has to save a tenth: its quartets take longer, which shows where a class has
+// few of them ((32|32) of a 5-atom molecule, 320 quartets: 4.0 ms on 32 lanes,
+// 4.8 ms on 16).
 __host__ __device__ constexpr int grad_team_for(int la, int lb, int lc, int ld) {
   if (g_acc_total(la, lb, lc, ld) <= 40) return 1;
   const int nev = la + lb + 1, nfv = lc + ld + 1;
@@ -182,7 +185,7 @@ __host__ __device__ constexpr int grad_team_for(int la, int lb, int lc, int ld) 
     const int cols = g_main_cols(lc, ld);
     const int c = p.npass * 12 * (nev + 1) * (nfv + 1) +
                   rl * t * (6 * (nfv + 1) + cols + g_acc_before(la, lb, lc, ld, cols) / 2);
-    if (c < cost) {
+    if (t == 32 || c < cost - cost / 10) {
       cost = c;
       best = t;
     }
