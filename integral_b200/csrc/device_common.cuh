@@ -120,8 +120,7 @@ __device__ __forceinline__ int addr_lz(int a) { return (c_addr_lxyz[a] >> 16) & 
 // ----------------------------------------------------------------- Rys
 
 // Whether a kernel stages its N-root table in shared memory: the
-// one-thread classes and the FP32 teams up to four roots (at most 39 KB in
-// FP64, 14 KB in FP32 per block).  FP64 teams, whose shared memory holds the
+// one-thread classes and the FP32 teams up to four roots (at most 46 KB per block).  FP64 teams, whose shared memory holds the
 // recurrence tables of their primitive quartets, and larger N read it through
 // L1 (a team evaluates one root per lane, a small part of its work).
 template <int N, typename R>
@@ -130,7 +129,7 @@ __host__ __device__ constexpr bool rys_staged(int team) {
 }
 template <int N, typename R>
 __host__ __device__ constexpr int rys_smem(int team) {
-  return rys_staged<N, R>(team) ? rys_nsub(N) * rys_row<R>(N) : 4;
+  return rys_staged<N, R>(team) ? rys_nsub<R>(N) * rys_row<R>(N) : 4;
 }
 
 template <int N, typename R>
@@ -149,18 +148,18 @@ __device__ __forceinline__ void stage_rys_table(R* s_tab) {
     constexpr int PER = 16 / sizeof(R);
     const uint4* src = reinterpret_cast<const uint4*>(rys_global<N, R>());
     uint4* dst = reinterpret_cast<uint4*>(s_tab);
-    for (int i = threadIdx.x; i < rys_nsub(N) * rys_row<R>(N) / PER; i += blockDim.x) dst[i] = __ldg(src + i);
+    for (int i = threadIdx.x; i < rys_nsub<R>(N) * rys_row<R>(N) / PER; i += blockDim.x) dst[i] = __ldg(src + i);
   }
   __syncthreads();
 }
 
-// One polynomial of a table row (16-byte aligned; GLOBAL: read through the
-// read-only path) by Horner's scheme.  The series on unit intervals replaces
-// 17-term Chebyshev sums on intervals about six times as wide: 11 FP64
-// operations and 6 wide reads a value for 32 and 17, and xi without rounding
-// or division.
-template <bool GLOBAL>
+// One polynomial of NC coefficients of a table row (16-byte aligned; GLOBAL:
+// read through the read-only path) by Horner's scheme.  The short intervals
+// replace 17-term Chebyshev sums on intervals about six wide, and their position
+// needs no rounding or division.
+template <int NC, bool GLOBAL>
 __device__ __forceinline__ double rys_poly(const double* c, double xi) {
+  static_assert(NC % 2 == 0, "two coefficients a read");
   const double2* q = reinterpret_cast<const double2*>(c);
   auto at = [q](int k) {
     if constexpr (GLOBAL)
@@ -168,18 +167,19 @@ __device__ __forceinline__ double rys_poly(const double* c, double xi) {
     else
       return q[k];
   };
-  double2 t = at(5);
+  double2 t = at(NC / 2 - 1);
   double v = fma(t.y, xi, t.x);
 #pragma unroll
-  for (int k = 4; k >= 0; --k) {
+  for (int k = NC / 2 - 2; k >= 0; --k) {
     t = at(k);
     v = fma(v, xi, t.y);
     v = fma(v, xi, t.x);
   }
   return v;
 }
-template <bool GLOBAL>
+template <int NC, bool GLOBAL>
 __device__ __forceinline__ float rys_poly(const float* c, float xi) {
+  static_assert(NC % 4 == 0, "four coefficients a read");
   const float4* q = reinterpret_cast<const float4*>(c);
   auto at = [q](int k) {
     if constexpr (GLOBAL)
@@ -187,21 +187,24 @@ __device__ __forceinline__ float rys_poly(const float* c, float xi) {
     else
       return q[k];
   };
-  const float4 u = at(1), t = at(0);
-  float v = fmaf(u.w, xi, u.z);
-  v = fmaf(v, xi, u.y);
-  v = fmaf(v, xi, u.x);
-  v = fmaf(v, xi, t.w);
-  v = fmaf(v, xi, t.z);
-  v = fmaf(v, xi, t.y);
-  return fmaf(v, xi, t.x);
+  float v = 0.f;
+#pragma unroll
+  for (int k = NC / 4 - 1; k >= 0; --k) {
+    const float4 t = at(k);
+    v = k == NC / 4 - 1 ? t.w : fmaf(v, xi, t.w);
+    v = fmaf(v, xi, t.z);
+    v = fmaf(v, xi, t.y);
+    v = fmaf(v, xi, t.x);
+  }
+  return v;
 }
 
 // Interval of T < rys_t_hi(N) and the position in it.
-template <typename R>
+template <int N, typename R>
 __device__ __forceinline__ int rys_interval(R T, R& xi) {
-  const int s = (int)T;
-  xi = R(2) * (T - R(s)) - R(1);
+  const R u = T * R(rys_div<R>(N));
+  const int s = (int)u;
+  xi = R(2) * (u - R(s)) - R(1);
   return s;
 }
 
@@ -226,11 +229,11 @@ __device__ __forceinline__ void rys_roots_s(const R* tab, R T, R* x, R* w) {
     return;
   }
   R xi;
-  const R* row = tab + rys_interval(T, xi) * rys_row<R>(N);
+  const R* row = tab + rys_interval<N>(T, xi) * rys_row<R>(N);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    x[i] = rys_poly<GLOBAL>(row + (2 * i) * rys_nc<R>(), xi);
-    w[i] = rys_poly<GLOBAL>(row + (2 * i + 1) * rys_nc<R>(), xi);
+    x[i] = rys_poly<rys_nc<R>(N), GLOBAL>(row + (2 * i) * rys_nc<R>(N), xi);
+    w[i] = rys_poly<rys_nc<R>(N), GLOBAL>(row + (2 * i + 1) * rys_nc<R>(N), xi);
   }
 }
 
@@ -248,9 +251,9 @@ __device__ __forceinline__ void rys_root_one(const R* tab, R T, int r, R& x, R& 
     return;
   }
   R xi;
-  const R* c = tab + rys_interval(T, xi) * rys_row<R>(N) + 2 * r * rys_nc<R>();
-  x = rys_poly<GLOBAL>(c, xi);
-  w = rys_poly<GLOBAL>(c + rys_nc<R>(), xi);
+  const R* c = tab + rys_interval<N>(T, xi) * rys_row<R>(N) + 2 * r * rys_nc<R>(N);
+  x = rys_poly<rys_nc<R>(N), GLOBAL>(c, xi);
+  w = rys_poly<rys_nc<R>(N), GLOBAL>(c + rys_nc<R>(N), xi);
 }
 
 // Per-axis Rys vertical recurrence g[n][m], n <= NE (bra power on A),

@@ -309,37 +309,48 @@ void cheb_fit(const GL& gl, int n, double a, double b, double* out) {
     }
 }
 
-// Interpolating polynomial of degree NC - 1 through the values v[0..NC-1] at
-// the Chebyshev nodes node(j, NC), as coefficients of the powers of xi
-// (ascending): the Chebyshev sums by discrete orthogonality, expanded in long
-// double.  Their terms fall by 4^-k / k!, so the power basis on [-1, 1] is as
+// Interpolating polynomial through the values v[0..nc-1] at the Chebyshev nodes
+// node(j, nc), as coefficients of the powers of xi (ascending): the Chebyshev
+// sums by discrete orthogonality, expanded in long double.  Their terms fall by
+// (h / 4)^k / k! on intervals of length h, so the power basis on [-1, 1] is as
 // accurate as the Chebyshev one.
 double node(int j, int nc) { return std::cos(PI * ((double)j + 0.5) / (double)nc); }
-template <int NC>
 struct PowerFit {
-  long double m[NC][NC] = {};  // coefficient = sum_j m[.][j] v[j]
-  PowerFit() {
-    long double t0[NC] = {1.0L}, t1[NC] = {0.0L}, t2[NC];  // T_k and T_{k-1} as powers
-    for (int k = 0; k < NC; ++k) {
-      for (int j = 0; j < NC; ++j) {
-        const long double ck = std::cos((long double)PI * k * (j + 0.5L) / NC) * (k ? 2.0L : 1.0L) / NC;
-        for (int p = 0; p < NC; ++p) m[p][j] += ck * t0[p];
+  int nc;
+  long double m[16][16] = {};  // coefficient p = sum_j m[p][j] v[j]
+  explicit PowerFit(int nc_) : nc(nc_) {
+    long double t0[16] = {1.0L}, t1[16] = {0.0L}, t2[16];  // T_k and T_{k-1} as powers
+    for (int k = 0; k < nc; ++k) {
+      for (int j = 0; j < nc; ++j) {
+        const long double ck = std::cos((long double)PI * k * (j + 0.5L) / nc) * (k ? 2.0L : 1.0L) / nc;
+        for (int p = 0; p < nc; ++p) m[p][j] += ck * t0[p];
       }
-      for (int p = 0; p < NC; ++p) t2[p] = (k ? 2.0L : 1.0L) * (p ? t0[p - 1] : 0.0L) - (k ? t1[p] : 0.0L);
-      for (int p = 0; p < NC; ++p) {
+      for (int p = 0; p < nc; ++p) t2[p] = (k ? 2.0L : 1.0L) * (p ? t0[p - 1] : 0.0L) - (k ? t1[p] : 0.0L);
+      for (int p = 0; p < nc; ++p) {
         t1[p] = t0[p];
         t0[p] = t2[p];
       }
     }
   }
-  void operator()(const double* v, double* out) const {
-    for (int p = 0; p < NC; ++p) {
-      long double s = 0.0L;
-      for (int j = 0; j < NC; ++j) s += m[p][j] * (long double)v[j];
-      out[p] = (double)s;
-    }
-  }
 };
+
+// The n-point table of precision R: `values(t, v)` gives root 0, weight 0, ...
+template <typename R, typename V>
+void fill_table(int n, const V& values, std::vector<R>& out) {
+  const int nc = rys_nc<R>(n);
+  const PowerFit fit(nc);
+  std::vector<double> v((size_t)nc * 2 * n);
+  for (int s = 0; s < rys_nsub<R>(n); ++s) {
+    for (int j = 0; j < nc; ++j) values((s + 0.5 * (node(j, nc) + 1.0)) / rys_div<R>(n), &v[(size_t)j * 2 * n]);
+    R* row = &out[rys_off<R>(n) + (size_t)s * rys_row<R>(n)];
+    for (int q = 0; q < 2 * n; ++q)
+      for (int p = 0; p < nc; ++p) {
+        long double c = 0.0L;
+        for (int j = 0; j < nc; ++j) c += fit.m[p][j] * (long double)v[(size_t)j * 2 * n + q];
+        row[q * nc + p] = (R)c;
+      }
+  }
+}
 }  // namespace
 
 const RysTables& rys_tables() {
@@ -347,9 +358,6 @@ const RysTables& rys_tables() {
   static std::once_flag once;
   std::call_once(once, [] {
     GL gl;
-    constexpr int NC = rys_nc<double>(), NF = rys_nc<float>();
-    const PowerFit<NC> fit;
-    const PowerFit<NF> fit_f;
     T.coef.assign(rys_off<double>(MAX_ROOTS + 1), 0.0);
     T.coef_f.assign(rys_off<float>(MAX_ROOTS + 1), 0.0f);
     for (int n = 1; n <= MAX_ROOTS; ++n) {
@@ -357,35 +365,20 @@ const RysTables& rys_tables() {
       const size_t cell = (size_t)2 * n * CHEB_NC;
       std::vector<double> cheb(CHEB_SUB[n] * cell);
       for (int k = 0; k < CHEB_SUB[n]; ++k) cheb_fit(gl, n, k * width, k * width + width, &cheb[k * cell]);
-      for (int s = 0; s < rys_nsub(n); ++s) {
-        double vx[NC][MAX_ROOTS], vw[NC][MAX_ROOTS];
-        for (int j = 0; j < NC; ++j) {
-          const double t = s + 0.5 * (node(j, NC) + 1.0);
-          if (t >= t_hi) {  // the end of the last interval, which no T reads
-            finite_quadrature(gl, n, t, vx[j], vw[j]);
-            continue;
-          }
-          const int k = std::min((int)(t / width), CHEB_SUB[n] - 1);
-          const double xi = (2.0 * t - (2 * k + 1) * width) / width;
-          for (int i = 0; i < n; ++i) {
-            vx[j][i] = clenshaw(&cheb[k * cell + (2 * i) * CHEB_NC], xi);
-            vw[j][i] = clenshaw(&cheb[k * cell + (2 * i + 1) * CHEB_NC], xi);
-          }
+      // roots and weights at t; beyond t_hi (the end of the last interval,
+      // which no T reads) from the quadrature
+      auto values = [&](double t, double* v) {
+        double x[MAX_ROOTS], w[MAX_ROOTS];
+        if (t >= t_hi) finite_quadrature(gl, n, t, x, w);
+        const int k = std::min((int)(t / width), CHEB_SUB[n] - 1);
+        const double xi = (2.0 * t - (2 * k + 1) * width) / width;
+        for (int i = 0; i < n; ++i) {
+          v[2 * i] = t >= t_hi ? x[i] : clenshaw(&cheb[k * cell + (2 * i) * CHEB_NC], xi);
+          v[2 * i + 1] = t >= t_hi ? w[i] : clenshaw(&cheb[k * cell + (2 * i + 1) * CHEB_NC], xi);
         }
-        for (int q = 0; q < 2 * n; ++q) {
-          double v[NC], vf[NF], c[NC], cf[NF];
-          for (int j = 0; j < NC; ++j) v[j] = q % 2 ? vw[j][q / 2] : vx[j][q / 2];
-          fit(v, c);
-          // the FP32 polynomial through the FP64 one's values
-          for (int j = 0; j < NF; ++j) {
-            vf[j] = 0.0;
-            for (int m = NC - 1; m >= 0; --m) vf[j] = vf[j] * node(j, NF) + c[m];
-          }
-          fit_f(vf, cf);
-          std::copy(c, c + NC, &T.coef[rys_off<double>(n) + (size_t)s * rys_row<double>(n) + q * NC]);
-          std::copy(cf, cf + NF, &T.coef_f[rys_off<float>(n) + (size_t)s * rys_row<float>(n) + q * NF]);
-        }
-      }
+      };
+      fill_table<double>(n, values, T.coef);
+      fill_table<float>(n, values, T.coef_f);
       // generalized Gauss-Laguerre(-1/2): a_k = 2k + 1/2, b_k = k(k - 1/2), b_0 = sqrt(pi)
       double a[MAX_ROOTS], b[MAX_ROOTS];
       for (int k = 0; k < n; ++k) {

@@ -86,27 +86,40 @@ struct PairD {
 };
 
 // Rys tables of the n-point quadrature: below rys_t_hi(n) the roots and
-// weights are polynomials on unit intervals of T, in xi = 2 (T - s) - 1 on
-// [s, s + 1] (exact in both precisions), 12 coefficients in FP64 (within
-// 3e-15 of the quadrature for every n) and 8 in FP32 (4e-11, below its
-// rounding), ascending.  Row s holds root 0, weight 0, root 1, ...; its stride
+// weights are polynomials on intervals of T of length 1 / rys_div(n) (a power
+// of two, so that the position xi in [-1, 1] is exact in both precisions), with
+// ascending coefficients.  Row s holds root 0, weight 0, root 1, ...; its stride
 // is an odd multiple of 16 bytes, so that the 16-byte reads of lanes in
 // different intervals start in different shared-memory banks.  Above it the
 // generalised Gauss-Laguerre limit holds.
+//
+// A one-thread kernel spends most of its shared-memory rate on these rows (its
+// lanes are in different intervals), so in FP64 n <= 2, where little else is
+// done per primitive quartet, takes 8 coefficients on quarters (as far as a
+// block's 48 KB allow): 1.1 to 1.2 times as fast as 12 on unit intervals in
+// (20|00), (10|10), (10|00).  The others take 12, FP32 8 (4 on sixteenths gained
+// nothing there), on unit intervals.
 template <typename R>
-IGPU_HD constexpr int rys_nc() {
-  return sizeof(R) == 8 ? 12 : 8;
+IGPU_HD constexpr int rys_div(int n) {
+  return sizeof(R) == 8 && n <= 2 ? 4 : 1;
+}
+template <typename R>
+IGPU_HD constexpr int rys_nc(int n) {
+  return sizeof(R) == 8 && n > 2 ? 12 : 8;
 }
 IGPU_HD constexpr double rys_t_hi(int n) { return 30.5 + 5.0 * n; }
-IGPU_HD constexpr int rys_nsub(int n) { return 31 + 5 * n; }
+template <typename R>
+IGPU_HD constexpr int rys_nsub(int n) {
+  return (31 + 5 * n) * rys_div<R>(n);
+}
 template <typename R>
 IGPU_HD constexpr int rys_row(int n) {
-  return 2 * n * rys_nc<R>() + 16 / (int)sizeof(R);
+  return 2 * n * rys_nc<R>(n) + 16 / (int)sizeof(R);
 }
 template <typename R>
 IGPU_HD constexpr int rys_off(int n) {
   int o = 0;
-  for (int k = 1; k < n; ++k) o += rys_nsub(k) * rys_row<R>(k);
+  for (int k = 1; k < n; ++k) o += rys_nsub<R>(k) * rys_row<R>(k);
   return o;
 }
 
