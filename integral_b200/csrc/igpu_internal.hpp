@@ -232,6 +232,7 @@ struct KernelArgs {
   const unsigned* bra_bitmap;  // optional: reference bra pairs to keep (bit per pair)
   unsigned long long* work_counter;  // next unclaimed task (dynamic chunks)
   unsigned long long chunk;          // tasks claimed per grab (per warp)
+  int split;             // one-thread kernels: lanes sharing a quartet's bra primitives (power of two)
   size_t acc_offset;     // slot offset of the running bra-block J accumulators
   int kinds;             // 0 all shells Cartesian, 1 all spherical, 2 mixed
   double omega;          // 0: Coulomb 1/r; > 0: long-range erf(omega r)/r

@@ -309,6 +309,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     size_t li, grid, stream;
     size_t slot, acc;         // scratch doubles per unit, and before its J sums
     size_t units;             // teams (wide kernels: blocks) in the grid
+    int split;                // lanes per quartet of a one-thread launch
     const KernelEntry* e;
     const WideEntry* wide;    // its one-thread-per-quartet kernel runs instead
     double load;
@@ -332,6 +333,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     Planned r{};
     r.li = li;
     r.e = e;
+    r.split = 1;
     if (A.mode == MODE_JK && A.jk.symmetric && A.kinds == 0 && L->total >= wide_min_tasks())
       r.wide = wide_entry(L->pcb, L->pck, L->fp32);
     const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
@@ -341,7 +343,15 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
       r.slot = r.acc + 128 * sums;
     } else {
-      r.grid = grid_for(e, L->fp32, L->total, bps_cap);
+      // a quartet of a small one-thread launch takes several lanes, as far as
+      // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
+      // (tuned launches keep the shape they were tuned in)
+      const bool tuned = P->tune_mult || P->tune_bps || P->tuned_mult.count(tune_key(L->pcb, L->pck, L->fp32, grad));
+      if (e->team == 1 && !grad && !tuned)
+        while (r.split < 16 && r.split < L->prim_pairs &&
+               L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
+          r.split *= 2;
+      r.grid = grid_for(e, L->fp32, L->total * r.split, bps_cap);
       r.units = r.grid * (128 / e->team);
       // one-thread classes finish symmetric J/K of one shell kind in registers
       r.acc = e->team == 1 && A.mode == MODE_JK && A.jk.symmetric && A.kinds != 2 ? 0 : e->slot;
@@ -351,11 +361,11 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     // a team's lanes
     const int la = pc_la_host(L->pcb), lb = L->pcb - la * (la + 1) / 2;
     const int lc = pc_la_host(L->pck), ld = L->pck - lc * (lc + 1) / 2;
-    const double teams = r.wide ? (double)r.grid * 128 : (double)r.units;
+    const double teams = r.wide ? (double)r.grid * 128 : (double)r.units / r.split;
     const double np = (double)L->prim_pairs * L->prim_pairs;
     r.full = (double)L->total >= kFullRounds * teams;
     r.load = std::ceil((double)L->total / teams) * np *
-             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / (r.wide ? 1 : e->team);
+             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / (r.wide ? 1 : e->team * r.split);
     if (!grad && (r.wide || e->team == 1) && L->ket_class >= 0) {
       const int rc = ensure_kets(P);
       if (rc) return rc;
@@ -438,13 +448,14 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     A.slot_doubles = pl.slot;
     A.acc_offset = pl.acc;
     A.work_counter = lg.work.p + li;
-    // tasks a warp claims per grab: (32 / team) x mult.  Untuned, mult is 16,
+    // tasks a warp claims per grab: the quartets it runs side by side x mult.  Untuned, mult is 16,
     // or less when the launch has so few tasks that 16 would leave warps of
     // the grid without work: every warp should find at least four grabs,
     // which matters for classes of few, heavy quartets (g shells, small
     // molecules)
     const unsigned long long warps = (unsigned long long)grid * 4;
-    const unsigned long long fill = L->total / (4 * warps * (unsigned long long)(32 / e->team));
+    const unsigned long long per_warp = 32 / (e->team * pl.split);  // quartets side by side
+    const unsigned long long fill = L->total / (4 * warps * per_warp);
     int mult = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(16, fill));
     if (P->tune_mult) {
       mult = P->tune_mult;
@@ -452,9 +463,13 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       auto t = P->tuned_mult.find(tune_key(L->pcb, L->pck, L->fp32, grad));
       if (t != P->tuned_mult.end()) mult = t->second;
     }
-    A.chunk = (unsigned long long)(32 / e->team) * mult;
+    A.chunk = per_warp * mult;
+    A.split = pl.split;
     // a wide block takes 128 quartets at a time
-    if (pl.wide) A.chunk = 128 * std::max<unsigned long long>(1, std::min<unsigned long long>(4, L->total / (512 * grid)));
+    if (pl.wide) {
+      A.chunk = 128;
+      while (A.chunk < 512 && L->total >= 8 * A.chunk * grid) A.chunk *= 2;
+    }
     A.counters = counters ? counters + li : nullptr;
     A.task.bra_pair = L->bra_pair.p;
     A.task.ket_pairs = L->ket_list;

@@ -122,6 +122,9 @@ constexpr size_t kRunStreams = 8;
 // left a 5-atom g molecule two streams and cost it 52 against 35 ms, an f
 // gradient 39 against 28 ms; allocating the 4 GiB adds 3 ms to a first run.
 constexpr size_t kScratchBudget = (size_t)1 << 29;
+// Lanes per SM up to which a one-thread launch of few quartets is widened, by
+// lanes that share a quartet (KernelArgs::split).
+constexpr unsigned long long kSplitLanes = 256;
 // Rounds of 128 quartets per SM from which a launch takes the wide kernels.
 constexpr double kWideRounds = 3.0;
 // Quartets per resident team from which a launch fills the device by itself:

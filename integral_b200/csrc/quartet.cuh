@@ -145,7 +145,7 @@ constexpr int MAX_SURV = 256;
 
 template <int LA, int LB, int LC, int LD, typename R>
 __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* tab, const PairD& pb,
-                                                  const PairD& pk, int kpos, R (&G)[ClassShape<LA, LB, LC, LD>::NG]) {
+                                                  const PairD& pk, int kpos, int sub, int split, R (&G)[ClassShape<LA, LB, LC, LD>::NG]) {
   using S = ClassShape<LA, LB, LC, LD>;
   constexpr int NE = S::NE, NF = S::NF, NR = S::NR;
 #pragma unroll
@@ -159,7 +159,7 @@ __device__ __forceinline__ void accumulate_thread(const KernelArgs& A, const R* 
     acy = (float)(sa.cy - sc.cy);
     acz = (float)(sa.cz - sc.cz);
   }
-  for (int ip = 0; ip < pb.nprim; ++ip) {
+  for (int ip = sub; ip < pb.nprim; ip += split) {
     for (int kq = 0; kq < pk.nprim; ++kq) {
       QuartetHdr<R> h;
       if constexpr (sizeof(R) == 4) {
@@ -481,8 +481,12 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
   // Warps claim contiguous chunks of the task list; the teams of a warp
   // interleave inside a chunk, so consecutive quartets (same bra pair, same
   // primitive-pair count) stay on the same lanes.
-  constexpr int TPW = 32 / T;
-  const int tw = (threadIdx.x & 31) / T;
+  // In a one-thread launch of few quartets, `split` lanes share one: each sums
+  // every split-th bra primitive, and the first finishes the quartet.
+  const int split = T == 1 && A.split > 1 ? A.split : 1;
+  const int TPW = 32 / (T * split);
+  const int tw = (threadIdx.x & 31) / (T * split);
+  const int sub = T == 1 ? (threadIdx.x & 31) % split : 0;
   for (;;) {
     unsigned long long base = 0;
     if ((threadIdx.x & 31) == 0) base = atomicAdd(A.work_counter, A.chunk);
@@ -498,10 +502,17 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
       const PairD pk = A.pairs[pki];
       Screen sc = screen_quartet(A, pb, pk);
       if (!sc.keep) continue;
-      if (lane == 0) cnt.add(sc, pb, pk, A.fp32);
+      if (lane == 0 && sub == 0) cnt.add(sc, pb, pk, A.fp32);
       if constexpr (T == 1) {
         R G[S::NG];
-        accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, kpos, G);
+        accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, kpos, sub, split, G);
+        if (split > 1) {
+          const unsigned group = (split == 32 ? 0xffffffffu : (1u << split) - 1u) << ((threadIdx.x & 31) - sub);
+#pragma unroll
+          for (int q = 0; q < S::NG; ++q)
+            for (int o = 1; o < split; o *= 2) G[q] += __shfl_xor_sync(group, G[q], o);
+          if (sub) continue;
+        }
         if (use_acc && A.kinds != 2) {
           // the post phase runs in the launch's arithmetic (FP32 launches
           // read the FP32 densities); J/K accumulate in FP64
