@@ -293,8 +293,9 @@ static int ensure_kets(igpu_plan* P) {
 // The launches are independent (J/K, gradient and counters are summed with
 // atomics, every other mode stores each element once), so those with fewer
 // than kFullRounds quartets per resident team are spread over up to
-// kRunStreams streams, longest first, each onto the stream with the least
-// estimated load; `s` waits for all of them.  A class of a small molecule
+// kRunStreams streams (fewer where their grids fill the device anyway), longest
+// first, each onto the stream with the least estimated load; `s` waits for all
+// of them.  A class of a small molecule
 // fills a fraction of the device (the 120 (gg|gg) quartets of a 5-atom
 // molecule run on 30 of 148 SMs for 19 ms), and a launch of a few rounds
 // leaves it idle over its last quartets.  Longer launches gain nothing from
@@ -313,7 +314,8 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     const KernelEntry* e;
     const WideEntry* wide;    // its one-thread-per-quartet kernel runs instead
     double load;
-    bool full;  // enough rounds to fill the device by itself
+    bool full;    // enough rounds to fill the device by itself
+    double fill;  // share of the resident blocks that its grid takes
   };
   std::vector<Planned> run;
   for (size_t li = 0; li < nl; ++li) {
@@ -338,7 +340,9 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       r.wide = wide_entry(L->pcb, L->pck, L->fp32);
     const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
     if (r.wide) {
-      r.grid = grid_blocks(L->total, 128, blocks_per_sm(r.wide, L->fp32), bps_cap);
+      const int bps = blocks_per_sm(r.wide, L->fp32);
+      r.grid = grid_blocks(L->total, 128, bps, bps_cap);
+      r.fill = (double)r.grid / ((double)bps * sm_count());
       r.units = r.grid;
       r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
       r.slot = r.acc + 128 * sums;
@@ -352,6 +356,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
                L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
           r.split *= 2;
       r.grid = grid_for(e, L->fp32, L->total * r.split, bps_cap);
+      r.fill = (double)r.grid / ((double)blocks_per_sm(e, L->fp32) * sm_count());
       r.units = r.grid * (128 / e->team);
       // one-thread classes finish symmetric J/K of one shell kind in registers
       r.acc = e->team == 1 && A.mode == MODE_JK && A.jk.symmetric && A.kinds != 2 ? 0 : e->slot;
@@ -379,7 +384,15 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     return run[x].full != run[y].full ? run[x].full : run[x].load > run[y].load;
   });
   auto doubles = [](const Planned& r) { return r.units * r.slot; };
-  size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(kRunStreams, run.size()));
+  // as many streams as it takes to fill the device about twice over
+  double busy = 0.0, work = 0.0;
+  for (const Planned& r : run)
+    if (!r.full) {
+      busy += r.load * std::min(1.0, r.fill);
+      work += r.load;
+    }
+  const size_t want = work > 0.0 ? (size_t)std::min((double)kRunStreams, std::ceil(2.0 * work / busy)) : 1;
+  size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(want, run.size()));
   std::vector<size_t> region;  // scratch doubles per stream
   for (;; ns = (ns + 1) / 2) {
     std::vector<double> load(ns, 0.0);
