@@ -173,8 +173,9 @@ __host__ __device__ constexpr GradPassPlan make_grad_plan(int la, int lb, int lc
 // shared-memory stores) and, per row slot, the row's loads and the columns'
 // products and sums, idle lanes of the last row slot included.  A smaller team
 // has to save a tenth: its quartets take longer, which shows where a class has
-// few of them ((32|32) of a 5-atom molecule, 320 quartets: 4.0 ms on 32 lanes,
-// 4.8 ms on 16).
+// few of them (the spherical f gradient of 5 atoms: 28.3 ms with (32|32),
+// (32|31), (32|21) and (33|21) on 16 lanes for a count up to 7 % smaller,
+// 26.6 ms on 32).
 __host__ __device__ constexpr int grad_team_for(int la, int lb, int lc, int ld) {
   if (g_acc_total(la, lb, lc, ld) <= 40) return 1;
   const int nev = la + lb + 1, nfv = lc + ld + 1;

@@ -71,9 +71,10 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
   // FP64 builds of general densities run the one-orientation sums on their
   // symmetric parts (all of J, and K's symmetric part) and antisymmetric parts
   // (the rest of K): six sums a matrix in the specialised kernels against
-  // fourteen in the general ones (19.2 against 15.2 ms for two densities of an
-  // 11-atom molecule).  Mixed builds keep the general sums, which read the
-  // FP64 densities in every launch.
+  // fourteen in the general ones (two densities of an 11-atom molecule:
+  // 12.6 ms, 19.2 before, a little of it from shorter Rys tables).  Mixed
+  // builds keep the general sums, which read the FP64 densities in every
+  // launch.
   const int nmat = want_k ? 2 * ndens : ndens;
   const bool parts = asym != 0 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
   if (parts) {

@@ -411,7 +411,9 @@ __device__ __forceinline__ int screen_prims(const KernelArgs& A, const PairD& pb
 
 // Minimum resident 128-thread blocks per SM (register budget): team
 // classes 3 (168 registers; measured faster than the unconstrained
-// allocation, whose unrolled J/K sums take up to 255), thread-per-quartet
+// allocation, whose unrolled J/K sums take up to 255), FP64 teams with an f or
+// g bra 2 (their row tiles spill at 168: mixed J/K of 8 atoms with spherical f
+// shells 198 against 181 ms), thread-per-quartet
 // classes by the size of their register-resident G table (spilling large
 // tables costs more than the occupancy gains).
 #ifndef IGPU_FP32_TEAM_MINB
@@ -420,7 +422,7 @@ __device__ __forceinline__ int screen_prims(const KernelArgs& A, const PairD& pb
 template <int LA, int LB, int LC, int LD, typename R>
 __host__ __device__ constexpr int quartet_min_blocks() {
   return team_size<LA, LB, LC, LD>() > 1
-             ? (sizeof(R) == 4 ? IGPU_FP32_TEAM_MINB : 3)
+             ? (sizeof(R) == 4 ? IGPU_FP32_TEAM_MINB : (LA >= 3 ? 2 : 3))
              : (ClassShape<LA, LB, LC, LD>::NG <= 9 ? 5 : (ClassShape<LA, LB, LC, LD>::NG <= 27 ? 3 : 1));
 }
 
