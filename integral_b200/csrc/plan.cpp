@@ -349,9 +349,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     } else {
       // a quartet of a small one-thread launch takes several lanes, as far as
       // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
-      // (tuned launches keep the shape they were tuned in)
-      const bool tuned = P->tune_mult || P->tune_bps || P->tuned_mult.count(tune_key(L->pcb, L->pck, L->fp32, grad));
-      if (e->team == 1 && !grad && !tuned)
+      if (e->team == 1 && !grad)
         while (r.split < 16 && r.split < L->prim_pairs &&
                L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
           r.split *= 2;
@@ -507,7 +505,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     r.lc = pc_la_host(L->pck);
     r.ld = L->pck - r.lc * (r.lc + 1) / 2;
     r.fp32 = L->fp32 ? 1 : 0;
-    r.team = pl.wide ? 1 : e->team;
+    r.team = pl.wide ? 1 : e->team * pl.split;
     r.grid = (uint32_t)grid;
     r.tasks = L->total;
     r.chunk = (uint32_t)A.chunk;
