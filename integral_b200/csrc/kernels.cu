@@ -260,15 +260,19 @@ cudaError_t launch_ket_copy(const PairD* pairs, const PrimPairD* prims, const in
   return cudaGetLastError();
 }
 
-// flag[0] += 1 for every element with M[r][c] != M[c][r] (bitwise compare).
+// flag[0]: bit 0 with any element M[r][c] != M[c][r] (bitwise compare), bit 1
+// with any that is infinite or NaN, or whose sum with its mirror overflows.
 __global__ void asym_count_kernel(const double* __restrict__ D, int nmat, int nao, unsigned long long* flag) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t n2 = (size_t)nao * nao;
   if (t >= n2 * nmat) return;
   const size_t d = t / n2, r = (t % n2) / nao, c = t % nao;
-  if (c <= r) return;
+  if (c < r) return;
   const double* M = D + d * n2;
-  if (__double_as_longlong(M[r * nao + c]) != __double_as_longlong(M[c * nao + r])) atomicAdd(flag, 1ull);
+  const double x = M[r * nao + c], y = M[c * nao + r];
+  unsigned long long f = __double_as_longlong(x) != __double_as_longlong(y) ? 1 : 0;
+  if (!(fabs(x) + fabs(y) < INFINITY)) f |= 2;
+  if (f) atomicOr(flag, f);
 }
 
 cudaError_t launch_asym_count(const double* D, int nmat, int nao, unsigned long long* flag, cudaStream_t s) {

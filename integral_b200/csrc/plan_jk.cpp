@@ -67,16 +67,17 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
   A.jk.bounds = P->d_bounds.p;
   A.jk.ndens = A.jk.nscreen = A.jk.nj = ndens;
   A.jk.want_k = want_k ? 1 : 0;
-  A.jk.symmetric = asym == 0 ? 1 : 0;
+  A.jk.symmetric = asym & 1 ? 0 : 1;
   // FP64 builds of general densities run the one-orientation sums on their
   // symmetric parts (all of J, and K's symmetric part) and antisymmetric parts
   // (the rest of K): six sums a matrix in the specialised kernels against
   // fourteen in the general ones (two densities of an 11-atom molecule:
   // 12.6 ms, 19.2 before, a little of it from shorter Rys tables).  Mixed
   // builds keep the general sums, which read the FP64 densities in every
-  // launch.
+  // launch, and so do densities with an infinity or NaN, which the parts would
+  // spread.
   const int nmat = want_k ? 2 * ndens : ndens;
-  const bool parts = asym != 0 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
+  const bool parts = asym == 1 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
   if (parts) {
     CK(P->d_parts.ensure((size_t)P->nao * P->nao * nmat));
     CK(launch_split_symmetry(d_dens, P->d_parts.p, ndens, P->nao, want_k ? 1 : 0, s));

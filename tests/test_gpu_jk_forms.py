@@ -41,6 +41,28 @@ def test_general_densities(spherical, ndens, want_k):
         assert rel(K, K0) < 1e-12
 
 
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_general_density_without_finite_parts(value):
+    """One element that the symmetric and antisymmetric parts cannot hold: the
+    elements of J and K that the general sums leave finite stay so."""
+    import torch
+
+    dc = ib.Basis(S.jk_system(natom=2, side=3.0, ndens=1)["shells"]).direct_contractor()
+    n = dc.nao()
+    D = np.random.default_rng(5).normal(size=(1, n, n))
+    D[0, 1, 4] = value
+    D = torch.tensor(D, device="cuda")
+    J, K, J0, K0 = (torch.zeros_like(D) for _ in range(4))
+    dc.jk_device(D.data_ptr(), 1, J.data_ptr(), K.data_ptr(), 1e-13)
+    dc.jk_device_static(D.data_ptr(), 1, J0.data_ptr(), K0.data_ptr(), 1e-13)
+    torch.cuda.synchronize()
+    for a, b in ((J, J0), (K, K0)):
+        ok = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), ok)
+        if bool(ok.any()):
+            assert rel(a[ok], b[ok]) < 1e-12
+
+
 @pytest.mark.parametrize("natom", [1, 2, 4])
 @pytest.mark.parametrize("nprim", [1, 3, 5])
 def test_shared_quartets_of_small_launches(natom, nprim):
