@@ -51,10 +51,10 @@ sys.path.insert(0, ROOT)
 METRIC = "Fock J/K build quartets/s (FP32-mixed, <=1e-6 Eh vs FP64) on B200"
 UNIT = "quartets/s"
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one full-size launch of
-# this workload's kernels, from a one-pass ncu capture on a B200
-# (profiles/quartet_kernel_2120_fp32_traffic.md); bytes per launch.
-NCU_TRAFFIC = {"quartet_kernel(21|20) fp32": 68.02e6 + 70.12e6}
+# dram__bytes_read.sum + dram__bytes_write.sum of one full-size launch of this
+# workload's kernels as they are, by kernel name, from a one-pass ncu capture;
+# bytes per launch.  No capture of the present kernels has been taken.
+NCU_TRAFFIC = {}
 
 
 def parse():
