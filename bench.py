@@ -261,8 +261,8 @@ def dense_bench(args):
                    "l2": "flushed before every step (256 MB write)"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": None,
-                     "note": "algorithmic bytes = the 68 MB tensor written once per step, over the summed "
-                             "device time of the step's launches (%s peak)" % peak_kind},
+                     "note": "algorithmic bytes = the 68 MB tensor written once per step, over the "
+                             "device time of the step's overlapping launches (%s peak)" % peak_kind},
         "top_launch": {"class": "(%d%d|%d%d)" % (top["la"], top["lb"], top["lc"], top["ld"]), "ms": top["ms"]},
         "gpu_launches": launches,
         "clocks": clocks,
