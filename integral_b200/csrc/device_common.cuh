@@ -199,21 +199,12 @@ __device__ __forceinline__ float rys_poly(const float* c, float xi) {
   return v;
 }
 
-// Interval of T < rys_t_hi(N) and the position in it.
-template <int N, typename R>
-__device__ __forceinline__ int rys_interval(R T, R& xi) {
-  const R u = T * R(rys_div<R>(N));
-  const int s = (int)u;
-  xi = R(2) * (u - R(s)) - R(1);
-  return s;
-}
-
 // N-point Rys quadrature at parameter T (src/math/rys.rs:174-215): the
 // generalized-Laguerre(-1/2) limit above the crossover, else the tables.
 // x = squared roots, w = weights.
 template <int N, bool GLOBAL, typename R>
 __device__ __forceinline__ void rys_roots_s(const R* tab, R T, R* x, R* w) {
-  if (T >= R(rys_t_hi(N))) {
+  if (!rys_tabulated(N, T)) {
     const R r = rsqrt(T);
     const R inv_t = R(1) / T;
 #pragma unroll
@@ -229,7 +220,7 @@ __device__ __forceinline__ void rys_roots_s(const R* tab, R T, R* x, R* w) {
     return;
   }
   R xi;
-  const R* row = tab + rys_interval<N>(T, xi) * rys_row<R>(N);
+  const R* row = tab + rys_interval(N, T, xi) * rys_row<R>(N);
 #pragma unroll
   for (int i = 0; i < N; ++i) {
     x[i] = rys_poly<rys_nc<R>(N), GLOBAL>(row + (2 * i) * rys_nc<R>(N), xi);
@@ -240,7 +231,7 @@ __device__ __forceinline__ void rys_roots_s(const R* tab, R T, R* x, R* w) {
 // Root r of the N-point quadrature.
 template <int N, bool GLOBAL, typename R>
 __device__ __forceinline__ void rys_root_one(const R* tab, R T, int r, R& x, R& w) {
-  if (T >= R(rys_t_hi(N))) {
+  if (!rys_tabulated(N, T)) {
     if constexpr (sizeof(R) == 8) {
       x = c_lag_x[N - 1][r] / T;
       w = c_lag_w[N - 1][r] * R(0.5) * rsqrt(T);
@@ -251,7 +242,7 @@ __device__ __forceinline__ void rys_root_one(const R* tab, R T, int r, R& x, R& 
     return;
   }
   R xi;
-  const R* c = tab + rys_interval<N>(T, xi) * rys_row<R>(N) + 2 * r * rys_nc<R>(N);
+  const R* c = tab + rys_interval(N, T, xi) * rys_row<R>(N) + 2 * r * rys_nc<R>(N);
   x = rys_poly<rys_nc<R>(N), GLOBAL>(c, xi);
   w = rys_poly<rys_nc<R>(N), GLOBAL>(c + rys_nc<R>(N), xi);
 }

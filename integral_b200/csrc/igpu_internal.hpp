@@ -112,6 +112,22 @@ template <typename R>
 IGPU_HD constexpr int rys_nsub(int n) {
   return (31 + 5 * n) * rys_div<R>(n);
 }
+// The tables hold T < rys_t_hi(n).  A NaN compares false: the closed form, which
+// takes no index, returns it.
+template <typename R>
+IGPU_HD constexpr bool rys_tabulated(int n, R T) {
+  return T < R(rys_t_hi(n));
+}
+// Interval of a tabulated T and the position in it.  A negative T (a negative
+// exponent gives one) extrapolates the first interval.
+template <typename R>
+IGPU_HD inline int rys_interval(int n, R T, R& xi) {
+  const R u = T * R(rys_div<R>(n));
+  int s = (int)u;
+  s = s < 0 ? 0 : s;
+  xi = R(2) * (u - R(s)) - R(1);
+  return s;
+}
 template <typename R>
 IGPU_HD constexpr int rys_row(int n) {
   return 2 * n * rys_nc<R>(n) + 16 / (int)sizeof(R);
