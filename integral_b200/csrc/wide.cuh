@@ -61,8 +61,10 @@ __device__ __forceinline__ void wide_sync(int gt) {
 }
 
 // Rows [E0, E0 + ROWS) of the tables of the group's 32 quartets.
+// A lane whose quartet has no primitives, or none at all (!has), runs along on
+// another lane's pairs (the caller's choice) with weight zero.
 template <int LA, int LB, int LC, int LD, typename R, int E0>
-__device__ __forceinline__ void wide_rows(const KernelArgs& A, const R* tab, R* s_roots, bool keep, const PairD& pb,
+__device__ __forceinline__ void wide_rows(const KernelArgs& A, const R* tab, R* s_roots, bool has, const PairD& pb,
                                           const PairD& pk, int kpos, int npb, int npk, int wi, int gt, int lane,
                                           R* G) {
   using S = ClassShape<LA, LB, LC, LD>;
@@ -86,7 +88,7 @@ __device__ __forceinline__ void wide_rows(const KernelArgs& A, const R* tab, R* 
     const int bi = pb.prim_off + (ip < pb.nprim ? ip : 0);
     for (int kq = 0; kq < npk; ++kq) {
       const int kk = kq < pk.nprim ? kq : 0;
-      bool live = keep && ip < pb.nprim && kq < pk.nprim;
+      bool live = has && ip < pb.nprim && kq < pk.nprim;
       QuartetHdr<R> h;
       if constexpr (sizeof(R) == 4) {
         const PrimPairF bp = A.primsf[bi], kp = load_ket(A, pk.prim_off, kpos, kk, 0.f);
@@ -396,8 +398,8 @@ __global__ void __launch_bounds__(128, 2) wide_kernel(KernelArgs A) {
         int pbi, pki, kpos;
         cursor_seek(A.task, t < end ? t : b0, cur);
         cursor_decode(A.task, t < end ? t : b0, cur, pbi, pki, kpos);
-        const PairD pb = A.pairs[pbi];
-        const PairD pk = A.pairs[pki];
+        PairD pb = A.pairs[pbi];
+        PairD pk = A.pairs[pki];
         const Screen sc = screen_quartet(A, pb, pk);
         const bool keep = t < end && sc.keep;
         if (wi == 0) {
@@ -407,14 +409,32 @@ __global__ void __launch_bounds__(128, 2) wide_kernel(KernelArgs A) {
           if (keep) cnt.add(sc, pb, pk, A.fp32);
         }
         if (!__any_sync(0xffffffffu, keep)) continue;
-        const int npb = __reduce_max_sync(0xffffffffu, keep ? pb.nprim : 0);
-        const int npk = __reduce_max_sync(0xffffffffu, keep ? pk.nprim : 0);
+        // A pair can lose every primitive to the pair screen and still be
+        // listed (a threshold of zero or less keeps every bound): there is no
+        // primitive 0 to run along on, in the interleaved copies or in A.prims.
+        // Such lanes take the pairs of the first lane that has primitives.
+        const bool has = keep && pb.nprim > 0 && pk.nprim > 0;
+        const unsigned any = __ballot_sync(0xffffffffu, has);
+        const int src = any ? __ffs(any) - 1 : 0;
+        const int sb = __shfl_sync(0xffffffffu, pb.prim_off, src), nb = __shfl_sync(0xffffffffu, pb.nprim, src);
+        const int sk = __shfl_sync(0xffffffffu, pk.prim_off, src), nk = __shfl_sync(0xffffffffu, pk.nprim, src);
+        const int sp = __shfl_sync(0xffffffffu, kpos, src);
+        if (!has) {
+          pb.prim_off = sb;
+          pb.nprim = nb;
+          pk.prim_off = sk;
+          pk.nprim = nk;
+          kpos = sp;
+        }
+        // no lane with primitives: no passes, the tables are zero
+        const int npb = __reduce_max_sync(0xffffffffu, has ? pb.nprim : 0);
+        const int npk = __reduce_max_sync(0xffffffffu, has ? pk.nprim : 0);
         R* Gg = G + (size_t)g * S::NG * 32;
         static_for<W::PPW>([&](auto p) {
           static_for<WPG>([&](auto v) {
             constexpr int blk = decltype(p)::value * WPG + decltype(v)::value;
             if (wi == decltype(v)::value)
-              wide_rows<LA, LB, LC, LD, R, blk * W::ROWS>(A, tab, s_roots[gt], keep, pb, pk, kpos, npb, npk, wi, gt,
+              wide_rows<LA, LB, LC, LD, R, blk * W::ROWS>(A, tab, s_roots[gt], has, pb, pk, kpos, npb, npk, wi, gt,
                                                           lane, Gg);
           });
           // the next row block reuses the root buffers from the start

@@ -88,3 +88,47 @@ def test_wide_kernels_in_fp32(system):
         dc.set_mixed_cutoff(cutoff)
     assert WIDE32 <= {(r["la"], r["lb"], r["lc"], r["ld"]) for r in prof if r["team"] == 1 and r["fp32"] and r["quartets"]}
     assert rel(J32, J) < 1e-5 and rel(K32, K) < 1e-5
+
+
+@pytest.fixture(scope="module")
+def spread_system():
+    """18 atoms in a 60-bohr cube: every wide class has enough quartets at
+    threshold zero, which keeps every bound, and near half of its pairs of
+    shells have no primitives left.  The device memory that the plan gets held
+    NaN before, so that a value read without having been written shows."""
+    import torch
+
+    x = torch.full((1 << 28,), float("nan"), dtype=torch.float64, device="cuda")
+    del x
+    torch.cuda.empty_cache()
+    s = S.jk_system(natom=18, side=60.0, ndens=1)
+    dc = ib.Basis(s["shells"]).direct_contractor()
+    return dc, torch.tensor(s["dens"], dtype=torch.float64, device="cuda")
+
+
+def test_wide_kernels_on_pairs_without_primitives(spread_system):
+    import torch
+
+    dc, D = spread_system
+    J, K = build(dc, D, 0.0)
+    ran = {(r["la"], r["lb"], r["lc"], r["ld"]) for r in dc.plan.profile() if r["team"] == 1}
+    J0, K0 = torch.zeros_like(D), torch.zeros_like(D)
+    dc.jk_device_static(D.data_ptr(), 1, J0.data_ptr(), K0.data_ptr(), 0.0)
+    torch.cuda.synchronize()
+    assert WIDE <= ran
+    assert bool(torch.isfinite(J0).all()) and bool(torch.isfinite(K0).all())
+    assert rel(J, J0) < 1e-12 and rel(K, K0) < 1e-12
+
+
+def test_wide_kernels_in_fp32_on_pairs_without_primitives(spread_system):
+    dc, D = spread_system
+    J, K = build(dc, D, 0.0)
+    cutoff, _ = dc.mixed_cutoffs()
+    dc.set_mixed_cutoff(1e3)
+    try:
+        J32, K32 = build(dc, D, 0.0, precision=1)
+        prof = dc.plan.profile()
+    finally:
+        dc.set_mixed_cutoff(cutoff)
+    assert WIDE32 <= {(r["la"], r["lb"], r["lc"], r["ld"]) for r in prof if r["team"] == 1 and r["fp32"] and r["quartets"]}
+    assert rel(J32, J) < 1e-5 and rel(K32, K) < 1e-5
