@@ -49,18 +49,18 @@ __host__ __device__ constexpr size_t wide_tab_doubles() {
   return (WideShape<LA, LB, LC, LD, R>::TAB + 7) / 8;
 }
 
-// Barrier of the WPG warps of group team gt.
+// Barrier of the WPG warps of group team gt: by number, since the warps reach it
+// from the different row blocks that they sum (wide_rows).  Every row block, the
+// empty ones too, passes the same barriers: one per primitive quartet of the
+// group, skipped by all warps or none.
 template <int WPG>
 __device__ __forceinline__ void wide_sync(int gt) {
   if constexpr (WPG == 1)
     __syncwarp();
-  else if constexpr (WPG == 4)
-    __syncthreads();
   else
     asm volatile("bar.sync %0, %1;" ::"r"(1 + gt), "r"(WPG * 32) : "memory");
 }
 
-// Rows [E0, E0 + ROWS) of the tables of the group's 32 quartets.
 // A lane whose quartet has no primitives, or none at all (!has), runs along on
 // another lane's pairs (the caller's choice) with weight zero.
 template <int LA, int LB, int LC, int LD, typename R, int E0>
