@@ -10,6 +10,7 @@
 // the kets accepted by Q_bra*Q_ket >= tau form a prefix of every bra's ket
 // list; the per-class task lists are cached per threshold.
 #include "plan_internal.hpp"
+#include "run_streams.hpp"
 
 namespace igpu {
 namespace host {
@@ -261,7 +262,8 @@ int ensure_side_streams(igpu_plan* P, size_t n) {
 }
 
 // The lane-interleaved ket copies (KET_VALS) of every main class that a
-// one-thread launch can have as its ket: shells up to d.
+// one-thread launch can have as its ket: shells up to d.  Without room for them
+// the kernels read the pair list, so a refused allocation is no error.
 static int ensure_kets(igpu_plan* P) {
   if (!P->ket_off.empty()) return IGPU_OK;
   const int npc = std::min<int>((int)P->class_pairs.size(), pair_class(2, 2) + 1);
@@ -275,8 +277,14 @@ static int ensure_kets(igpu_plan* P) {
     n += P->class_pairs[c].size() * (size_t)maxprim[c] * KET_VALS;
     nf += P->class_pairs[c].size() * (size_t)maxprim[c] * KET_VALS_F;
   }
-  CK(P->d_kets.ensure(n));
-  CK(P->d_ketsf.ensure(nf));
+  cudaError_t e = P->d_kets.ensure(n);
+  if (e == cudaSuccess) e = P->d_ketsf.ensure(nf);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    P->d_kets.release();
+    return IGPU_OK;
+  }
+  CK(e);
   for (int c = 0; c < npc; ++c)
     CK(launch_ket_copy(P->d_pairs.p, P->d_prims.p, P->d_class_lists.p + P->class_list_off[c],
                        (int)P->class_pairs[c].size(), maxprim[c], P->d_kets.p + off[c], P->d_ketsf.p + offf[c],
@@ -300,113 +308,139 @@ static int ensure_kets(igpu_plan* P) {
 // molecule run on 30 of 148 SMs for 19 ms), and a launch of a few rounds
 // leaves it idle over its last quartets.  Longer launches gain nothing from
 // company and stay on `s`, one after another (their records then hold their own
-// times).  Each stream has a scratch region of its own.  The launch-shape tuner
-// times all launches one after another.
+// times).  Each stream has a scratch region of its own; where the device has no
+// room for them, fewer streams run.  The launch-shape tuner times all launches
+// one after another.
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches) {
   const bool grad = A.mode == MODE_GRAD;
   auto entry = [grad](int pcb, int pck) { return grad ? grad_entry(pcb, pck) : kernel_entry(pcb, pck); };
   const size_t nl = ts.launches.size();
+  P->no_scratch = false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(s, &cap));
+  const bool capturing = cap == cudaStreamCaptureStatusActive;
   struct Planned {
-    size_t li, grid, stream;
+    size_t li, grid;
     size_t slot, acc;         // scratch doubles per unit, and before its J sums
     size_t units;             // teams (wide kernels: blocks) in the grid
     int split;                // lanes per quartet of a one-thread launch
     const KernelEntry* e;
     const WideEntry* wide;    // its one-thread-per-quartet kernel runs instead
-    double load;
-    bool full;    // enough rounds to fill the device by itself
-    double fill;  // share of the resident blocks that its grid takes
+    double fill;              // share of the resident blocks that its grid takes
   };
   std::vector<Planned> run;
-  for (size_t li = 0; li < nl; ++li) {
-    Launch* L = ts.launches[li].get();
-    if (L->total == 0) continue;
-    const KernelEntry* e = entry(L->pcb, L->pck);
-    if (!e) return fail(IGPU_ERR_UNSUPPORTED, "angular class not compiled for the GPU");
-    if (A.mode == MODE_JK && L->fp32 && !A.jk.Df)
-      return fail(IGPU_ERR_INVALID_ARGUMENT, "FP32 J/K launch without the FP32 densities");
-    int bps_cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
-    if (P->tune_bps) {
-      bps_cap = P->tune_bps > 0 ? P->tune_bps : 0;
-    } else if (A.mode == MODE_JK || grad) {
-      auto t = P->tuned_bps.find(tune_key(L->pcb, L->pck, L->fp32, grad));
-      if (t != P->tuned_bps.end()) bps_cap = t->second;
+  std::vector<StreamItem> items;  // the same launches
+  auto plan = [&](bool wide) -> int {
+    run.clear();
+    items.clear();
+    for (size_t li = 0; li < nl; ++li) {
+      Launch* L = ts.launches[li].get();
+      if (L->total == 0) continue;
+      const KernelEntry* e = entry(L->pcb, L->pck);
+      if (!e) return fail(IGPU_ERR_UNSUPPORTED, "angular class not compiled for the GPU");
+      if (A.mode == MODE_JK && L->fp32 && !A.jk.Df)
+        return fail(IGPU_ERR_INVALID_ARGUMENT, "FP32 J/K launch without the FP32 densities");
+      int bps_cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
+      if (P->tune_bps) {
+        bps_cap = P->tune_bps > 0 ? P->tune_bps : 0;
+      } else if (A.mode == MODE_JK || grad) {
+        auto t = P->tuned_bps.find(tune_key(L->pcb, L->pck, L->fp32, grad));
+        if (t != P->tuned_bps.end()) bps_cap = t->second;
+      }
+      Planned r{};
+      r.li = li;
+      r.e = e;
+      r.split = 1;
+      if (wide && A.mode == MODE_JK && A.jk.symmetric && A.kinds == 0 && L->total >= wide_min_tasks())
+        r.wide = wide_entry(L->pcb, L->pck, L->fp32);
+      const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
+      if (r.wide) {
+        const int bps = blocks_per_sm(r.wide, L->fp32);
+        r.grid = grid_blocks(L->total, 128, bps, bps_cap);
+        r.fill = (double)r.grid / ((double)bps * sm_count());
+        r.units = r.grid;
+        r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
+        r.slot = r.acc + 128 * sums;
+      } else {
+        // a quartet of a small one-thread launch takes several lanes, as far as
+        // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
+        if (e->team == 1 && !grad)
+          while (r.split < 16 && r.split < L->prim_pairs &&
+                 L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
+            r.split *= 2;
+        r.grid = grid_for(e, L->fp32, L->total * r.split, bps_cap);
+        r.fill = (double)r.grid / ((double)blocks_per_sm(e, L->fp32) * sm_count());
+        r.units = r.grid * (128 / e->team);
+        // one-thread classes finish symmetric J/K of one shell kind in registers
+        r.acc = e->team == 1 && A.mode == MODE_JK && A.jk.symmetric && A.kinds != 2 ? 0 : e->slot;
+        r.slot = r.acc + sums;
+      }
+      // rounds of quartets over the resident teams times one quartet's work on
+      // a team's lanes
+      const int la = pc_la_host(L->pcb), lb = L->pcb - la * (la + 1) / 2;
+      const int lc = pc_la_host(L->pck), ld = L->pck - lc * (lc + 1) / 2;
+      const double teams = r.wide ? (double)r.grid * 128 : (double)r.units / r.split;
+      const double np = (double)L->prim_pairs * L->prim_pairs;
+      const double load = std::ceil((double)L->total / teams) * np *
+                          (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) /
+                          (r.wide ? 1 : e->team * r.split);
+      run.push_back(r);
+      items.push_back({load, (double)L->total >= kFullRounds * teams, r.units * r.slot, 0});
     }
-    Planned r{};
-    r.li = li;
-    r.e = e;
-    r.split = 1;
-    if (A.mode == MODE_JK && A.jk.symmetric && A.kinds == 0 && L->total >= wide_min_tasks())
-      r.wide = wide_entry(L->pcb, L->pck, L->fp32);
-    const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
-    if (r.wide) {
-      const int bps = blocks_per_sm(r.wide, L->fp32);
-      r.grid = grid_blocks(L->total, 128, bps, bps_cap);
-      r.fill = (double)r.grid / ((double)bps * sm_count());
-      r.units = r.grid;
-      r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
-      r.slot = r.acc + 128 * sums;
-    } else {
-      // a quartet of a small one-thread launch takes several lanes, as far as
-      // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
-      if (e->team == 1 && !grad)
-        while (r.split < 16 && r.split < L->prim_pairs &&
-               L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
-          r.split *= 2;
-      r.grid = grid_for(e, L->fp32, L->total * r.split, bps_cap);
-      r.fill = (double)r.grid / ((double)blocks_per_sm(e, L->fp32) * sm_count());
-      r.units = r.grid * (128 / e->team);
-      // one-thread classes finish symmetric J/K of one shell kind in registers
-      r.acc = e->team == 1 && A.mode == MODE_JK && A.jk.symmetric && A.kinds != 2 ? 0 : e->slot;
-      r.slot = r.acc + sums;
+    return IGPU_OK;
+  };
+  // without room for the scratch of a single stream, the wide kernels, whose
+  // running sums are per lane, give way to the teams
+  std::vector<size_t> order, region;  // launches as they are started; scratch doubles per stream
+  size_t ns = 0;
+  cudaError_t scratch_err = cudaErrorStreamCaptureUnsupported;
+  auto have = [&](size_t total, bool several) {
+    if (total <= P->d_scratch.n) return true;
+    if (capturing) return false;
+    size_t free = 0, all = 0;
+    if (several && cudaMemGetInfo(&free, &all) == cudaSuccess &&
+        total > (free / sizeof(double) + P->d_scratch.n) / kScratchShare)
+      return false;
+    scratch_err = P->d_scratch.ensure(total);
+    if (scratch_err != cudaSuccess) cudaGetLastError();
+    return scratch_err == cudaSuccess;
+  };
+  for (bool wide = true; ns == 0; wide = false) {
+    int rc = plan(wide);
+    if (rc) return rc;
+    // longest first
+    order.resize(run.size());
+    std::iota(order.begin(), order.end(), (size_t)0);
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
+      return items[x].full != items[y].full ? items[x].full : items[x].load > items[y].load;
+    });
+    // as many streams as it takes to fill the device about twice over
+    double busy = 0.0, work = 0.0;
+    for (size_t x = 0; x < run.size(); ++x)
+      if (!items[x].full) {
+        busy += items[x].load * std::min(1.0, run[x].fill);
+        work += items[x].load;
+      }
+    const size_t want = work > 0.0 ? (size_t)std::min((double)kRunStreams, std::ceil(2.0 * work / busy)) : 1;
+    size_t most = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(want, run.size()));
+    // no stream is made and nothing is allocated under capture
+    if (capturing) most = std::min(most, P->side.size() + 1);
+    ns = assign_streams(items, order, most, have, region);
+    if (ns == 0 && std::none_of(run.begin(), run.end(), [](const Planned& r) { return r.wide != nullptr; })) {
+      P->no_scratch = true;
+      return cuda_fail(scratch_err, "scratch");
     }
-    // rounds of quartets over the resident teams times one quartet's work on
-    // a team's lanes
-    const int la = pc_la_host(L->pcb), lb = L->pcb - la * (la + 1) / 2;
-    const int lc = pc_la_host(L->pck), ld = L->pck - lc * (lc + 1) / 2;
-    const double teams = r.wide ? (double)r.grid * 128 : (double)r.units / r.split;
-    const double np = (double)L->prim_pairs * L->prim_pairs;
-    r.full = (double)L->total >= kFullRounds * teams;
-    r.load = std::ceil((double)L->total / teams) * np *
-             (grad ? model_flops_grad_prim(la, lb, lc, ld) : model_flops_prim(la, lb, lc, ld)) / (r.wide ? 1 : e->team * r.split);
-    if (!grad && (r.wide || e->team == 1) && L->ket_class >= 0) {
-      const int rc = ensure_kets(P);
-      if (rc) return rc;
-    }
-    run.push_back(r);
-  }
-  // longest first; fewer streams while the scratch regions exceed the budget
-  std::vector<size_t> order(run.size());
-  std::iota(order.begin(), order.end(), (size_t)0);
-  std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) {
-    return run[x].full != run[y].full ? run[x].full : run[x].load > run[y].load;
-  });
-  auto doubles = [](const Planned& r) { return r.units * r.slot; };
-  // as many streams as it takes to fill the device about twice over
-  double busy = 0.0, work = 0.0;
-  for (const Planned& r : run)
-    if (!r.full) {
-      busy += r.load * std::min(1.0, r.fill);
-      work += r.load;
-    }
-  const size_t want = work > 0.0 ? (size_t)std::min((double)kRunStreams, std::ceil(2.0 * work / busy)) : 1;
-  size_t ns = P->tune_mult || P->tune_bps ? 1 : std::max<size_t>(1, std::min(want, run.size()));
-  std::vector<size_t> region;  // scratch doubles per stream
-  for (;; ns = (ns + 1) / 2) {
-    std::vector<double> load(ns, 0.0);
-    region.assign(ns, 0);
-    for (size_t x : order) {
-      Planned& r = run[x];
-      r.stream = r.full ? 0 : (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
-      load[r.stream] += r.load;
-      region[r.stream] = std::max(region[r.stream], doubles(r));
-    }
-    if (ns == 1 || std::accumulate(region.begin(), region.end(), (size_t)0) <= kScratchBudget) break;
   }
   if (ns == 1) std::iota(order.begin(), order.end(), (size_t)0);
-  CK(P->d_scratch.ensure(std::accumulate(region.begin(), region.end(), (size_t)0)));
   std::vector<double*> base(ns, P->d_scratch.p);
   for (size_t k = 1; k < ns; ++k) base[k] = base[k - 1] + region[k - 1];
+  // the interleaved kets in what room is left
+  if (!grad && !capturing && std::any_of(run.begin(), run.end(), [&](const Planned& r) {
+        return (r.wide || r.e->team == 1) && ts.launches[r.li]->ket_class >= 0;
+      })) {
+    const int rc = ensure_kets(P);
+    if (rc) return rc;
+  }
   if (ns > 1) {
     const int rc = ensure_side_streams(P, ns - 1);
     if (rc) return rc;
@@ -423,9 +457,6 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   }
   lg.profile.assign(run.size(), igpu_launch_record{});
   lg.profile_launch.resize(run.size());
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(s, &cap));
-  const bool capturing = cap == cudaStreamCaptureStatusActive;
   // under stream capture the records are external nodes, so that the graph
   // records them on every replay (the flag is only valid there)
   auto record = [capturing](cudaEvent_t ev, cudaStream_t st) {
@@ -454,8 +485,9 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     Launch* L = ts.launches[pl.li].get();
     const KernelEntry* e = pl.e;
     const size_t li = pl.li, grid = pl.grid;
-    const cudaStream_t st = stream_of(pl.stream);
-    A.scratch = base[pl.stream];
+    const size_t k = items[x].stream;
+    const cudaStream_t st = stream_of(k);
+    A.scratch = base[k];
     A.slot_doubles = pl.slot;
     A.acc_offset = pl.acc;
     A.work_counter = lg.work.p + li;

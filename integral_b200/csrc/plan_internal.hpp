@@ -63,17 +63,18 @@ template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
+  ~DevBuf() { release(); }
   cudaError_t ensure(size_t count) {
     if (count <= n && p) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
+    release();
     cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
     if (e == cudaSuccess) n = std::max<size_t>(count, 1);
     return e;
+  }
+  void release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    n = 0;
   }
   cudaError_t upload(const std::vector<T>& v, cudaStream_t s) {
     cudaError_t e = ensure(v.size());
@@ -117,11 +118,6 @@ struct LaunchLog {
 // Streams that a run's class launches are spread over, the caller's among
 // them (device connections by default: more would share one queue).
 constexpr size_t kRunStreams = 8;
-// Scratch doubles (4 GiB) above which a run uses fewer streams, each of which
-// needs a scratch region of its own.  256 MiB (or twice the largest launch's)
-// left a 5-atom g molecule two streams and cost it 52 against 35 ms, an f
-// gradient 39 against 28 ms; allocating the 4 GiB adds 3 ms to a first run.
-constexpr size_t kScratchBudget = (size_t)1 << 29;
 // Lanes per SM up to which a one-thread launch of few quartets is widened, by
 // lanes that share a quartet (KernelArgs::split).
 constexpr unsigned long long kSplitLanes = 256;
@@ -202,6 +198,7 @@ struct igpu_plan {
   DevBuf<float> d_ketsf;
   std::vector<size_t> ket_off, ketf_off;
   DevBuf<double> d_scratch;
+  bool no_scratch = false;  // the last run_tasks found no room for its scratch and launched nothing
   DevBuf<Counters> d_counters;
   DevBuf<double> d_schwarz_pair;
   // per-call device buffers
