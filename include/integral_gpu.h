@@ -107,8 +107,9 @@ typedef struct {
   uint64_t tasks;             /* quartets in the launch's task list */
   uint64_t quartets;          /* of them accepted by the screening */
   uint64_t prim_quartets;
-  double ms;                  /* device time (CUDA events); launches of one call overlap, so
-                               * this includes waiting for the others (not while autotuning) */
+  double ms;                  /* its part of the call's device time (CUDA events): launches of one
+                               * call overlap, and every moment is divided among those in flight
+                               * by the share of the device that each one's grid takes */
   double model_flops;         /* fixed Rys flop model of the accepted work */
   uint32_t chunk;             /* tasks a warp claims per grab */
   uint32_t reserved;

@@ -11,6 +11,7 @@
 // list; the per-class task lists are cached per threshold.
 #include "plan_internal.hpp"
 #include "run_streams.hpp"
+#include "run_times.hpp"
 
 namespace igpu {
 namespace host {
@@ -184,10 +185,12 @@ int tune_key(int pcb, int pck, bool fp32, bool grad) {
 // (a chunk multiplier, or a blocks-per-SM cap), then keep per class the
 // candidate of the shortest time.
 void tune_record(igpu_plan* P, int m, bool grad, std::map<int, std::map<int, float>>& best) {
-  for (const igpu_launch_record& r : P->log.profile) {
+  const std::vector<double> ms = launch_times(P->log);
+  for (size_t k = 0; k < ms.size(); ++k) {
+    const igpu_launch_record& r = P->log.profile[k];
     auto& slot = best[tune_key(pair_class(r.la, r.lb), pair_class(r.lc, r.ld), r.fp32 != 0, grad)];
     auto it = slot.find(m);
-    if (it == slot.end() || r.ms < it->second) slot[m] = r.ms;
+    if (it == slot.end() || ms[k] < it->second) slot[m] = (float)ms[k];
   }
 }
 void tune_keep(igpu_plan* P, const std::map<int, std::map<int, float>>& best, bool bps) {
@@ -303,14 +306,12 @@ static int ensure_kets(igpu_plan* P) {
 // than kFullRounds quartets per resident team are spread over up to
 // kRunStreams streams (fewer where their grids fill the device anyway), longest
 // first, each onto the stream with the least estimated load; `s` waits for all
-// of them.  A class of a small molecule
-// fills a fraction of the device (the 120 (gg|gg) quartets of a 5-atom
-// molecule run on 30 of 148 SMs for 19 ms), and a launch of a few rounds
-// leaves it idle over its last quartets.  Longer launches gain nothing from
-// company and stay on `s`, one after another (their records then hold their own
-// times).  Each stream has a scratch region of its own; where the device has no
-// room for them, fewer streams run.  The launch-shape tuner times all launches
-// one after another.
+// of them.  A class of a small molecule fills a fraction of the device (the 120
+// (gg|gg) quartets of a 5-atom molecule run on 30 of 148 SMs for 10.5 ms), and a
+// launch of a few rounds leaves it idle over its last quartets.  Longer launches
+// gain nothing from company and stay on `s`, one after another.  Each stream has
+// a scratch region of its own; where the device has no room for them, fewer
+// streams run.  The launch-shape tuner times all launches one after another.
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches) {
   const bool grad = A.mode == MODE_GRAD;
   auto entry = [grad](int pcb, int pck) { return grad ? grad_entry(pcb, pck) : kernel_entry(pcb, pck); };
@@ -457,6 +458,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   }
   lg.profile.assign(run.size(), igpu_launch_record{});
   lg.profile_launch.resize(run.size());
+  lg.fill.resize(run.size());
   // under stream capture the records are external nodes, so that the graph
   // records them on every replay (the flag is only valid there)
   auto record = [capturing](cudaEvent_t ev, cudaStream_t st) {
@@ -542,6 +544,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     r.tasks = L->total;
     r.chunk = (uint32_t)A.chunk;
     lg.profile_launch[x] = li;
+    lg.fill[x] = pl.fill;
   }
   for (size_t k = 1; k < ns; ++k) {
     CK(cudaEventRecord(P->side_ev[k - 1], stream_of(k)));
@@ -553,7 +556,28 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   return IGPU_OK;
 }
 
-// After the stream is synchronised: per-launch times, counters, model flops.
+// Milliseconds between two events; 0 without usable records of them (and no
+// error left behind).
+static double event_ms(cudaEvent_t a, cudaEvent_t b) {
+  float ms = 0.f;
+  if (cudaEventElapsedTime(&ms, a, b) == cudaSuccess) return ms;
+  cudaGetLastError();
+  return 0.0;
+}
+
+// Device time of every launch of a finished run (igpu_launch_record::ms), from
+// its events when somebody asks for it.
+std::vector<double> launch_times(const LaunchLog& lg) {
+  std::vector<LaunchSpan> l;
+  for (size_t k = 0; k < lg.profile.size(); ++k) {
+    const cudaEvent_t e0 = lg.events[2 * lg.profile_launch[k]], e1 = lg.events[2 * lg.profile_launch[k] + 1];
+    const double begin = event_ms(lg.events[lg.span_event], e0);
+    l.push_back({begin, begin + event_ms(e0, e1), lg.fill[k]});
+  }
+  return share_time(l);
+}
+
+// After the stream is synchronised: the run's time, counters, model flops.
 int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c, int grad_terms_x) {
   LaunchLog& lg = *P->cur_log;
   size_t nl = 0;
@@ -564,12 +588,6 @@ int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c, int grad
   for (size_t k = 0; k < lg.profile.size(); ++k) {
     igpu_launch_record& r = lg.profile[k];
     const size_t li = lg.profile_launch[k];
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, lg.events[2 * li], lg.events[2 * li + 1]) != cudaSuccess) {
-      cudaGetLastError();  // a launch without a usable record: no time, no sticky error
-      ms = 0.f;
-    }
-    r.ms = ms;
     r.quartets = c[li].quartets;
     r.prim_quartets = c[li].prim_quartets;
     if (grad_terms_c >= 0)
@@ -586,13 +604,8 @@ int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c, int grad
     P->last.model_flops += r.model_flops;
   }
   // the launches overlap: the run's device time is its span
-  float span = 0.f;
-  if (!lg.profile.empty() &&
-      cudaEventElapsedTime(&span, lg.events[lg.span_event], lg.events[lg.span_event + 1]) != cudaSuccess) {
-    cudaGetLastError();
-    span = 0.f;
-  }
-  P->last.kernel_ms = span;
+  P->last.kernel_ms =
+      lg.profile.empty() ? 0.0 : event_ms(lg.events[lg.span_event], lg.events[lg.span_event + 1]);
   P->last.launches = (uint32_t)lg.profile.size();
   return IGPU_OK;
 }
@@ -1279,7 +1292,12 @@ int igpu_last_stats(const igpu_plan* P, igpu_stats* st) {
 int igpu_last_profile(const igpu_plan* P, igpu_launch_record* out, size_t cap, size_t* n) {
   if (!P || !n) return fail(IGPU_ERR_INVALID_ARGUMENT, "NULL argument");
   *n = P->log.profile.size();
-  for (size_t k = 0; k < P->log.profile.size() && k < cap && out; ++k) out[k] = P->log.profile[k];
+  if (!out || cap == 0) return IGPU_OK;
+  const std::vector<double> ms = launch_times(P->log);
+  for (size_t k = 0; k < P->log.profile.size() && k < cap; ++k) {
+    out[k] = P->log.profile[k];
+    out[k].ms = ms[k];
+  }
   return IGPU_OK;
 }
 

@@ -110,6 +110,7 @@ struct LaunchLog {
   size_t span_event = 0;  // first of the run's two events
   std::vector<igpu_launch_record> profile;
   std::vector<size_t> profile_launch;
+  std::vector<double> fill;  // share of the resident blocks that each grid takes
   ~LaunchLog() {
     for (cudaEvent_t ev : events) cudaEventDestroy(ev);
   }
@@ -270,6 +271,7 @@ int tune_two_stage(igpu_plan* P, bool grad, const std::function<int()>& run);
 size_t slot_with_acc(const KernelEntry* e, int pcb, const KernelArgs& A);
 int ensure_side_streams(igpu_plan* P, size_t n);
 int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t& launches);
+std::vector<double> launch_times(const LaunchLog& lg);
 int collect_profile(igpu_plan* P, int ndens, bool jk, int grad_terms_c = -1, int grad_terms_x = 0);
 std::unique_ptr<Launch> make_launch(igpu_plan* P, int pcb, int pck, bool fp32, const std::vector<int>& bras,
                                     const std::vector<int>& nket, const std::vector<int>& kstart,

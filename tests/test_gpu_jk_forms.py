@@ -78,3 +78,22 @@ def test_shared_quartets_of_small_launches(natom, nprim):
     assert rel(J, Jo) < 1e-12 and rel(K, Ko) < 1e-12
     gpu, ref = ib.Basis(shells).eri(), O.OracleBasis(shells).eri()
     assert float(np.max(np.abs(gpu - ref))) < 1e-13 * max(1.0, float(np.max(np.abs(ref))))
+
+
+@pytest.mark.parametrize("natom", [3, 8])
+def test_launch_records_add_up(natom):
+    """The class launches of a small molecule overlap; their records divide the
+    run's device time (moments without a launch in flight, and the events'
+    resolution of 0.5 us a launch, aside)."""
+    import torch
+
+    s = S.jk_system(natom=natom, side=5.0 * natom ** (1 / 3), ndens=1)
+    dc = ib.Basis(s["shells"]).direct_contractor()
+    D = torch.tensor(s["dens"], device="cuda")
+    J, K = torch.zeros_like(D), torch.zeros_like(D)
+    for _ in range(3):
+        dc.jk_device(D.data_ptr(), 1, J.data_ptr(), K.data_ptr(), s["threshold"])
+    span, prof = dc.last_stats()["kernel_ms"], dc.plan.profile()
+    total = sum(r["ms"] for r in prof)
+    assert len(prof) > 10 and all(r["ms"] >= 0.0 for r in prof)
+    assert 0.5 * span <= total <= span + 1e-3 * len(prof), (total, span)
