@@ -43,24 +43,33 @@ def test_general_densities(spherical, ndens, want_k):
 
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 def test_general_density_without_finite_parts(value):
-    """One element that the symmetric and antisymmetric parts cannot hold: the
-    elements of J and K that the general sums leave finite stay so."""
+    """One element that the symmetric and antisymmetric parts cannot hold, between
+    two atoms 80 bohr apart: the general sums keep it out of J and out of three
+    quarters of K, the parts would bring it into half of K."""
     import torch
 
-    dc = ib.Basis(S.jk_system(natom=2, side=3.0, ndens=1)["shells"]).direct_contractor()
+    rng = np.random.default_rng(5)
+    shells = S.build_shells(rng, np.array([[0.0, 0.0, 0.0], [0.0, 0.0, 80.0]]), "sssppd", 3, 0.1, 2.5, 0.2, 1.0)
+    dc = ib.Basis(shells).direct_contractor()
     n = dc.nao()
-    D = np.random.default_rng(5).normal(size=(1, n, n))
-    D[0, 1, 4] = value
+    D = rng.normal(size=(1, n, n))
+    D[0, 1, n // 2 + 4] = value
+    ob = O.OracleBasis(shells)
+    Jo, Ko, _, _ = ob.direct_jk(D, 1e-13)
+    Dt = D.transpose(0, 2, 1)
+    with np.errstate(invalid="ignore"):
+        Kp = sum(ob.direct_jk(0.5 * p, 1e-13)[1] for p in (D + Dt, D - Dt))
+    assert np.isfinite(Jo).all() and np.isfinite(Ko).sum() == 3 * n * n // 4
+    assert np.isfinite(Kp).sum() == n * n // 2
     D = torch.tensor(D, device="cuda")
     J, K, J0, K0 = (torch.zeros_like(D) for _ in range(4))
     dc.jk_device(D.data_ptr(), 1, J.data_ptr(), K.data_ptr(), 1e-13)
     dc.jk_device_static(D.data_ptr(), 1, J0.data_ptr(), K0.data_ptr(), 1e-13)
     torch.cuda.synchronize()
-    for a, b in ((J, J0), (K, K0)):
-        ok = torch.isfinite(b)
-        assert torch.equal(torch.isfinite(a), ok)
-        if bool(ok.any()):
-            assert rel(a[ok], b[ok]) < 1e-12
+    for a, b in ((J, Jo), (J0, Jo), (K, Ko), (K0, Ko)):
+        a, ok = a.cpu().numpy(), np.isfinite(b)
+        assert np.array_equal(np.isfinite(a), ok)
+        assert rel(a[ok], b[ok]) < 1e-12
 
 
 @pytest.mark.parametrize("natom", [1, 2, 4])
