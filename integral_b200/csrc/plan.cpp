@@ -175,20 +175,23 @@ double mixed_split(double cutoff, double dmax) {
   return cut > 0.0 ? cut : std::numeric_limits<double>::min();
 }
 
-// Key of a launch class in the tuned-chunk table; gradient classes have
-// their own keys.
-int tune_key(int pcb, int pck, bool fp32, bool grad) {
-  return ((pcb * 64 + pck) * 2 + (fp32 ? 1 : 0)) | (grad ? (1 << 20) : 0);
+// Key of a launch class in the tables of tuned shapes.  Gradient classes have
+// their own, and so has every form of a class's launch: what is best for one
+// says nothing about another.
+int tune_key(int pcb, int pck, bool fp32, bool grad, LaunchForm form) {
+  return ((pcb * 64 + pck) * 2 + (fp32 ? 1 : 0)) | (grad ? (1 << 20) : 0) | ((int)form << 21);
 }
 
 // Tuning: note every launch time of the last call made with candidate m
 // (a chunk multiplier, or a blocks-per-SM cap), then keep per class the
-// candidate of the shortest time.
-void tune_record(igpu_plan* P, int m, bool grad, std::map<int, std::map<int, float>>& best) {
+// candidate of the shortest time.  Wide launches take no multiplier.
+void tune_record(igpu_plan* P, int m, bool grad, bool bps, std::map<int, std::map<int, float>>& best) {
   const std::vector<double> ms = launch_times(P->log);
   for (size_t k = 0; k < ms.size(); ++k) {
     const igpu_launch_record& r = P->log.profile[k];
-    auto& slot = best[tune_key(pair_class(r.la, r.lb), pair_class(r.lc, r.ld), r.fp32 != 0, grad)];
+    const LaunchForm form = P->log.form[k];
+    if (form == LaunchForm::wide && !bps) continue;
+    auto& slot = best[tune_key(pair_class(r.la, r.lb), pair_class(r.lc, r.ld), r.fp32 != 0, grad, form)];
     auto it = slot.find(m);
     if (it == slot.end() || ms[k] < it->second) slot[m] = (float)ms[k];
   }
@@ -222,7 +225,7 @@ int tune_two_stage(igpu_plan* P, bool grad, const std::function<int()>& run) {
       const int rc = run();
       P->tune_mult = 0;
       if (rc) return rc;
-      tune_record(P, m, grad, best);
+      tune_record(P, m, grad, false, best);
     }
   tune_keep(P, best, false);
   // cap 0 is the occupancy limit itself
@@ -234,7 +237,7 @@ int tune_two_stage(igpu_plan* P, bool grad, const std::function<int()>& run) {
       const int rc = run();
       P->tune_bps = 0;
       if (rc) return rc;
-      tune_record(P, c, grad, best_bps);
+      tune_record(P, c, grad, true, best_bps);
     }
   tune_keep(P, best_bps, true);
   return IGPU_OK;
@@ -328,6 +331,8 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     const KernelEntry* e;
     const WideEntry* wide;    // its one-thread-per-quartet kernel runs instead
     double fill;              // share of the resident blocks that its grid takes
+    int key;                  // of its tuned shapes
+    LaunchForm form() const { return wide ? LaunchForm::wide : (split > 1 ? LaunchForm::split : LaunchForm::plain); }
   };
   std::vector<Planned> run;
   std::vector<StreamItem> items;  // the same launches
@@ -341,19 +346,26 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
       if (!e) return fail(IGPU_ERR_UNSUPPORTED, "angular class not compiled for the GPU");
       if (A.mode == MODE_JK && L->fp32 && !A.jk.Df)
         return fail(IGPU_ERR_INVALID_ARGUMENT, "FP32 J/K launch without the FP32 densities");
-      int bps_cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
-      if (P->tune_bps) {
-        bps_cap = P->tune_bps > 0 ? P->tune_bps : 0;
-      } else if (A.mode == MODE_JK || grad) {
-        auto t = P->tuned_bps.find(tune_key(L->pcb, L->pck, L->fp32, grad));
-        if (t != P->tuned_bps.end()) bps_cap = t->second;
-      }
       Planned r{};
       r.li = li;
       r.e = e;
       r.split = 1;
       if (wide && A.mode == MODE_JK && A.jk.symmetric && A.kinds == 0 && L->total >= wide_min_tasks())
         r.wide = wide_entry(L->pcb, L->pck, L->fp32);
+      // a quartet of a small one-thread launch takes several lanes, as far as
+      // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
+      if (!r.wide && e->team == 1 && !grad)
+        while (r.split < 16 && r.split < L->prim_pairs &&
+               L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
+          r.split *= 2;
+      r.key = tune_key(L->pcb, L->pck, L->fp32, grad, r.form());
+      int bps_cap = 0;  // blocks-per-SM cap of the grid (0: the occupancy limit)
+      if (P->tune_bps) {
+        bps_cap = P->tune_bps > 0 ? P->tune_bps : 0;
+      } else if (A.mode == MODE_JK || grad) {
+        auto t = P->tuned_bps.find(r.key);
+        if (t != P->tuned_bps.end()) bps_cap = t->second;
+      }
       const size_t sums = slot_with_acc(e, L->pcb, A) - e->slot;  // running J sums per team
       if (r.wide) {
         const int bps = blocks_per_sm(r.wide, L->fp32);
@@ -363,12 +375,6 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
         r.acc = L->fp32 ? r.wide->tab32 : r.wide->tab64;
         r.slot = r.acc + 128 * sums;
       } else {
-        // a quartet of a small one-thread launch takes several lanes, as far as
-        // they find room: 81 primitive quartets of (11|11) are 165 us on one lane
-        if (e->team == 1 && !grad)
-          while (r.split < 16 && r.split < L->prim_pairs &&
-                 L->total * 2 * r.split <= kSplitLanes * (unsigned long long)sm_count())
-            r.split *= 2;
         r.grid = grid_for(e, L->fp32, L->total * r.split, bps_cap);
         r.fill = (double)r.grid / ((double)blocks_per_sm(e, L->fp32) * sm_count());
         r.units = r.grid * (128 / e->team);
@@ -459,6 +465,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
   lg.profile.assign(run.size(), igpu_launch_record{});
   lg.profile_launch.resize(run.size());
   lg.fill.resize(run.size());
+  lg.form.resize(run.size());
   // under stream capture the records are external nodes, so that the graph
   // records them on every replay (the flag is only valid there)
   auto record = [capturing](cudaEvent_t ev, cudaStream_t st) {
@@ -505,7 +512,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     if (P->tune_mult) {
       mult = P->tune_mult;
     } else if (A.mode == MODE_JK || grad) {
-      auto t = P->tuned_mult.find(tune_key(L->pcb, L->pck, L->fp32, grad));
+      auto t = P->tuned_mult.find(pl.key);
       if (t != P->tuned_mult.end()) mult = t->second;
     }
     A.chunk = per_warp * mult;
@@ -545,6 +552,7 @@ int run_tasks(igpu_plan* P, TaskSet& ts, KernelArgs A, cudaStream_t s, uint32_t&
     r.chunk = (uint32_t)A.chunk;
     lg.profile_launch[x] = li;
     lg.fill[x] = pl.fill;
+    lg.form[x] = pl.form();
   }
   for (size_t k = 1; k < ns; ++k) {
     CK(cudaEventRecord(P->side_ev[k - 1], stream_of(k)));

@@ -97,6 +97,10 @@ struct Launch {
   int ket_class = -1;             // the main class whose list that is (-1: another list)
 };
 
+// How a class launch runs: a quartet on one thread or one team, on several
+// lanes that share its primitives, or in the wide kernels.
+enum class LaunchForm { plain = 0, split = 1, wide = 2 };
+
 struct TaskSet {
   std::vector<std::unique_ptr<Launch>> launches;
 };
@@ -111,6 +115,7 @@ struct LaunchLog {
   std::vector<igpu_launch_record> profile;
   std::vector<size_t> profile_launch;
   std::vector<double> fill;  // share of the resident blocks that each grid takes
+  std::vector<LaunchForm> form;
   ~LaunchLog() {
     for (cudaEvent_t ev : events) cudaEventDestroy(ev);
   }
@@ -264,8 +269,8 @@ double model_flops_grad_quartet(int la, int lb, int lc, int ld, bool sph, int nt
 double mixed_split(double cutoff, double dmax);
 double fp32_class_scale(int lmax);
 int class_lmax(int pca, int pcb);
-int tune_key(int pcb, int pck, bool fp32, bool grad);
-void tune_record(igpu_plan* P, int m, bool grad, std::map<int, std::map<int, float>>& best);
+int tune_key(int pcb, int pck, bool fp32, bool grad, LaunchForm form);
+void tune_record(igpu_plan* P, int m, bool grad, bool bps, std::map<int, std::map<int, float>>& best);
 void tune_keep(igpu_plan* P, const std::map<int, std::map<int, float>>& best, bool bps);
 int tune_two_stage(igpu_plan* P, bool grad, const std::function<int()>& run);
 size_t slot_with_acc(const KernelEntry* e, int pcb, const KernelArgs& A);

@@ -46,3 +46,28 @@ def test_gradient_autotune_keeps_results():
     for r in gc._plan.profile():
         assert r["chunk"] // (32 // r["team"]) in (4, 8, 16, 32, 64)
     assert float(np.max(np.abs(g0 - g1))) < 1e-12 * float(np.max(np.abs(g0)))
+
+
+def test_shapes_tuned_for_wide_kernels_stay_with_them():
+    """A class's wide launch and its team launch are tuned apart: a general
+    density, which the wide kernels do not take, keeps the untuned shapes of the
+    classes that ran wide under the tuner."""
+    import torch
+    s = S.jk_system(natom=18, side=13.1, ndens=1)
+    dc = ib.Basis(s["shells"]).direct_contractor()
+    D = torch.from_numpy(s["dens"]).cuda()
+    G = D.clone()
+    G[0, 0, 1] *= 1.0 + 1e-6
+    J, K = torch.zeros_like(D), torch.zeros_like(D)
+
+    def shapes(M):
+        dc.jk_device(M.data_ptr(), 1, J.data_ptr(), K.data_ptr(), s["threshold"], True, 1)
+        return {(r["la"], r["lb"], r["lc"], r["ld"], r["fp32"]): (r["team"], r["grid"], r["chunk"])
+                for r in dc.plan.profile()}
+
+    sym, before = shapes(D), shapes(G)
+    wide = [c for c, r in sym.items() if r[0] == 1 and before[c][0] > 1]
+    assert len(wide) >= 6
+    dc.autotune_device(D.data_ptr(), 1, s["threshold"], 1)
+    after = shapes(G)
+    assert {c: after[c] for c in wide} == {c: before[c] for c in wide}
