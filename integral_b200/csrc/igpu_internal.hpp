@@ -123,8 +123,17 @@ IGPU_HD constexpr bool rys_tabulated(int n, R T) {
 template <typename R>
 IGPU_HD inline int rys_interval(int n, R T, R& xi) {
   const R u = T * R(rys_div<R>(n));
+#ifdef __CUDA_ARCH__
+  // to unsigned: this conversion saturates, so a negative u gives 0 by itself
+  int s;
+  if constexpr (sizeof(R) == 8)
+    s = (int)__double2uint_rz(u);
+  else
+    s = (int)__float2uint_rz(u);
+#else
   int s = (int)u;
   s = s < 0 ? 0 : s;
+#endif
   xi = R(2) * (u - R(s)) - R(1);
   return s;
 }
