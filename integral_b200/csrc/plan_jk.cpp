@@ -63,28 +63,9 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
   if (!tasks) return trc;
   KernelArgs A = base_args(P);
   A.mode = MODE_JK;
-  A.jk.D = d_dens;
   A.jk.bounds = P->d_bounds.p;
-  A.jk.ndens = A.jk.nscreen = A.jk.nj = ndens;
+  A.jk.nscreen = A.jk.nj = ndens;
   A.jk.want_k = want_k ? 1 : 0;
-  A.jk.symmetric = asym & 1 ? 0 : 1;
-  // FP64 builds of general densities run the one-orientation sums on their
-  // symmetric parts (all of J, and K's symmetric part) and antisymmetric parts
-  // (the rest of K): six sums a matrix in the specialised kernels against
-  // fourteen in the general ones (two densities of an 11-atom molecule:
-  // 12.6 ms, 19.2 before, a little of it from shorter Rys tables).  Mixed
-  // builds keep the general sums, which read the FP64 densities in every
-  // launch, and so do densities with an infinity or NaN, which the parts would
-  // spread.
-  const int nmat = want_k ? 2 * ndens : ndens;
-  const bool parts = asym == 1 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
-  if (parts) {
-    CK(P->d_parts.ensure((size_t)P->nao * P->nao * nmat));
-    CK(launch_split_symmetry(d_dens, P->d_parts.p, ndens, P->nao, want_k ? 1 : 0, s));
-    A.jk.D = P->d_parts.p;
-    A.jk.ndens = nmat;
-    A.jk.symmetric = 1;
-  }
   A.jk.threshold = threshold;
   A.prim_cut = prim_cut;
   A.bra_bitmap = bra_subset ? P->d_bitmap.p : nullptr;
@@ -95,23 +76,61 @@ int igpu_jk_device(igpu_plan* P, const double* d_dens, int ndens, const uint32_t
     CK(launch_to_float(d_dens, P->d_Df.p, n2, s));
     A.jk.Df = P->d_Df.p;
   }
-  if (A.jk.symmetric) {
-    // one-orientation accumulators, symmetrised into the caller's J/K below
-    CK(P->d_Jh.ensure(n2));
-    CK(cudaMemsetAsync(P->d_Jh.p, 0, n2 * sizeof(double), s));
-    A.jk.J = P->d_Jh.p;
-    if (want_k) {
-      const size_t nk = parts ? 2 * n2 : n2;
-      CK(P->d_Kh.ensure(nk));
-      CK(cudaMemsetAsync(P->d_Kh.p, 0, nk * sizeof(double), s));
-      A.jk.K = P->d_Kh.p;
-    }
-  } else {
-    A.jk.J = d_J;
-    A.jk.K = want_k ? d_K : nullptr;
-  }
+  // FP64 builds of general densities run the one-orientation sums on their
+  // symmetric parts (all of J, and K's symmetric part) and antisymmetric parts
+  // (the rest of K): six sums a matrix in the specialised kernels against
+  // fourteen in the general ones (two densities of an 11-atom molecule:
+  // 12.6 ms, 19.2 before, a little of it from shorter Rys tables).  Mixed
+  // builds keep the general sums, which read the FP64 densities in every
+  // launch, and so do densities with an infinity or NaN, which the parts would
+  // spread, and a device without room for the parts and their sums (up to five
+  // matrices a density and the running sums of twice the matrices; the general
+  // sums take none of these).
+  const int nmat = want_k ? 2 * ndens : ndens;
+  const size_t nm2 = (size_t)P->nao * P->nao * nmat;
+  bool parts = asym == 1 && precision == IGPU_PRECISION_FP64 && nmat <= MAX_DENS;
+  auto release_parts = [P] {
+    P->d_parts.release();
+    P->d_Jh.release();
+    P->d_Kh.release();
+  };
   uint32_t launches = 3;
-  int rc = run_tasks(P, *tasks, A, s, launches);
+  int rc;
+  for (;; parts = false) {
+    if (parts) {
+      cudaError_t e = P->d_parts.ensure(nm2);
+      if (e == cudaSuccess) e = P->d_Jh.ensure(n2);
+      if (e == cudaSuccess && want_k) e = P->d_Kh.ensure(nm2);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        release_parts();
+        continue;
+      }
+      CK(e);
+      CK(launch_split_symmetry(d_dens, P->d_parts.p, ndens, P->nao, want_k ? 1 : 0, s));
+    }
+    A.jk.D = parts ? P->d_parts.p : d_dens;
+    A.jk.ndens = parts ? nmat : ndens;
+    A.jk.symmetric = parts || !(asym & 1) ? 1 : 0;
+    if (A.jk.symmetric) {
+      // one-orientation accumulators, symmetrised into the caller's J/K below
+      CK(P->d_Jh.ensure(n2));
+      CK(cudaMemsetAsync(P->d_Jh.p, 0, n2 * sizeof(double), s));
+      A.jk.J = P->d_Jh.p;
+      if (want_k) {
+        const size_t nk = parts ? nm2 : n2;
+        CK(P->d_Kh.ensure(nk));
+        CK(cudaMemsetAsync(P->d_Kh.p, 0, nk * sizeof(double), s));
+        A.jk.K = P->d_Kh.p;
+      }
+    } else {
+      A.jk.J = d_J;
+      A.jk.K = want_k ? d_K : nullptr;
+    }
+    rc = run_tasks(P, *tasks, A, s, launches);
+    if (!(rc && parts && P->no_scratch)) break;
+    release_parts();
+  }
   if (rc) return rc;
   if (A.jk.symmetric) {
     CK(launch_symmetrize_add(P->d_Jh.p, d_J, ndens, P->nao, s));

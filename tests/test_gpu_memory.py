@@ -59,3 +59,33 @@ def test_overlapped_launches_without_room():
     with little_memory(256 * MB):
         got = gradient()
     assert rel(got, want) < 1e-12
+
+
+@pytest.mark.parametrize("rest", [200, 500])
+def test_general_densities_without_room(rest):
+    """32 general densities of 330 functions, 28 MB as a stack: 139 MB of parts
+    and their sums and 0.7 GB for the running sums of 64 matrices, beside some
+    140 MB of every build; run in 200 MB, which ends with the parts, and in
+    500 MB, which ends with the running sums."""
+    import torch
+
+    s = S.jk_system(natom=22, side=30.0, ndens=1)
+    D = torch.tensor(np.random.default_rng(3).normal(size=(32, 330, 330)), device="cuda")
+    J, K, J0, K0 = (torch.zeros_like(D) for _ in range(4))
+    bras = np.arange(0, len(s["shells"]) * (len(s["shells"]) + 1) // 2, 64)
+
+    def build(J, K, ndens):
+        dc = ib.Basis(s["shells"]).direct_contractor()
+        dc.jk_device(D.data_ptr(), ndens, J.data_ptr(), K.data_ptr(), 1e-9, bras=bras)
+
+    build(J0, K0, 32)
+    # the general sums' kernels too: a NaN keeps a density on them
+    D[0, 0, 1] = float("nan")
+    build(J, K, 1)
+    D[0, 0, 1] = D[0, 1, 0]
+    torch.cuda.synchronize()
+    build(J0.zero_(), K0.zero_(), 32)
+    J.zero_(), K.zero_()
+    with little_memory(rest * MB):
+        build(J, K, 32)
+    assert rel(J, J0) < 1e-12 and rel(K, K0) < 1e-12
