@@ -133,14 +133,6 @@ constexpr double kWideRounds = 3.0;
 // its last round is then at most a sixteenth of it.
 constexpr double kFullRounds = 16.0;
 
-// A plan's share in the pinned buffers of copy_to_host (host_copy.cpp).
-struct StageRef {
-  StageRef();
-  ~StageRef();
-  StageRef(const StageRef&) = delete;
-  StageRef& operator=(const StageRef&) = delete;
-};
-
 // Mixed-precision J/K task lists kept per plan (see igpu_plan::mixed_keys).
 constexpr size_t kMixedTaskSets = 4;
 
@@ -183,7 +175,6 @@ struct igpu_plan {
   // device
   cudaStream_t stream = nullptr;
   // the other streams of a run and the events that join them (run_tasks)
-  StageRef stage;
   std::vector<cudaStream_t> side;
   std::vector<cudaEvent_t> side_ev;
   ~igpu_plan() {
