@@ -1,8 +1,9 @@
 """The Rys roots and weights on the device: polynomials on unit intervals of T
-below 30.5 + 5 N, the Gauss-Laguerre limit above.  A quartet (aa|bb) of two
-single-primitive shells of exponent 1/2 has zeta 1 on both sides and T equal
-to half the squared distance, so the distance sets T: at interval edges, inside
-the first and last intervals, on both sides of the crossover and beyond.
+(FP64 tables of one and two roots: quarter intervals) below 30.5 + 5 N, the
+Gauss-Laguerre limit above.  A quartet (aa|bb) of two single-primitive shells
+of exponent 1/2 has zeta 1 on both sides and T equal to half the squared
+distance, so the distance sets T: at interval edges, inside the first and last
+intervals, on both sides of the crossover and beyond.
 
 s shells (N = 1) are held to the closed form within the fits' 2e-14 of a
 weight (the reference's bound for its tables) and rounding; p, d and f

@@ -4,13 +4,15 @@ which a J/K class launch takes from 3 x 128 quartets per SM.
 Their results are compared with igpu_jk_device_static, whose general
 eight-image path runs the team kernels on the same quartet list, within the
 J/K contract (1e-12 of the maxima; sums of some 1e4 products per element
-round to about 1e-14).  An 18-atom s,s,s,p,p,d system puts every wide class
-above the line; subsets, erf, missing exchange and several density counts
-take their branches."""
+round to about 1e-14), and on a sample of the bra pairs with the oracle.  An
+18-atom s,s,s,p,p,d system puts every wide class above the line; subsets, erf,
+missing exchange, several density counts and pairs without primitives take
+their branches."""
 import numpy as np
 import pytest
 
 import integral_b200 as ib
+import oracle_py as O
 from integral_b200 import systems as S
 
 pytestmark = pytest.mark.gpu
@@ -88,6 +90,22 @@ def test_wide_kernels_in_fp32(system):
         dc.set_mixed_cutoff(cutoff)
     assert WIDE32 <= {(r["la"], r["lb"], r["lc"], r["ld"]) for r in prof if r["team"] == 1 and r["fp32"] and r["quartets"]}
     assert rel(J32, J) < 1e-5 and rel(K32, K) < 1e-5
+
+
+def test_wide_kernels_match_the_oracle(system):
+    """A sample of the bra pairs (the launches keep their lists, so the wide
+    kernels run), quartet list and values."""
+    dc, D, thr = system
+    n = len(dc.bra_pairs())
+    bras = np.arange(7, n, 61)
+    J, K = build(dc, D[:2].contiguous(), thr, bras=bras)
+    st = dc.last_stats()
+    assert WIDE <= {(r["la"], r["lb"], r["lc"], r["ld"]) for r in dc.plan.profile() if r["team"] == 1 and r["quartets"]}
+    shells = S.jk_system(natom=18, side=13.1, ndens=5)["shells"]
+    Jo, Ko, cnt, hsh = O.OracleBasis(shells).direct_jk(D[:2].cpu().numpy(), thr, bras=bras, nthreads=8)
+    assert st["quartets"] == cnt and st["quartet_hash"] == hsh
+    for a, b in ((J, Jo), (K, Ko)):
+        assert float(np.max(np.abs(a.cpu().numpy() - b))) < 1e-12 * float(np.max(np.abs(b)))
 
 
 @pytest.fixture(scope="module")
