@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(128, quartet_min_blocks<LA, LB, LC, LD, R>()) 
         R G[S::NG];
         accumulate_thread<LA, LB, LC, LD, R>(A, tab, pb, pk, kpos, sub, split, G);
         if (split > 1) {
-          const unsigned group = (split == 32 ? 0xffffffffu : (1u << split) - 1u) << ((threadIdx.x & 31) - sub);
+          const unsigned group = ((1u << split) - 1u) << ((threadIdx.x & 31) - sub);  // split <= 16
 #pragma unroll
           for (int q = 0; q < S::NG; ++q)
             for (int o = 1; o < split; o *= 2) G[q] += __shfl_xor_sync(group, G[q], o);
