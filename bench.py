@@ -52,9 +52,9 @@ METRIC = "Fock J/K build quartets/s (FP32-mixed, <=1e-6 Eh vs FP64) on B200"
 UNIT = "quartets/s"
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one full-size launch of this
-# workload's kernels as they are, by kernel name, from a one-pass ncu capture;
-# bytes per launch.  No capture of the present kernels has been taken.
-NCU_TRAFFIC = {}
+# workload's dominant kernel, by kernel name, from a one-pass ncu capture on a
+# B200 (profiles/quartet_kernel_2221_fp32_traffic.md); bytes per launch.
+NCU_TRAFFIC = {"quartet_kernel(22|21) fp32": 38.07e6 + 687.56e6}
 
 
 def parse():

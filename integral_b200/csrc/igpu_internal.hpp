@@ -66,7 +66,7 @@ struct alignas(16) PrimPairF {
 // k of the class list lies at (q * KET_VALS + v) * stride + k, so that lanes
 // on consecutive kets read consecutive values.  From PrimPairD each such read
 // of a warp takes one L1 wavefront per lane (96 bytes apart), which bound
-// those kernels: 85-92% of the L1 rate in FP64.
+// those kernels: 82-92% of the L1 rate in FP64.
 constexpr int KET_VALS = 9;    // zeta, inv2z, ez, px, py, pz, pax, pay, paz
 constexpr int KET_VALS_F = 6;  // zeta, inv2z, ez, pax, pay, paz
 
